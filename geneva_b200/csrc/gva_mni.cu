@@ -22,7 +22,8 @@
 //           Each lane first searches its own seed for up to 64 candidates (32
 //           independent searches per warp keep many loads in flight); seeds
 //           still undecided are searched by the whole warp, 32 candidates per
-//           step, one seed at a time
+//           step, one seed at a time; what a warp leaves undecided after a
+//           few steps is cut into pieces that all warps share (MniWork)
 //   stop    a task stops once its count reaches the cap (default: the minimum
 //           support, which decides frequency) or the smallest exhausted orbit
 //           of its pattern, so the support returned is min(MNI, cap) exactly
@@ -115,85 +116,166 @@ __device__ __forceinline__ bool root_ok(const MniTask& T, const PartPtr* __restr
     return true;
 }
 
-// Whether some embedding maps level 0 to `root`.  Called by all 32 lanes with
-// the same root; the search state is identical in every lane.
-__device__ bool mni_dfs(const MniTask& T, const PartPtr* __restrict__ parts, uint32_t L, uint32_t root, uint32_t lane,
-                        unsigned long long* cnt) {
+// State of a warp's depth-first search, identical in every lane: the vertices
+// matched so far and, per open level, what is left of its candidate list.
+struct Dfs {
     uint32_t f[kMniMaxVertices];
     uint32_t pos[kMniMaxVertices], end[kMniMaxVertices], gsel[kMniMaxVertices];
     const uint32_t* gadj[kMniMaxVertices];
-    const int n = (int)T.n;
-    f[0] = root;
-    if (n <= 1) return true;
-    // candidates of level lv: the shortest segment among its matched neighbours
-    auto open = [&](int lv) {
-        uint32_t blo = 0, bhi = 0, bj = 0;
-        const uint32_t* ba = nullptr;
-        bool have = false;
-        uint32_t m = T.nbmask[lv];
-        while (m) {
-            const int j = __ffs(m) - 1;
-            m &= m - 1;
-            const PartPtr P = parts[T.part[lv][j] - 1];
-            uint32_t lo, hi;
-            seg_of(P.off, L, f[j], T.lab[lv], lo, hi);
-            if (!have || hi - lo < bhi - blo) {
-                blo = lo;
-                bhi = hi;
-                bj = (uint32_t)j;
-                ba = P.adj;
-                have = true;
-            }
+};
+
+// Candidates of level lv: the shortest segment among its matched neighbours.
+__device__ __forceinline__ void dfs_open(const MniTask& T, const PartPtr* __restrict__ parts, uint32_t L, Dfs& s,
+                                         int lv) {
+    uint32_t blo = 0, bhi = 0, bj = 0;
+    const uint32_t* ba = nullptr;
+    bool have = false;
+    uint32_t m = T.nbmask[lv];
+    while (m) {
+        const int j = __ffs(m) - 1;
+        m &= m - 1;
+        const PartPtr P = parts[T.part[lv][j] - 1];
+        uint32_t lo, hi;
+        seg_of(P.off, L, s.f[j], T.lab[lv], lo, hi);
+        if (!have || hi - lo < bhi - blo) {
+            blo = lo;
+            bhi = hi;
+            bj = (uint32_t)j;
+            ba = P.adj;
+            have = true;
         }
-        pos[lv] = blo;
-        end[lv] = bhi;
-        gadj[lv] = ba;
-        gsel[lv] = bj;
-        cnt[P_OPENS] += lane == 0 ? 1 : 0;
-    };
-    int i = 1;
-    open(1);
-    for (;;) {
-        if (pos[i] >= end[i]) {
-            if (--i == 0) return false;
+    }
+    s.pos[lv] = blo;
+    s.end[lv] = bhi;
+    s.gadj[lv] = ba;
+    s.gsel[lv] = bj;
+}
+
+// Searches, by the whole warp, the levels from `base` (its range open, the
+// levels below it matched) for one embedding: 1 = found, 0 = none in the
+// ranges left open, -1 = `budget` steps of 32 candidates taken (the state, and
+// the current level in `i`, then say what is left).  A step loads 32
+// candidates and, where other matched neighbours bind the level, the index
+// and a few words of their segments for each: a chain of dependent loads that
+// only other warps can hide, so a root that takes long must not stay with one
+// warp.
+__device__ int warp_search(const MniTask& T, const PartPtr* __restrict__ parts, uint32_t L, Dfs& s, int base, int& i,
+                           uint32_t budget, uint32_t lane, unsigned long long* cnt) {
+    const int n = (int)T.n;
+    for (uint32_t steps = 0;;) {
+        if (s.pos[i] >= s.end[i]) {
+            if (--i < base) return 0;
             continue;
         }
-        const uint32_t p = pos[i] + lane;
+        if (steps++ >= budget) return -1;
+        const uint32_t p = s.pos[i] + lane;
         uint32_t c = 0;
         bool ok = false;
-        if (p < end[i]) {
-            c = __ldg(gadj[i] + p);
+        if (p < s.end[i]) {
+            c = __ldg(s.gadj[i] + p);
             ok = true;
             cnt[P_SCANNED] += 1;
             uint32_t e = T.eqmask[i];
             while (e && ok) {
                 const int j = __ffs(e) - 1;
                 e &= e - 1;
-                ok = c != f[j];
+                ok = c != s.f[j];
             }
-            uint32_t m = T.nbmask[i] & ~(1u << gsel[i]);
+            uint32_t m = T.nbmask[i] & ~(1u << s.gsel[i]);
             while (m && ok) {
                 const int j = __ffs(m) - 1;
                 m &= m - 1;
                 const PartPtr P = parts[T.part[i][j] - 1];
                 uint32_t lo, hi;
-                seg_of(P.off, L, f[j], T.lab[i], lo, hi);
+                seg_of(P.off, L, s.f[j], T.lab[i], lo, hi);
                 ok = find_in(P.adj, lo, hi, c) != 0xffffffffu;
                 cnt[P_CHECKS] += 1;
             }
         }
         const uint32_t b = __ballot_sync(0xffffffffu, ok);
         if (!b) {
-            pos[i] += 32;
+            s.pos[i] += 32;
             continue;
         }
         const int l = __ffs(b) - 1;
-        f[i] = __shfl_sync(0xffffffffu, c, l);
-        pos[i] += (uint32_t)l + 1;
-        if (i + 1 == n) return true;
+        s.f[i] = __shfl_sync(0xffffffffu, c, l);
+        s.pos[i] += (uint32_t)l + 1;
+        if (i + 1 == n) return 1;
         ++i;
-        open(i);
+        dfs_open(T, parts, L, s, i);
+        cnt[P_OPENS] += lane == 0 ? 1 : 0;
     }
+}
+
+// What is left of a search that ran out of its budget, as pieces that any
+// warp can take: the matched prefix f[0 .. level) and a range of the
+// candidates of `level`, read from the segment of f[gsel].
+struct MniWork {
+    uint32_t hard;  // the root's flag in MniHard::found
+    uint32_t task;
+    uint32_t cap;   // of the root's slot
+    uint32_t level;
+    uint32_t pos, end;
+    uint32_t gsel;
+    uint32_t f[kMniMaxVertices - 1];
+};
+constexpr uint32_t kWorkWords = sizeof(MniWork) / 4;
+static_assert(kWorkWords <= 32, "one lane per word");
+
+// The pieces of one round: two queues (a launch takes from one and puts what
+// its searches leave into the other) and the roots they belong to.
+struct MniHard {
+    MniWork* queue[2];
+    unsigned long long* state;  // [0 .. 2) = queue 0: pieces, head; [2 .. 4) = queue 1; [4] = roots
+    uint32_t* found;            // per root: an embedding was found
+    uint32_t cap_work, cap_roots;
+};
+constexpr uint32_t kMniWorkCap = 1u << 18, kMniRootCap = 1u << 18;
+constexpr uint32_t kMniPieces = 16;      // pieces of one level's range
+constexpr uint32_t kMniCrowded = 1u << 15;  // with this many pieces waiting, ranges are no longer cut
+
+// Room for n entries in a counted array of `cap`; cap or more: there is none.
+__device__ __forceinline__ unsigned long long reserve(unsigned long long* count, uint32_t n, uint32_t cap) {
+    unsigned long long at = *(volatile unsigned long long*)count;
+    while (at + n <= cap) {
+        const unsigned long long seen = atomicCAS(count, at, at + n);
+        if (seen == at) return at;
+        at = seen;
+    }
+    return cap;
+}
+
+// Puts the open levels base .. i of a search into queue `q`; false: it is
+// full (nothing was put there).
+__device__ bool put_pieces(const MniHard& H, int q, const Dfs& s, int base, int i, uint32_t hard, uint32_t task,
+                           uint32_t cap, uint32_t lane) {
+    unsigned long long* count = H.state + 2 * q;
+    uint32_t most = 1, total = 0;
+    unsigned long long at = 0;
+    if (lane == 0) most = *(volatile unsigned long long*)count < kMniCrowded ? kMniPieces : 1;
+    most = __shfl_sync(0xffffffffu, most, 0);
+    for (int j = base; j <= i; ++j)
+        if (s.pos[j] < s.end[j]) total += min(most, s.end[j] - s.pos[j]);
+    if (lane == 0) at = reserve(count, total, H.cap_work);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (at >= H.cap_work) return total == 0;
+    for (int j = base; j <= i; ++j) {
+        if (s.pos[j] >= s.end[j]) continue;
+        const uint32_t len = s.end[j] - s.pos[j], np = min(most, len);
+        if (lane < np) {
+            MniWork& w = H.queue[q][at + lane];
+            w.hard = hard;
+            w.task = task;
+            w.cap = cap;
+            w.level = (uint32_t)j;
+            w.pos = s.pos[j] + (uint32_t)((uint64_t)len * lane / np);
+            w.end = s.pos[j] + (uint32_t)((uint64_t)len * (lane + 1) / np);
+            w.gsel = s.gsel[j];
+            for (int k = 0; k < kMniMaxVertices - 1; ++k) w.f[k] = k < j ? s.f[k] : 0u;
+        }
+        at += np;
+    }
+    return true;
 }
 
 // One lane's own depth-first search for an embedding with level 0 at `root`,
@@ -204,85 +286,90 @@ __device__ bool mni_dfs(const MniTask& T, const PartPtr* __restrict__ parts, uin
 // fail within a few candidates.
 __device__ int lane_dfs(const MniTask& T, const PartPtr* __restrict__ parts, uint32_t L, uint32_t root,
                         uint32_t budget, unsigned long long* cnt) {
-    uint32_t f[kMniMaxVertices];
-    uint32_t pos[kMniMaxVertices], end[kMniMaxVertices], gsel[kMniMaxVertices];
-    const uint32_t* gadj[kMniMaxVertices];
+    Dfs s;
     const int n = (int)T.n;
-    f[0] = root;
+    s.f[0] = root;
     if (n <= 1) return 1;
-    auto open = [&](int lv) {
-        uint32_t blo = 0, bhi = 0, bj = 0;
-        const uint32_t* ba = nullptr;
-        bool have = false;
-        uint32_t m = T.nbmask[lv];
-        while (m) {
-            const int j = __ffs(m) - 1;
-            m &= m - 1;
-            const PartPtr P = parts[T.part[lv][j] - 1];
-            uint32_t lo, hi;
-            seg_of(P.off, L, f[j], T.lab[lv], lo, hi);
-            if (!have || hi - lo < bhi - blo) {
-                blo = lo;
-                bhi = hi;
-                bj = (uint32_t)j;
-                ba = P.adj;
-                have = true;
-            }
-        }
-        pos[lv] = blo;
-        end[lv] = bhi;
-        gadj[lv] = ba;
-        gsel[lv] = bj;
-        cnt[P_OPENS] += 1;
-    };
     int i = 1;
-    open(1);
+    dfs_open(T, parts, L, s, 1);
+    cnt[P_OPENS] += 1;
     uint32_t steps = 0;
     for (;;) {
-        if (pos[i] >= end[i]) {
+        if (s.pos[i] >= s.end[i]) {
             if (--i == 0) return 0;
             continue;
         }
         if (++steps > budget) return -1;
-        const uint32_t c = __ldg(gadj[i] + pos[i]);
-        ++pos[i];
+        const uint32_t c = __ldg(s.gadj[i] + s.pos[i]);
+        ++s.pos[i];
         cnt[P_SCANNED] += 1;
         bool ok = true;
         uint32_t e = T.eqmask[i];
         while (e && ok) {
             const int j = __ffs(e) - 1;
             e &= e - 1;
-            ok = c != f[j];
+            ok = c != s.f[j];
         }
-        uint32_t m = T.nbmask[i] & ~(1u << gsel[i]);
+        uint32_t m = T.nbmask[i] & ~(1u << s.gsel[i]);
         while (m && ok) {
             const int j = __ffs(m) - 1;
             m &= m - 1;
             const PartPtr P = parts[T.part[i][j] - 1];
             uint32_t lo, hi;
-            seg_of(P.off, L, f[j], T.lab[i], lo, hi);
+            seg_of(P.off, L, s.f[j], T.lab[i], lo, hi);
             ok = find_in(P.adj, lo, hi, c) != 0xffffffffu;
             cnt[P_CHECKS] += 1;
         }
         if (!ok) continue;
-        f[i] = c;
+        s.f[i] = c;
         if (i + 1 == n) return 1;
         ++i;
-        open(i);
+        dfs_open(T, parts, L, s, i);
+        cnt[P_OPENS] += 1;
     }
 }
 
 constexpr uint32_t kLaneBudget = 64;  // candidates a lane search may take before the warp search decides
+// Steps of 32 candidates that a warp may take on a root before what is left
+// is cut into pieces for every warp, and on a piece before it is cut again.
+constexpr uint32_t kWarpBudget = 32, kPieceBudget = 128;
+
+__device__ __forceinline__ void load_task(MniTask& T, const MniTask* __restrict__ src, uint32_t lane) {
+    __syncwarp();
+    const uint32_t* s = reinterpret_cast<const uint32_t*>(src);
+    uint32_t* dst = reinterpret_cast<uint32_t*>(&T);
+    for (uint32_t k = lane; k < sizeof(MniTask) / 4; k += 32) dst[k] = __ldg(s + k);
+    __syncwarp();
+}
+
+__device__ __forceinline__ void add_prof(unsigned long long* prof, const unsigned long long* cnt, uint32_t lane) {
+    if (!prof) return;
+    for (int k = 0; k < P_NUM; ++k) {
+        const unsigned long long x = warp_sum(cnt[k]);
+        if (lane == 0 && x) atomicAdd(prof + k, x);
+    }
+}
 
 // Persistent: every warp pulls 128-seed items; per 32 seeds it checks the
 // task's count against its cap, filters roots by neighbour-label degrees and
-// runs one search per surviving root.
+// runs one search per surviving root.  A root that neither a lane nor the
+// warp decides within its budget goes to the pieces of mni_piece_kernel.
+//
+// Why: nearly every root is decided within a few candidates, but one without
+// an embedding under a hub can take millions of steps (pairs of a hub's
+// neighbours, each closed or not by a third list), and one warp then works
+// alone while the chip waits.  On an R-MAT graph of 2^17 vertices and 2M edges
+// one root of one pattern of 1,200 held its warp for 247 of the launch's
+// 254 ms; with the pieces the same 1,200 supports (cap 1,000) take 3.0 ms of
+// device time.  What bounds the kernel now is the latency of the searches'
+// dependent loads (index record, list, index record): 0.12 TB/s of
+// algorithmic bytes.
 __global__ void __launch_bounds__(kMniWarps * 32, 6)
 mni_search_kernel(const MniTask* __restrict__ tasks, const MniSlot* __restrict__ slots,
                   const uint64_t* __restrict__ item0, const uint32_t* __restrict__ item_slot, uint64_t nitems,
                   const uint32_t* __restrict__ seeds, uint32_t item_len,
                   const PartPtr* __restrict__ parts, uint32_t L, uint32_t* __restrict__ counts,
-                  unsigned long long* __restrict__ queue, unsigned long long* __restrict__ prof) {
+                  unsigned long long* __restrict__ queue, MniHard H, unsigned long long* __restrict__ prof) {
     __shared__ MniTask tsh[kMniWarps];
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     MniTask& T = tsh[w];
@@ -296,11 +383,7 @@ mni_search_kernel(const MniTask* __restrict__ tasks, const MniSlot* __restrict__
         const int s = (int)__ldg(item_slot + it);
         const MniSlot sl = slots[s];
         if ((int)sl.task != cur) {
-            __syncwarp();
-            const uint32_t* src = reinterpret_cast<const uint32_t*>(tasks + sl.task);
-            uint32_t* dst = reinterpret_cast<uint32_t*>(&T);
-            for (uint32_t k = lane; k < sizeof(MniTask) / 4; k += 32) dst[k] = __ldg(src + k);
-            __syncwarp();
+            load_task(T, tasks + sl.task, lane);
             cur = (int)sl.task;
         }
         const uint32_t a = sl.start + (uint32_t)(it - item0[s]) * item_len;
@@ -328,20 +411,78 @@ mni_search_kernel(const MniTask* __restrict__ tasks, const MniSlot* __restrict__
             while (m) {
                 const int l = __ffs(m) - 1;
                 m &= m - 1;
-                const uint32_t root = __shfl_sync(0xffffffffu, v, l);
-                if (mni_dfs(T, parts, L, root, lane, cnt)) ++found;
+                Dfs st;
+                st.f[0] = __shfl_sync(0xffffffffu, v, l);
+                int i = 1;
+                dfs_open(T, parts, L, st, 1);
+                cnt[P_OPENS] += lane == 0 ? 1 : 0;
+                int r = warp_search(T, parts, L, st, 1, i, kWarpBudget, lane, cnt);
+                if (r < 0) {
+                    unsigned long long hard = 0;
+                    if (lane == 0) hard = reserve(H.state + 4, 1, H.cap_roots);
+                    hard = __shfl_sync(0xffffffffu, hard, 0);
+                    if (hard >= H.cap_roots ||
+                        !put_pieces(H, 0, st, 1, i, (uint32_t)hard, sl.task, sl.cap, lane))
+                        r = warp_search(T, parts, L, st, 1, i, 0xffffffffu, lane, cnt);  // no room: to its end here
+                }
+                if (r > 0) ++found;
             }
             if (found && lane == 0) atomicAdd(counts + sl.task, found);
             if (lane == 0) cnt[P_FOUND] += found;
         }
     }
-    if (prof) {
-        for (int k = 0; k < P_NUM; ++k) {
-            unsigned long long x = cnt[k];
-            x = warp_sum(x);
-            if (lane == 0 && x) atomicAdd(prof + k, x);
+    add_prof(prof, cnt, lane);
+}
+
+// The pieces of queue q, one per warp at a time: each is searched for up to
+// kPieceBudget steps and what is left goes, cut again, to the other queue (a
+// search thus spreads over the chip within two or three launches).  The first
+// embedding of a root counts it; the root's other pieces are then skipped, as
+// are pieces of a task at its cap.
+__global__ void __launch_bounds__(kMniWarps * 32, 6)
+mni_piece_kernel(const MniTask* __restrict__ tasks, const PartPtr* __restrict__ parts, uint32_t L,
+                 uint32_t* __restrict__ counts, MniHard H, int q, unsigned long long* __restrict__ prof) {
+    __shared__ MniTask tsh[kMniWarps];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    MniTask& T = tsh[w];
+    unsigned long long cnt[P_NUM] = {0, 0, 0, 0, 0, 0};
+    unsigned long long* state = H.state + 2 * q;
+    const unsigned long long n = state[0];  // only read by this launch
+    uint32_t cur = 0xffffffffu;
+    for (;;) {
+        unsigned long long it = 0;
+        if (lane == 0) it = atomicAdd(state + 1, 1ull);
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it >= n) break;
+        uint32_t word = 0;
+        if (lane < kWorkWords) word = __ldg(reinterpret_cast<const uint32_t*>(H.queue[q] + it) + lane);
+        auto field = [&](int k) { return __shfl_sync(0xffffffffu, word, k); };
+        const uint32_t hard = field(0), task = field(1), cap = field(2);
+        bool skip = false;
+        if (lane == 0)
+            skip = *(volatile const uint32_t*)(H.found + hard) || *(volatile const uint32_t*)(counts + task) >= cap;
+        if (__shfl_sync(0xffffffffu, skip, 0)) continue;
+        if (task != cur) {
+            load_task(T, tasks + task, lane);
+            cur = task;
+        }
+        const int base = (int)field(3);
+        Dfs s;
+        for (int k = 0; k < kMniMaxVertices - 1; ++k) s.f[k] = field(7 + k);
+        s.pos[base] = field(4);
+        s.end[base] = field(5);
+        s.gsel[base] = field(6);
+        s.gadj[base] = parts[T.part[base][s.gsel[base]] - 1].adj;
+        int i = base;
+        int r = warp_search(T, parts, L, s, base, i, kPieceBudget, lane, cnt);
+        if (r < 0 && !put_pieces(H, q ^ 1, s, base, i, hard, task, cap, lane))
+            r = warp_search(T, parts, L, s, base, i, 0xffffffffu, lane, cnt);
+        if (r > 0 && lane == 0 && atomicExch(H.found + hard, 1u) == 0) {
+            atomicAdd(counts + task, 1u);
+            cnt[P_FOUND] += 1;
         }
     }
+    add_prof(prof, cnt, lane);
 }
 
 std::atomic<uint64_t> g_mni_launches{0};
@@ -588,7 +729,12 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
     const size_t bytes_prof = P_NUM * 8;
     void* dmem = nullptr;
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    const size_t fixed = al(bytes_tasks) + al(bytes_counts) + al(bytes_parts) + al(bytes_prof) + 256;
+    // the counts, the search queue's head and the pieces' state lie together:
+    // one copy reads back the counts and whether pieces are left
+    const size_t o_queue = (bytes_counts + 15) & ~(size_t)15, bytes_state = 6 * 8;
+    const size_t bytes_found = (size_t)kMniRootCap * 4, bytes_work = 2 * (size_t)kMniWorkCap * sizeof(MniWork);
+    const size_t fixed = al(bytes_tasks) + al(o_queue + bytes_state) + al(bytes_parts) + al(bytes_prof) +
+                         al(bytes_found) + bytes_work;
     if (cudaMallocAsync(&dmem, fixed, s) != cudaSuccess) return fail(GVA_ERR_NOMEM, "MNI task allocation failed");
     struct Free {
         void* p;
@@ -599,18 +745,27 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
     MniTask* d_tasks = (MniTask*)cur;
     cur += al(bytes_tasks);
     uint32_t* d_counts = (uint32_t*)cur;
-    cur += al(bytes_counts);
+    unsigned long long* d_queue = (unsigned long long*)(cur + o_queue);  // head, then MniHard::state
+    cur += al(o_queue + bytes_state);
     PartPtr* d_parts = (PartPtr*)cur;
     cur += al(bytes_parts);
     unsigned long long* d_prof = (unsigned long long*)cur;
     cur += al(bytes_prof);
-    unsigned long long* d_queue = (unsigned long long*)cur;
+    MniHard H{};
+    H.found = (uint32_t*)cur;
+    cur += al(bytes_found);
+    H.queue[0] = (MniWork*)cur;
+    H.queue[1] = H.queue[0] + kMniWorkCap;
+    H.state = d_queue + 1;
+    H.cap_work = kMniWorkCap;
+    H.cap_roots = kMniRootCap;
     // every host<->device copy goes through pinned staging: a pageable copy
     // blocks its thread inside the driver until the stream drains, which
     // other threads' CUDA calls (a server's matching loop) would wait behind
     Staging tstage, cstage;
     char* ht = tstage.get(al(bytes_tasks) + P * sizeof(PartPtr));
-    uint32_t* hcounts = (uint32_t*)cstage.get(bytes_counts);
+    const size_t bytes_back = o_queue + bytes_state;
+    uint32_t* hcounts = (uint32_t*)cstage.get(bytes_back);
     if (!ht || !hcounts) return fail(GVA_ERR_NOMEM, "pinned staging allocation failed");
     memcpy(ht, tasks.data(), bytes_tasks);
     memcpy(ht + al(bytes_tasks), hparts.data(), P * sizeof(PartPtr));
@@ -618,6 +773,7 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
     GVA_CUDA_M(cudaMemcpyAsync(d_parts, ht + al(bytes_tasks), P * sizeof(PartPtr), cudaMemcpyHostToDevice, s));
     GVA_CUDA_M(cudaMemsetAsync(d_counts, 0, bytes_counts, s));
     GVA_CUDA_M(cudaMemsetAsync(d_prof, 0, bytes_prof, s));
+    GVA_CUDA_M(cudaMemsetAsync(H.found, 0, bytes_found, s));
 
     int sms = 148, per_sm = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, db.device);
@@ -704,7 +860,7 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
             uint64_t* d_item0 = (uint64_t*)((char*)dround + al(ns * sizeof(MniSlot)));
             uint32_t* d_item_slot = (uint32_t*)((char*)dround + al(need));
             if (cudaMemcpyAsync(dround, h, need, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-                cudaMemsetAsync(d_queue, 0, 8, s) != cudaSuccess) {
+                cudaMemsetAsync(d_queue, 0, bytes_state, s) != cudaSuccess) {
                 rc = fail(GVA_ERR_CUDA, "MNI round upload failed");
                 break;
             }
@@ -720,25 +876,47 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
             if (profile) prof.begin(K_MNI, 0.0, s, ev);
             mni_search_kernel<<<(unsigned)std::max<uint64_t>(grid, 1), kMniWarps * 32, 0, s>>>(
                 d_tasks, d_slots, d_item0, d_item_slot, nitems, db.seed_by_degree, (uint32_t)item_len, d_parts, db.kernel_L(),
-                d_counts, d_queue,
-                profile ? d_prof : nullptr);
+                d_counts, d_queue, H, profile ? d_prof : nullptr);
             if (profile) prof.end(ev, K_MNI, 0.0, s, rows);
             st.launches += 2;
             g_mni_launches += 2;
             st.rounds++;
-            cudaError_t le = cudaGetLastError();
-            if (le == cudaSuccess) le = cudaMemcpyAsync(hcounts, d_counts, bytes_counts, cudaMemcpyDeviceToHost, s);
-            if (le != cudaSuccess) {
-                rc = fail(GVA_ERR_CUDA, std::string("MNI search launch failed: ") + cudaGetErrorString(le));
-                break;
+            // counts back, and how many pieces are left for the piece kernel:
+            // they are taken four launches at a time until none is
+            const unsigned long long* hstate = (const unsigned long long*)((const char*)hcounts + o_queue) + 1;
+            uint64_t hard_roots = 0;
+            for (int q = 0;;) {
+                cudaError_t le = cudaGetLastError();
+                if (le == cudaSuccess) le = cudaMemcpyAsync(hcounts, d_counts, bytes_back, cudaMemcpyDeviceToHost, s);
+                if (le != cudaSuccess) {
+                    rc = fail(GVA_ERR_CUDA, std::string("MNI search launch failed: ") + cudaGetErrorString(le));
+                    break;
+                }
+                const auto w0 = std::chrono::steady_clock::now();
+                const cudaError_t e = cudaStreamSynchronize(s);
+                st.wait_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - w0).count();
+                if (e != cudaSuccess) {
+                    rc = fail(GVA_ERR_CUDA, std::string("MNI search failed: ") + cudaGetErrorString(e));
+                    break;
+                }
+                hard_roots = hstate[4];
+                if (hstate[2 * q] == 0) break;
+                if (cancel && *cancel) {
+                    rc = fail(GVA_ERR_CANCELLED, "cancelled");
+                    break;
+                }
+                for (int k = 0; k < 4; ++k, q ^= 1) {
+                    cudaMemsetAsync(H.state + 2 * (q ^ 1), 0, 16, s);  // taken by the launch before
+                    if (profile) prof.begin(K_MNI, 0.0, s, ev);
+                    mni_piece_kernel<<<(unsigned)cta_cap, kMniWarps * 32, 0, s>>>(
+                        d_tasks, d_parts, db.kernel_L(), d_counts, H, q, profile ? d_prof : nullptr);
+                    if (profile) prof.end(ev, K_MNI, 0.0, s, 0.0);
+                }
+                st.launches += 4;
+                g_mni_launches += 4;
             }
-            const auto w0 = std::chrono::steady_clock::now();
-            const cudaError_t e = cudaStreamSynchronize(s);
-            st.wait_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - w0).count();
-            if (e != cudaSuccess) {
-                rc = fail(GVA_ERR_CUDA, std::string("MNI search failed: ") + cudaGetErrorString(e));
-                break;
-            }
+            if (rc) break;
+            if (hard_roots) cudaMemsetAsync(H.found, 0, hard_roots * 4, s);
             memcpy(counts.data(), hcounts, bytes_counts);
             // exhausted tasks fix their pattern's cap; capped ones retire
             w = 0;
