@@ -16,6 +16,10 @@
 // budget-sized pieces, deepest tasks first.  This replaces the reference's
 // kernel-abort/host-spill protocol (src/gpumine.cpp:406-467,
 // src/miningPattern.cu:3325-3343) and its one-query-per-process driver.
+// These counted rounds serve sessions, small budgets and profiled runs; a run
+// whose plans arrive in one wave walks its rows once, without counting them
+// first ("rounds in one pass" below).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -61,7 +65,7 @@ struct TaskDesc {
     uint32_t kind;     // STEP_EXT / STEP_REDUCE
     uint32_t mode;     // TaskMode
     uint32_t query;    // per-graph result slot
-    uint32_t pad;
+    uint32_t feeds;    // a child can match: the rows are needed
     union {
         ExtArgs e;
         RedArgs r;
@@ -92,21 +96,6 @@ constexpr int kTileRows = 64;           // output rows staged per warp before a 
 constexpr int kScanChunk = 4096;        // items per CTA of the item scan
 constexpr int kScanChunkLog2 = 12;
 
-// Device-side state of one round when the rounds are scheduled on the device
-// (BatchSession::run_device): the count pass's tasks and items (written by
-// the previous round's planning kernel, or by the host for the first round),
-// the write pass's (written by this round's planning kernel) and the four
-// work-queue heads (zero when the state is created).  A set `overflow` makes
-// every later launch of the run find no work.
-struct RunState {
-    uint64_t ni, ni_light;  // count items: all, light class (the light class's items come first)
-    uint64_t wi, wi_light;  // write items: all, light class
-    uint32_t nt, nt_light;  // count tasks: all, light class
-    uint32_t nw;            // writing tasks
-    uint32_t overflow;      // frontier region, task or item capacity exceeded
-    unsigned long long heads[4];  // queue heads: count light, count fused, write light, write fused
-};
-
 struct RoundArgs {
     const TaskDesc* nodes;
     const TaskRef* refs;
@@ -127,43 +116,14 @@ struct RoundArgs {
     uint32_t* const* task_out;    // write: output base of each task (null: not written this round)
     unsigned long long* read_words;  // optional: candidate-list words read (profiling)
     BatchCtx ctx;
-    RunState* dyn;                // device-scheduled rounds: item ranges, task counts and queue heads from
-                                  // here instead of the fields above (null: host-scheduled)
 };
 
-// The item range of one launch: from the arguments (host-scheduled rounds)
-// or from the round's device state.
+// The items [base, base + n) of one launch.
 struct Span {
-    uint64_t base, n;              // items [base, base + n) of this launch
-    uint64_t n_count_items, n_chunks;  // write pass: items and scan chunks of the count pass
+    uint64_t base, n;
     unsigned long long* queue;
-    uint32_t nt;                   // tasks (count) or writing tasks (write)
-    uint32_t warps;                // resident warps of the persistent grid
+    uint32_t warps;  // resident warps of the persistent grid
 };
-
-template <bool WRITE>
-__device__ __forceinline__ Span launch_span(const RoundArgs& a, bool fused) {
-    Span s;
-    s.warps = gridDim.x * kRoundWarps;
-    if (!a.dyn) {
-        s.base = a.item_base;
-        s.n = a.n_items;
-        s.nt = a.nt;
-        s.n_count_items = a.n_count_items;
-        s.n_chunks = a.n_chunks;
-        s.queue = a.queue;
-        return s;
-    }
-    const RunState& st = *a.dyn;
-    const uint64_t all = WRITE ? st.wi : st.ni, light = WRITE ? st.wi_light : st.ni_light;
-    s.base = fused ? light : 0;
-    s.n = fused ? all - light : light;
-    s.nt = WRITE ? st.nw : st.nt;
-    s.n_count_items = st.ni;
-    s.n_chunks = (st.ni + kScanChunk - 1) / kScanChunk;
-    s.queue = a.dyn->heads + (WRITE ? 2 : 0) + (fused ? 1 : 0);
-    return s;
-}
 
 // Per-(query, graph) accounting of a final-step row: lanes of a warp whose
 // rows lie in the same graph (rows arrive grouped by their first vertex)
@@ -206,15 +166,19 @@ __device__ __forceinline__ bool next_chunk(const Span& a, uint64_t& begin, uint6
     return begin < a.n;
 }
 
-// last t in [0, n) with pfx[t] <= x (pfx ascending, pfx[0] <= x)
+// Last t in [0, n) with pfx[t] <= x (pfx ascending, pfx[0] <= x), by the whole
+// warp: 32 pivots per step, so three dependent loads find one of 32,768
+// tasks (a binary search takes 15, about half of what a small round's only
+// item per warp waits for).
 __device__ __forceinline__ uint32_t find_slot(const uint64_t* __restrict__ pfx, uint32_t n, uint64_t x) {
-    uint32_t lo = 0, hi = n;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(pfx + mid) <= x)
-            lo = mid;
-        else
-            hi = mid;
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t lo = 0, len = n;
+    while (len > 1) {
+        const uint32_t step = (len + 31) / 32, at = lane * step;
+        const uint32_t m = __ballot_sync(0xffffffffu, at < len && __ldg(pfx + lo + at) <= x);
+        const uint32_t k = (31 - __clz(m)) * step;  // lane 0's pivot always qualifies
+        lo += k;
+        len = min(step, len - k);
     }
     return lo;
 }
@@ -541,8 +505,8 @@ struct WarpSmem {
     uint32_t* tile;
     GenState* gen;
 };
-template <bool WRITE, bool FUSED>
-__device__ __forceinline__ WarpSmem warp_smem(unsigned char* raw, const RoundArgs& a) {
+template <bool WRITE, bool FUSED, class Args>
+__device__ __forceinline__ WarpSmem warp_smem(unsigned char* raw, const Args& a) {
     const int warp = threadIdx.x >> 5;
     WarpSmem w;
     w.d = reinterpret_cast<TaskDesc*>(raw) + warp;
@@ -573,11 +537,11 @@ round_count_kernel(RoundArgs a) {
     uint64_t begin, end;
     uint32_t cur = 0;    // light class: buffer of the current item
     bool ready = false;  // light class: the current item's rows were issued with the previous item
-    const Span sp = launch_span<false>(a, FUSED);
+    const Span sp{a.item_base, a.n_items, a.queue, gridDim.x * kRoundWarps};
     while (next_chunk(sp, begin, end)) {
         for (uint64_t item = sp.base + begin; item < sp.base + end; ++item) {
             if (item >= t_hi || item < t_lo) {
-                t = find_slot(a.item0, sp.nt + 1, item);
+                t = find_slot(a.item0, a.nt + 1, item);
                 t_lo = __ldg(a.item0 + t);
                 t_hi = __ldg(a.item0 + t + 1);
                 const TaskRef& ref = a.refs[t];
@@ -626,14 +590,12 @@ round_count_kernel(RoundArgs a) {
 
 // --------------------------------------------------------- item scans ----
 // Exclusive scan of per-item counts in chunks of kScanChunk (in place);
-// chunks[c] receives chunk c's sum.  A block per chunk, the grid striding
-// over the chunks (n from the round's device state when `dyn` is given).
+// chunks[c] receives chunk c's sum.  A block per chunk.
 __global__ void __launch_bounds__(1024) scan_items_local_kernel(uint64_t* __restrict__ v, uint64_t n,
-                                                               uint64_t* __restrict__ chunks, const RunState* dyn) {
+                                                               uint64_t* __restrict__ chunks) {
     __shared__ uint64_t ws[32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (dyn) n = dyn->ni;
-    for (uint64_t c = blockIdx.x; c * kScanChunk < n; c += gridDim.x) {
+    const uint64_t c = blockIdx.x;
     const uint64_t base = c * kScanChunk + (uint64_t)threadIdx.x * 4;
     uint64_t x[4];
     uint64_t sum = 0;
@@ -667,8 +629,6 @@ __global__ void __launch_bounds__(1024) scan_items_local_kernel(uint64_t* __rest
         run += x[i];
     }
     if (threadIdx.x == 1023) chunks[c] = ws[31];
-    __syncthreads();  // ws read by every thread before the next chunk rewrites it
-    }
 }
 
 // Exclusive scan of the chunk sums (chunks[nc] = grand total), then each
@@ -676,13 +636,8 @@ __global__ void __launch_bounds__(1024) scan_items_local_kernel(uint64_t* __rest
 __global__ void __launch_bounds__(1024) scan_items_top_kernel(uint64_t* __restrict__ chunks, uint64_t nc,
                                                              const uint64_t* __restrict__ v, uint64_t n,
                                                              const uint64_t* __restrict__ item0, uint32_t nt,
-                                                             uint64_t* __restrict__ totals, const RunState* dyn) {
+                                                             uint64_t* __restrict__ totals) {
     __shared__ uint64_t ws[32];
-    if (dyn) {
-        n = dyn->ni;
-        nc = (n + kScanChunk - 1) / kScanChunk;
-        nt = dyn->nt;
-    }
     __shared__ uint64_t carry_s;
     if (threadIdx.x == 0) carry_s = 0;
     __syncthreads();
@@ -741,11 +696,11 @@ round_write_kernel(RoundArgs a) {
     uint64_t begin, end;
     uint32_t cur = 0;    // light class: buffer of the current item
     bool ready = false;  // light class: the current item's rows were issued with the previous item
-    const Span sp = launch_span<true>(a, FUSED);
+    const Span sp{a.item_base, a.n_items, a.queue, gridDim.x * kRoundWarps};
     while (next_chunk(sp, begin, end)) {
         for (uint64_t wi = sp.base + begin; wi < sp.base + end; ++wi) {
             if (wi >= w_hi || wi < w_lo) {
-                const uint32_t slot = find_slot(a.witem0, sp.nt + 1, wi);
+                const uint32_t slot = find_slot(a.witem0, a.nt + 1, wi);
                 w_lo = __ldg(a.witem0 + slot);
                 w_hi = __ldg(a.witem0 + slot + 1);
                 t = __ldg(a.wtask + slot);
@@ -760,8 +715,8 @@ round_write_kernel(RoundArgs a) {
             }
             const uint64_t item = t_item0 + (wi - w_lo);
             const uint64_t off = a.items[item] + a.chunks[item >> kScanChunkLog2];
-            const uint64_t off_next = item + 1 >= sp.n_count_items
-                                          ? a.chunks[sp.n_chunks]
+            const uint64_t off_next = item + 1 >= a.n_count_items
+                                          ? a.chunks[a.n_chunks]
                                           : a.items[item + 1] + a.chunks[(item + 1) >> kScanChunkLog2];
             const uint64_t row0 = (wi - w_lo) * a.rows_per_item;
             const uint32_t nr = (uint32_t)umin64(a.rows_per_item, nrows - row0);
@@ -810,209 +765,465 @@ round_write_kernel(RoundArgs a) {
     }
 }
 
-// ------------------------------------------------- device-side planning ----
-// Rounds scheduled on the device (BatchSession::run_device).  Every task of
-// a round sits at the same trie depth (nothing is deferred or split), so a
-// round's tasks are the children of the previous round's writing tasks.
-// Per node: the children that can match, light class first, as a range of
-// the children array, and the words of one output row.
-struct NodeRun {
-    uint32_t child0;
-    uint16_t n_light, n_fused;
-    uint32_t out_w;  // EXT: width + 1; REDUCE: width
+// ---------------------------------------------------- rounds in one pass ----
+// A run in one wave (BatchSession::run_pages) walks every row's candidates
+// once: a row's count is not needed before its output is placed, because
+// output goes to pages.  A page holds up to one item's rows of one node; a
+// warp that extends a task's items fills a page after another (slots taken
+// from the round's scratch region by one atomic) and lists each with its rows'
+// place among the node's rows.  pass_plan_kernel then prefixes the nodes'
+// rows and the next round's items (the slices of every node's rows, once for
+// each of its children), and pass_pack_kernel moves the rows there: without
+// it the pages of a mining level were a fifth full (a task's last page on
+// every warp that worked on it), and every child paid for the empty rest.
+//
+// What bounds it: issue slots and the latency of row -> index record -> list,
+// per lane; the counted rounds paid both twice for every row under a node
+// with children (222 of 259 million rows of a 16,384-pattern list), read the
+// rows twice and needed two scans and the totals between the passes.
+// Measured per call, one B200, counted rounds before / one pass: 16,384
+// patterns on 20,000 graphs 12.5 / 9.9 ms, 1,501 texts on 5,003 graphs 2.88 /
+// 2.35 ms, 16 patterns 852 / 516 us (9 launches a round / 4).
+//
+// Pages and staged rows lie column by column (a page's columns are
+// out_page_rows apart), so that neighbouring lanes touch neighbouring words
+// of shared memory and every store of a column is contiguous without an
+// index division.
+// State of one round in one pass: its items, its work-queue heads and the
+// page slots that its output has taken.
+struct PassState {
+    unsigned long long heads[2];  // light class, fused class
+    unsigned long long slots;
+    uint64_t ni, ni_light;        // items: all, light class (the light class's items come first)
+    uint32_t overflow;            // a region was too small: no later round finds work
     uint32_t pad;
 };
 
-struct PlanArgs {
-    RunState* st;              // this round
-    RunState* nx;              // the next round
-    const TaskRef* refs;       // this round's tasks (light class first)
-    const uint64_t* item0;     // [nt + 1] this round's count-pass item prefix
-    const uint64_t* totals;    // [nt] output rows per task
-    const NodeRun* info;
-    const uint32_t* children;
-    uint64_t* node_total;      // output rows per node (zeroed before the run)
-    uint32_t* region;          // this round's output frontier region
-    uint64_t region_words;
-    uint32_t** outs;           // [nt] output base per task (null: not written)
-    uint32_t* wtask;           // [nw] count-task index of each writing task
-    uint64_t* witem0;          // [nw + 1] item prefix over the writing tasks
-    TaskRef* next_refs;        // the next round's tasks
-    uint64_t* next_item0;      // [next nt + 1]
-    uint32_t refs_cap;         // capacity of next_refs
-    uint64_t items_cap;        // capacity of the per-item arrays
-    uint32_t rows_next;        // rows per item of the next round
-    uint32_t* overflow;        // set (never cleared) when a capacity is exceeded
-    uint64_t* bsum;            // [(nb + 1) * kPlanVals] per-block sums, then their exclusive scan and the totals
-    uint32_t nb;               // blocks of kPlanThreads tasks covering refs_cap
+struct PassArgs {
+    const TaskDesc* nodes;
+    const uint2* tasks;          // the round's tasks (node, its parent), light class first
+    const uint64_t* item0;       // [nt + 1] item prefix
+    const TaskRef* seeds;        // first round: the tasks' seed lists (null: pages)
+    const uint32_t* page_base;   // per node: its first page in in_region
+    const uint32_t* in_region;   // packed pages
+    uint32_t* out_region;        // scratch pages
+    uint32_t in_page_words, out_page_words;
+    uint32_t out_page_rows;
+    uint32_t slot_cap;           // slots of either region
+    uint32_t nt;
+    uint32_t rows_per_item;      // rows of an input page; of a slice of a seed list
+    uint32_t hub;
+    uint32_t kmax;
+    uint4* rec;                  // per slot written: (node, place among the node's rows, rows, width)
+    uint32_t* node_rows;         // per node: rows written
+    unsigned long long* node_total;  // per node: rows
+    PassState* st;
+    BatchCtx ctx;
 };
 
-constexpr int kPlanThreads = 512;
-constexpr int kPlanVals = 8;
 
-// Task t's contributions: 0 output words (rounded up to 16 bytes), 1 writes,
-// 2 write items, 3 write items of the light class, 4 / 5 light / fused child
-// tasks, 6 / 7 their items.  A task writes when it has output rows and a
-// child that can match.
-__device__ __forceinline__ void plan_values(const PlanArgs& p, uint32_t nt_light, uint32_t t, uint64_t v[kPlanVals],
-                                            uint32_t& node, uint64_t& tot, uint64_t& per) {
-    node = p.refs[t].node;
-    tot = p.totals[t];
-    const NodeRun nr = p.info[node];
-    const bool w = tot > 0 && nr.n_light + nr.n_fused > 0;
-    per = w ? (tot + p.rows_next - 1) / p.rows_next : 0;
-    const uint64_t items = p.item0[t + 1] - p.item0[t];
-    v[0] = w ? ((tot * nr.out_w + 3) & ~3ull) : 0;
-    v[1] = w ? 1 : 0;
-    v[2] = w ? items : 0;
-    v[3] = w && t < nt_light ? items : 0;
-    v[4] = w ? nr.n_light : 0;
-    v[5] = w ? nr.n_fused : 0;
-    v[6] = per * nr.n_light;
-    v[7] = per * nr.n_fused;
-}
+// A staged row: column c lies `stride` words after column c - 1.
+struct Col {
+    const uint32_t* p;
+    uint32_t stride;
+    __device__ __forceinline__ uint32_t operator[](uint32_t c) const { return p[c * stride]; }
+};
 
-// Exclusive block scan of kPlanVals values per thread; sum receives the
-// block totals.
-__device__ __forceinline__ void plan_scan(const uint64_t v[kPlanVals], uint64_t ex[kPlanVals], uint64_t sum[kPlanVals],
-                                          uint64_t (*sh)[kPlanVals]) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    constexpr int W = kPlanThreads / 32;
-    uint64_t inc[kPlanVals];
-#pragma unroll
-    for (int k = 0; k < kPlanVals; ++k) {
-        inc[k] = v[k];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint64_t y = __shfl_up_sync(0xffffffffu, inc[k], o);
-            if (lane >= o) inc[k] += y;
-        }
+constexpr uint32_t kNoPage = 0xffffffffu, kLostPage = 0xfffffffeu;
+
+// Where a warp's output of one node goes: the open page and its rows.
+struct Pages {
+    uint32_t slot = kNoPage, fill = 0, width = 0;
+
+    // Lists the open page among the node's rows.
+    __device__ __forceinline__ void close(const PassArgs& a, uint32_t node) {
+        if (slot < kLostPage && (threadIdx.x & 31) == 0)
+            a.rec[slot] = make_uint4(node, atomicAdd(a.node_rows + node, fill), fill, width);
+        slot = kNoPage;
+        fill = 0;
     }
-    if (lane == 31)
-        for (int k = 0; k < kPlanVals; ++k) sh[wid][k] = inc[k];
-    __syncthreads();
-    if (wid == 0) {
-#pragma unroll
-        for (int k = 0; k < kPlanVals; ++k) {
-            uint64_t w = lane < W ? sh[lane][k] : 0;
+    __device__ __forceinline__ void open(const PassArgs& a) {
+        uint32_t s = 0;
+        if ((threadIdx.x & 31) == 0) {
+            const unsigned long long got = atomicAdd(&a.st->slots, 1ull);
+            s = got < a.slot_cap ? (uint32_t)got : kLostPage;  // lost: the run starts over
+        }
+        slot = __shfl_sync(0xffffffffu, s, 0);
+    }
+    // Row rr of the staged rows (k columns), extended by c (`extend`), of
+    // every lane with `take`, in lane order.  Returns their number.
+    __device__ __forceinline__ uint32_t put(const PassArgs& a, uint32_t node, bool take, const uint32_t* rows_s,
+                                            uint32_t k, bool extend, uint32_t rr, uint32_t c) {
+        const uint32_t m = __ballot_sync(0xffffffffu, take), n = __popc(m), cap = a.out_page_rows;
+        if (n == 0) return 0;
+        if (slot == kNoPage) open(a);
+        uint32_t at = fill + __popc(m & ((1u << (threadIdx.x & 31)) - 1u));
+        auto store = [&]() {
+            uint32_t* out = a.out_region + ((uint64_t)slot * a.out_page_words + at);
+            for (uint32_t j = 0; j < k; ++j) out[j * cap] = rows_s[j * a.rows_per_item + rr];
+            if (extend) out[k * cap] = c;
+        };
+        if (take && at < cap && slot != kLostPage) store();
+        fill += n;
+        if (fill >= cap) {
+            const uint32_t rest = fill - cap;
+            fill = cap;
+            close(a, node);
+            if (rest) {
+                open(a);
+                if (take && at >= cap && slot != kLostPage) {
+                    at -= cap;
+                    store();
+                }
+                fill = rest;
+            }
+        }
+        return n;
+    }
+};
+
+// One page or slice of an extension: 32 rows at a time, their candidate lists
+// end to end are dealt out to the lanes 32 candidates per step, whatever
+// their lengths: rows of a small graph have about one candidate each and up
+// to six (a lane per row left two thirds of the lanes idle), a hub has
+// thousands (they are read as consecutive words).  FEEDS: accepted rows go
+// to the node's pages; else (fused class only) they are counted.
+template <bool FEEDS, bool FUSED>
+__device__ __forceinline__ uint64_t pass_extend(const PassArgs& a, const TaskDesc& d, uint32_t node,
+                                                const uint32_t* rows_s, uint32_t nr, GenState* gen_s, Pages& pg) {
+    const ExtArgs& p = d.e;
+    const uint32_t lane = threadIdx.x & 31, R = a.rows_per_item;
+    const bool graphs = d.mode == MODE_COUNT_GRAPHS || d.mode == MODE_WRITE_AND_GRAPHS;
+    uint64_t total = 0;
+    for (uint32_t base = 0; base < nr; base += 32) {
+        uint32_t lo = 0, hi = 0;
+        if (base + lane < nr) {
+            if (FUSED) {
+                ext_generator(p, Col{rows_s + base + lane, R}, gen_s[lane]);
+                lo = gen_s[lane].lo;
+                hi = gen_s[lane].hi;
+            } else {
+                seg_of(p.off, p.L, rows_s[p.src_col * R + base + lane], p.lab, lo, hi);
+            }
+        }
+        const uint32_t mine = hi > lo ? hi - lo : 0;
+        if (FUSED) __syncwarp();  // generator states written before other lanes read them
+        // lists so long that their sum might not fit a word: one row at a time
+        const bool huge = __any_sync(0xffffffffu, mine > (1u << 26));
+        for (uint32_t h = 0; h < (huge ? 32u : 1u); ++h) {
+            const uint32_t len = huge && lane != h ? 0 : mine;
+            uint32_t inc = len;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const uint64_t y = __shfl_up_sync(0xffffffffu, w, o);
-                if (lane >= o) w += y;
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= (uint32_t)o) inc += y;
             }
-            if (lane < W) sh[lane][k] = w;
+            const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
+            const uint32_t shift = lo - (inc - len);  // list position of candidate x: shift + x
+            for (uint32_t x0 = 0; x0 < all; x0 += 32) {
+                const uint32_t x = x0 + lane;
+                uint32_t q = 0;  // the row of candidate x: rows whose lists end at or before it
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    const uint32_t e = __shfl_sync(0xffffffffu, inc, q + o - 1);
+                    if (e <= x) q += o;
+                }
+                const uint32_t at = __shfl_sync(0xffffffffu, shift, q) + x;
+                bool ok = x < all;
+                uint32_t c = 0;
+                const Col row{rows_s + base + q, R};
+                if (ok) {
+                    if (FUSED) {
+                        c = __ldg(gen_s[q].gadj + at);
+                        ok = ext_accept(p, row, c, gen_s[q]);
+                    } else {
+                        c = __ldg(p.adj + at);
+                        if (p.bound_col >= 0) {
+                            const uint32_t b = row[p.bound_col];
+                            ok = p.bound_incl ? c <= b : c < b;
+                        }
+                        for (uint32_t e = 0; e < p.n_eq; ++e) ok &= row[p.eq_cols[e]] != c;
+                    }
+                }
+                if (FEEDS)
+                    total += pg.put(a, node, ok, rows_s, p.k, true, base + q, c);
+                else
+                    total += __popc(__ballot_sync(0xffffffffu, ok));
+                if (graphs) add_graph_count(a.ctx, d.query, row[0], ok ? 1u : 0u, true);
+            }
+        }
+        if (FUSED) __syncwarp();  // every lane done with the states before the next rows overwrite them
+    }
+    return total;
+}
+
+// The same for a plain extension that nothing follows: a lane counts its row.
+__device__ __forceinline__ uint64_t pass_count(const PassArgs& a, const TaskDesc& d, const uint32_t* rows_s,
+                                               uint32_t nr) {
+    const uint32_t lane = threadIdx.x & 31, R = a.rows_per_item;
+    const bool graphs = d.mode == MODE_COUNT_GRAPHS;
+    uint64_t total = 0;
+    for (uint32_t base = 0; base < nr; base += 32) {
+        const bool valid = base + lane < nr;
+        const Col row{rows_s + (valid ? base + lane : 0), R};
+        uint32_t cnt = 0;
+        if (valid) cnt = ext_count_plain(d.e, row);
+        if (graphs) add_graph_count(a.ctx, d.query, row[0], cnt, valid);
+        total += cnt;
+    }
+    return __shfl_sync(0xffffffffu, warp_sum(total), 0);
+}
+
+__device__ __forceinline__ uint64_t pass_reduce(const PassArgs& a, const TaskDesc& d, uint32_t node,
+                                                const uint32_t* rows_s, uint32_t nr, Pages& pg) {
+    const uint32_t lane = threadIdx.x & 31, R = a.rows_per_item;
+    const bool graphs = d.mode == MODE_COUNT_GRAPHS || d.mode == MODE_WRITE_AND_GRAPHS;
+    uint64_t total = 0;
+    for (uint32_t base = 0; base < nr; base += 32) {
+        const bool valid = base + lane < nr;
+        const Col row{rows_s + (valid ? base + lane : 0), R};
+        const bool keep = valid && red_keep_row(d.r, row);
+        if (d.feeds)
+            total += pg.put(a, node, keep, rows_s, d.r.k, false, base + lane, 0u);
+        else
+            total += __popc(__ballot_sync(0xffffffffu, keep));
+        if (graphs) add_graph_count(a.ctx, d.query, row[0], keep ? 1u : 0u, valid);
+    }
+    return total;
+}
+
+// Issues, without waiting, the copy of an item's rows into shared memory,
+// column by column: a page (k columns R apart, nr rows each) or a slice of a
+// seed list (one column); each lane commits one group.
+__device__ __forceinline__ void stage_page(uint32_t* rows_s, const uint32_t* __restrict__ src, uint32_t nr, uint32_t k,
+                                           uint32_t R, bool seeds) {
+    const uint32_t lane = threadIdx.x & 31;
+    if (seeds) {
+        for (uint32_t w = lane; w < nr; w += 32) cp_async4(rows_s + w, src + w);
+    } else {
+        const uint32_t words = k * R;
+        for (uint32_t w = 4 * lane; w < words; w += 128)
+            if ((w & (R - 1)) < nr) cp_async16(rows_s + w, src + w);  // R is a power of two
+    }
+    cp_async_commit();
+}
+
+// Shared memory of one warp: descriptor, row buffers, generator states.
+size_t pass_smem_bytes(uint32_t rows_per_item, uint32_t kmax, bool fused) {
+    return (size_t)kRoundWarps *
+           (sizeof(TaskDesc) + (fused ? kGenBytes : 0) + 4 * round_warp_words(rows_per_item, kmax, false, fused));
+}
+
+template <bool FUSED>
+__global__ void __launch_bounds__(kRoundWarps * 32, FUSED ? 4 : 6)
+round_pass_kernel(const __grid_constant__ PassArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    // the light class's launch may start on the SMs that this one no longer
+    // fills; it waits for this one before it ends (below)
+    if (FUSED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t lane = threadIdx.x & 31, R = a.rows_per_item;
+    const WarpSmem ws = warp_smem<false, FUSED>(smem_raw, a);
+    TaskDesc& d = *ws.d;
+    uint64_t t_lo = 0, t_hi = 0, begin, end, total = 0;
+    const uint32_t* in = nullptr;     // first round: the task's seed list; later: its parent's pages
+    uint64_t nrows = 0;
+    uint32_t node = 0, k = 0, cur = 0;
+    bool ready = false;               // light class: the current item's rows were issued with the previous item
+    Pages pg;
+    const uint64_t light = a.st->ni_light;
+    const Span sp{FUSED ? light : 0, FUSED ? a.st->ni - light : light, a.st->heads + (FUSED ? 1 : 0),
+                  gridDim.x * kRoundWarps};
+    auto task_done = [&]() {
+        pg.close(a, node);
+        if (lane == 0 && total) atomicAdd(a.node_total + node, (unsigned long long)total);
+        total = 0;
+    };
+    // the task's item i
+    const uint32_t words = a.seeds ? R : a.in_page_words;
+    auto stage = [&](uint32_t* rows_s, uint64_t i) {
+        stage_page(rows_s, in + i * words, (uint32_t)umin64(R, nrows - i * R), k, R, a.seeds != nullptr);
+    };
+    while (next_chunk(sp, begin, end)) {
+        const uint64_t stop = sp.base + end;
+        for (uint64_t item = sp.base + begin; item < stop; ++item) {
+            if (item >= t_hi || item < t_lo) {
+                task_done();
+                const uint32_t t = find_slot(a.item0, a.nt + 1, item);
+                t_lo = __ldg(a.item0 + t);
+                t_hi = __ldg(a.item0 + t + 1);
+                const uint2 task = __ldg(a.tasks + t);
+                if (a.seeds) {
+                    in = a.seeds[t].in;
+                    nrows = a.seeds[t].nrows;
+                } else {
+                    in = a.in_region + (uint64_t)a.page_base[task.y] * words;
+                    nrows = a.node_rows[task.y];
+                }
+                __syncwarp();
+                load_desc(d, a.nodes + task.x);
+                node = task.x;
+                k = d.kind == STEP_EXT ? d.e.k : d.r.k;
+                pg.width = d.kind == STEP_EXT ? k + 1 : k;
+            }
+            const uint64_t i = item - t_lo;
+            const uint32_t nr = (uint32_t)umin64(R, nrows - i * R);
+            uint32_t* rows = ws.rows;
+            if (FUSED) {
+                __syncwarp();
+                stage(rows, i);
+                cp_async_wait_all();
+            } else {
+                rows = cur ? ws.rows2 : ws.rows;
+                if (!ready) {
+                    __syncwarp();
+                    stage(rows, i);
+                }
+                // the next item of the same task and chunk: its rows are copied in meanwhile
+                ready = item + 1 < stop && item + 1 < t_hi;
+                if (ready) {
+                    stage(cur ? ws.rows : ws.rows2, i + 1);
+                    cp_async_wait_one();
+                } else {
+                    cp_async_wait_all();
+                }
+                cur ^= 1;
+            }
+            __syncwarp();
+            if (FUSED)
+                total += d.feeds ? pass_extend<true, true>(a, d, node, rows, nr, ws.gen, pg)
+                                 : pass_extend<false, true>(a, d, node, rows, nr, ws.gen, pg);
+            else if (d.kind != STEP_EXT)
+                total += pass_reduce(a, d, node, rows, nr, pg);
+            else
+                total += d.feeds ? pass_extend<true, false>(a, d, node, rows, nr, nullptr, pg)
+                                 : pass_count(a, d, rows, nr);
+            __syncwarp();  // every lane done with these rows before the buffer is refilled
         }
     }
+    task_done();
+    if (!FUSED) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Planning of the next round, by one cluster: the finished round's nodes get
+// their packed pages (a prefix over their rows) and the next round's tasks
+// their items (a task has its parent's pages).  A cluster's CTAs exchange
+// their sums through distributed shared memory, so a round of 10,000 tasks is
+// planned in one launch.
+constexpr int kPlanCtas = 8, kPlanThreads = 1024;
+struct PlanArgs {
+    PassState* st;             // the finished round
+    PassState* nx;             // the next round
+    const uint2* done;         // tasks of the finished round
+    const uint2* next;         // tasks of the next round, light class first
+    uint32_t n_done, n_next, n_next_light;
+    uint32_t slot_cap;
+    uint32_t page_rows;
+    uint32_t page_words;
+    const uint32_t* node_rows;
+    uint32_t* page_base;
+    uint64_t* item0;           // [n_next + 1]
+    const uint4* rec;
+    const uint32_t* scratch;
+    uint32_t* packed;
+    uint32_t* overflow;        // set (never cleared) when a region was too small
+};
+
+// Exclusive scan over the cluster of one value per thread; `sum` receives the
+// grand total.
+__device__ __forceinline__ uint64_t cluster_scan(uint64_t v, uint64_t& sum) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    __shared__ uint64_t ws[32];
+    __shared__ uint64_t mine;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint64_t inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    if (lane == 31) ws[wid] = inc;
     __syncthreads();
+    if (wid == 0) {
+        uint64_t w = ws[lane];
 #pragma unroll
-    for (int k = 0; k < kPlanVals; ++k) {
-        ex[k] = (wid > 0 ? sh[wid - 1][k] : 0) + inc[k] - v[k];
-        sum[k] = sh[W - 1][k];
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t y = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += y;
+        }
+        ws[lane] = w;
+        if (lane == 31) mine = w;
     }
-    __syncthreads();  // sh read by every thread before the next scan rewrites it
+    cl.sync();
+    uint64_t before = (wid > 0 ? ws[wid - 1] : 0) + inc - v;
+    sum = 0;
+    for (uint32_t r = 0; r < kPlanCtas; ++r) {
+        const uint64_t x = *cl.map_shared_rank(&mine, r);
+        if (r < cl.block_rank()) before += x;
+        sum += x;
+    }
+    cl.sync();  // sums read before the next scan (or the kernel's end) replaces them
+    return before;
 }
 
-// Planning of one round in three launches over blocks of kPlanThreads
-// tasks: the blocks' sums (plan_sum_kernel), their exclusive scan and the
-// round's totals (plan_top_kernel, one block), then every task's places
-// (plan_write_kernel): each task's output rows are recorded (node_total),
-// the writing tasks' outputs placed in the round's region and listed for the
-// write pass, and the next round's tasks (their children, light class first)
-// listed with their item prefix.  A region, task or item capacity exceeded
-// marks the run overflowed: no later launch of the run finds work, and the
-// host runs the session's rounds itself.
-__global__ void __launch_bounds__(kPlanThreads) plan_sum_kernel(PlanArgs p) {
-    __shared__ uint64_t sh[kPlanThreads / 32][kPlanVals];
-    const RunState& st = *p.st;
-    const uint32_t nt = st.overflow ? 0u : st.nt;
-    const uint32_t t = blockIdx.x * kPlanThreads + threadIdx.x;
-    uint64_t v[kPlanVals] = {}, ex[kPlanVals], sum[kPlanVals];
-    uint32_t node;
-    uint64_t tot, per;
-    if (t < nt) plan_values(p, st.nt_light, t, v, node, tot, per);
-    plan_scan(v, ex, sum, sh);
-    if (threadIdx.x < kPlanVals) p.bsum[(size_t)blockIdx.x * kPlanVals + threadIdx.x] = sum[threadIdx.x];
-}
-
-__global__ void __launch_bounds__(kPlanThreads) plan_top_kernel(PlanArgs p) {
-    __shared__ uint64_t sh[kPlanThreads / 32][kPlanVals];
-    RunState& st = *p.st;
-    RunState& nx = *p.nx;
-    uint64_t v[kPlanVals], ex[kPlanVals], sum[kPlanVals], carry[kPlanVals] = {};
-    for (uint32_t base = 0; base < p.nb; base += kPlanThreads) {
-        const uint32_t b = base + threadIdx.x;
-#pragma unroll
-        for (int k = 0; k < kPlanVals; ++k) v[k] = b < p.nb ? p.bsum[(size_t)b * kPlanVals + k] : 0;
-        plan_scan(v, ex, sum, sh);
-        if (b < p.nb)
-#pragma unroll
-            for (int k = 0; k < kPlanVals; ++k) p.bsum[(size_t)b * kPlanVals + k] = carry[k] + ex[k];
-#pragma unroll
-        for (int k = 0; k < kPlanVals; ++k) carry[k] += sum[k];
-    }
-    if (threadIdx.x == 0) {
-        const uint64_t* tot = carry;
-        const bool bad = st.overflow || tot[0] > p.region_words || tot[4] + tot[5] > p.refs_cap ||
-                         tot[6] + tot[7] > p.items_cap;
-        if (bad) {
-            st.overflow = 1;
-            st.nw = 0;
-            st.wi = st.wi_light = 0;
-            nx.overflow = 1;
-            nx.nt = nx.nt_light = 0;
-            nx.ni = nx.ni_light = 0;
+__global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanThreads) pass_plan_kernel(PlanArgs p) {
+    constexpr uint32_t kAll = kPlanCtas * kPlanThreads;
+    const uint32_t me = blockIdx.x * kPlanThreads + threadIdx.x;
+    const bool lost = p.st->overflow || p.st->slots > p.slot_cap;  // the same in every CTA
+    if (lost) {
+        if (me == 0) {
+            p.nx->overflow = 1;
             *p.overflow = 1;
-        } else {
-            st.nw = (uint32_t)tot[1];
-            st.wi = tot[2];
-            st.wi_light = tot[3];
-            nx.nt = (uint32_t)(tot[4] + tot[5]);
-            nx.nt_light = (uint32_t)tot[4];
-            nx.ni = tot[6] + tot[7];
-            nx.ni_light = tot[6];
-            p.witem0[tot[1]] = tot[2];
-            p.next_item0[tot[4] + tot[5]] = tot[6] + tot[7];
         }
-#pragma unroll
-        for (int k = 0; k < kPlanVals; ++k) p.bsum[(size_t)p.nb * kPlanVals + k] = tot[k];
+        return;
+    }
+    auto pages = [&](uint32_t node) { return (p.node_rows[node] + p.page_rows - 1) / p.page_rows; };
+    uint64_t sum;
+    {
+        const uint32_t per = (p.n_done + kAll - 1) / kAll;
+        const uint32_t b = min(p.n_done, me * per), e = min(p.n_done, b + per);
+        uint64_t v = 0;
+        for (uint32_t t = b; t < e; ++t) v += pages(p.done[t].x);
+        uint64_t at = cluster_scan(v, sum);
+        for (uint32_t t = b; t < e; ++t) {
+            const uint32_t node = p.done[t].x;
+            p.page_base[node] = (uint32_t)at;
+            at += pages(node);
+        }
+    }
+    const uint32_t per = (p.n_next + kAll - 1) / kAll;
+    const uint32_t b = min(p.n_next, me * per), e = min(p.n_next, b + per);
+    uint64_t v = 0;
+    for (uint32_t t = b; t < e; ++t) v += pages(p.next[t].y);
+    uint64_t at = cluster_scan(v, sum);
+    if (me == 0) {
+        p.item0[p.n_next] = sum;
+        p.nx->ni = sum;
+        if (p.n_next_light == p.n_next) p.nx->ni_light = sum;
+    }
+    for (uint32_t t = b; t < e; ++t) {
+        p.item0[t] = at;
+        if (t == p.n_next_light) p.nx->ni_light = at;
+        at += pages(p.next[t].y);
     }
 }
 
-__global__ void __launch_bounds__(kPlanThreads) plan_write_kernel(PlanArgs p) {
-    __shared__ uint64_t sh[kPlanThreads / 32][kPlanVals];
-    const RunState& st = *p.st;
-    if (st.overflow) return;  // uniform: set before this launch
-    const uint32_t nt = st.nt;
-    const uint32_t t = blockIdx.x * kPlanThreads + threadIdx.x;
-    uint64_t v[kPlanVals] = {}, ex[kPlanVals], sum[kPlanVals];
-    uint32_t node = 0;
-    uint64_t tot = 0, per = 0;
-    if (t < nt) plan_values(p, st.nt_light, t, v, node, tot, per);
-    plan_scan(v, ex, sum, sh);
-    if (t >= nt) return;
-    const uint64_t* carry = p.bsum + (size_t)blockIdx.x * kPlanVals;
-    const uint64_t light_tasks = p.bsum[(size_t)p.nb * kPlanVals + 4];
-    const uint64_t light_items = p.bsum[(size_t)p.nb * kPlanVals + 6];
-    p.node_total[node] = tot;
-    uint32_t* out = nullptr;
-    if (v[1]) {
-        out = p.region + carry[0] + ex[0];
-        const uint64_t slot = carry[1] + ex[1];
-        p.wtask[slot] = t;
-        p.witem0[slot] = carry[2] + ex[2];
-        const NodeRun nr = p.info[node];
-        const uint64_t j0 = carry[4] + ex[4], i0 = carry[6] + ex[6];
-        for (uint32_t i = 0; i < nr.n_light; ++i) {
-            p.next_refs[j0 + i] = TaskRef{__ldg(p.children + nr.child0 + i), 0u, out, tot};
-            p.next_item0[j0 + i] = i0 + (uint64_t)i * per;
-        }
-        const uint64_t j1 = light_tasks + carry[5] + ex[5], i1 = light_items + carry[7] + ex[7];
-        for (uint32_t i = 0; i < nr.n_fused; ++i) {
-            p.next_refs[j1 + i] = TaskRef{__ldg(p.children + nr.child0 + nr.n_light + i), 0u, out, tot};
-            p.next_item0[j1 + i] = i1 + (uint64_t)i * per;
+// The scratch pages' rows to their places in the packed pages, a warp per
+// page.  Bound by memory: every row is read and written once.
+__global__ void __launch_bounds__(256) pass_pack_kernel(PlanArgs p) {
+    if (p.nx->overflow) return;
+    const uint32_t lane = threadIdx.x & 31, R = p.page_rows, slots = (uint32_t)p.st->slots;
+    const uint32_t warps = gridDim.x * 8;
+    for (uint32_t s = blockIdx.x * 8 + (threadIdx.x >> 5); s < slots; s += warps) {
+        const uint4 r = __ldg(p.rec + s);
+        const uint32_t* src = p.scratch + (uint64_t)s * p.page_words;
+        const uint64_t first = (uint64_t)__ldg(p.page_base + r.x) * p.page_words;
+        for (uint32_t i = lane; i < r.z; i += 32) {
+            const uint32_t at = r.y + i, page = at / R;
+            uint32_t* dst = p.packed + first + (uint64_t)page * p.page_words + (at - page * R);
+            for (uint32_t c = 0; c < r.w; ++c) dst[c * R] = __ldg(src + c * R + i);
         }
     }
-    p.outs[t] = out;
 }
 
 std::atomic<uint64_t> g_batch_launches{0};
@@ -1158,6 +1369,8 @@ int BatchSession::init() {
         GVA_CUDA_B(cudaFuncSetAttribute(round_count_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
         GVA_CUDA_B(cudaFuncSetAttribute(round_write_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
         GVA_CUDA_B(cudaFuncSetAttribute(round_write_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        GVA_CUDA_B(cudaFuncSetAttribute(round_pass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        GVA_CUDA_B(cudaFuncSetAttribute(round_pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
         smem_set[dev].store(true, std::memory_order_release);
     }
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1269,6 +1482,7 @@ void BatchSession::fill_node_desc(int id, void* out) const {
     const Step& st = *node_steps[id];
     d.kind = st.kind;
     d.mode = nd.first_child < 0 ? MODE_COUNT : MODE_WRITE;
+    for (int c = nd.first_child; c >= 0 && !d.feeds; c = nodes[c].next_sibling) d.feeds = nodes[c].always_empty ? 0 : 1;
     if (per_graph && nd.first_term >= 0) {
         d.mode = nd.first_child < 0 ? MODE_COUNT_GRAPHS : MODE_WRITE_AND_GRAPHS;
         d.query = (uint32_t)plans[nd.first_term].slot;
@@ -1828,8 +2042,8 @@ int BatchSession::round() {
     }
     if (pf) pf->end(ev, K_EXT_COUNT, cbytes, s, crows);
     if (pf) pf->begin(K_SCAN, 16.0 * ni, s, ev);
-    scan_items_local_kernel<<<(unsigned)nc, 1024, 0, s>>>(d_items, ni, d_chunks, nullptr);
-    scan_items_top_kernel<<<1, 1024, 0, s>>>(d_chunks, nc, d_items, ni, d_item0, (uint32_t)nt, d_totals, nullptr);
+    scan_items_local_kernel<<<(unsigned)nc, 1024, 0, s>>>(d_items, ni, d_chunks);
+    scan_items_top_kernel<<<1, 1024, 0, s>>>(d_chunks, nc, d_items, ni, d_item0, (uint32_t)nt, d_totals);
     if (pf) pf->end(ev, K_SCAN, 16.0 * ni, s, (double)ni);
     launches += 2;
     g_batch_launches += 2;
@@ -2050,7 +2264,40 @@ static uint32_t resident_ctas(int device, const void* fn, size_t smem) {
     return n;
 }
 
-int BatchSession::run_device() {
+// The frontier regions come from a memory pool of their own, one per device:
+// allocations of one size leave it unfragmented (beside the sessions' small
+// ones the driver had to map gigabytes anew, 27 ms of a 120 ms mining run).
+// Freed memory stays in it for the next run; what is more than the regions of
+// two runs side by side at their first size (9 GiB) goes back to the driver
+// when a database is freed.
+static cudaMemPool_t round_pool(int device) {
+    static std::mutex mu;
+    static cudaMemPool_t pools[64] = {};
+    if (device < 0 || device >= 64) return nullptr;
+    std::lock_guard<std::mutex> lk(mu);
+    if (!pools[device]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t pool = nullptr;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        uint64_t keep = UINT64_MAX;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        pools[device] = pool;
+    }
+    return pools[device];
+}
+
+void trim_round_pool(int device) {
+    cudaMemPool_t pool = round_pool(device);
+    if (pool) cudaMemPoolTrimTo(pool, (size_t)9 << 30);
+}
+
+int BatchSession::run_pages() {
     if (host_rounds || profile || waves.size() != 1 || rounds != 0 || active.empty() || !db.seed_verts) return GVA_OK;
     const auto t_start = std::chrono::steady_clock::now();
     double wait_before = wait_ms;
@@ -2070,252 +2317,226 @@ int BatchSession::run_device() {
         phase_ms[k] += std::chrono::duration<double, std::milli>(now - t_lap).count();
         t_lap = now;
     };
+    auto wait = [&]() {
+        const auto w0 = std::chrono::steady_clock::now();
+        const cudaError_t e = cudaStreamSynchronize(s);
+        wait_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - w0).count();
+        return e;
+    };
     const size_t nn = nodes.size();
     for (const BTask& tk : active)
         if (nodes[tk.node].depth != 1) return GVA_OK;
     int D = 0;
     for (const BNode& nd : nodes) D = std::max(D, nd.depth);
     if (D < 1) return GVA_OK;
-    // per depth: widest input row, nodes, nodes of each class
-    std::vector<uint32_t> kmax(D + 2, 1), at_depth(D + 2, 0), light_at(D + 2, 0), fused_at(D + 2, 0);
+    // the rounds' tasks: every node that can match, by depth, light class
+    // first; per depth the widest input and output row
+    std::vector<uint32_t> kmax(D + 2, 1), wmax(D + 2, 1), first(D + 2, 0), n_light(D + 2, 0);
     for (const BNode& nd : nodes) {
         kmax[nd.depth] = std::max(kmax[nd.depth], nd.width_in);
-        at_depth[nd.depth]++;
-        (nd.fused ? fused_at : light_at)[nd.depth]++;
+        if (nd.kind == STEP_SEED || nd.always_empty) continue;
+        wmax[nd.depth] = std::max(wmax[nd.depth], nd.kind == STEP_EXT ? nd.width_in + 1 : nd.width_in);
+        first[nd.depth + 1]++;
+        if (!nd.fused) n_light[nd.depth]++;
     }
-    uint32_t refs_cap = 1;
-    for (int d = 1; d <= D; ++d) refs_cap = std::max(refs_cap, at_depth[d]);
+    for (int d = 1; d <= D + 1; ++d) first[d] += first[d - 1];
+    const size_t n_tasks = first[D + 1];
+    if (n_tasks == 0) return GVA_OK;
+    uint32_t most = 1;
+    for (int d = 1; d <= D; ++d) most = std::max(most, first[d + 1] - first[d]);
+    // one upload: tasks | first round's seed lists and item prefix | its state
+    auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    const uint32_t n1 = first[2] - first[1];
+    const size_t o_tasks = 0, o_seeds = o_tasks + al(n_tasks * sizeof(uint2));
+    const size_t o_item1 = o_seeds + al((size_t)n1 * sizeof(TaskRef));
+    const size_t o_state = o_item1 + al(((size_t)n1 + 1) * 8);
+    const size_t up_bytes = o_state + al((D + 2) * sizeof(PassState));
+    const size_t o_ntot = up_bytes, o_nrows = o_ntot + al(nn * 8), o_flag = o_nrows + al(nn * 4);
+    const size_t o_base = o_flag + 256, o_item0 = o_base + al(nn * 4);
+    const size_t o_rec = o_item0 + al(((size_t)most + 1) * 8);
+    const size_t o_back = al(std::max(up_bytes, nn * 8 + 64));  // staging: a round's state read back (stepped)
+    char* h = staging.get(o_back + sizeof(PassState));
+    if (!h) return fail(GVA_ERR_NOMEM, "pinned staging allocation failed");
     std::vector<uint32_t> R(D + 2, 32);
-    for (int d = 1; d <= D; ++d)
+    for (int d = 1; d <= D; ++d) {
         R[d] = std::min<uint32_t>(tune.rows_per_item, std::max<uint32_t>(32, (768 / kmax[d]) & ~31u));
-    // children that can match, light class first: counted per node, placed
-    // by a prefix over the nodes, then listed (both passes on the host's
-    // cores, by ranges of nodes)
-    std::vector<NodeRun> info(nn);
-    const unsigned T = nn >= 8192 ? std::min<unsigned>(pool_width(), 32) : 1u;
-    std::atomic<bool> too_many{false};
-    pool_run(T, [&](unsigned t) {
-        for (size_t id = nn * t / T; id < nn * (t + 1) / T; ++id) {
+        if (R[d] == 96) R[d] = 64;  // a power of two (stage_page)
+    }
+    uint2* h_tasks = (uint2*)(h + o_tasks);
+    {
+        std::vector<uint32_t> at(2 * (D + 2));
+        for (int d = 1; d <= D; ++d) {
+            at[2 * d] = first[d];
+            at[2 * d + 1] = first[d] + n_light[d];
+        }
+        for (size_t id = 0; id < nn; ++id) {
             const BNode& nd = nodes[id];
-            NodeRun r{};
-            r.out_w = nd.kind == STEP_EXT ? nd.width_in + 1 : nd.width_in;
-            size_t cnt[2] = {0, 0};
-            for (int c = nd.first_child; c >= 0; c = nodes[c].next_sibling)
-                if (!nodes[c].always_empty) cnt[nodes[c].fused ? 1 : 0]++;
-            if (cnt[0] > 0xffff || cnt[1] > 0xffff) too_many = true;  // beyond the schedule's child counts
-            r.n_light = (uint16_t)cnt[0];
-            r.n_fused = (uint16_t)cnt[1];
-            info[id] = r;
+            if (nd.kind == STEP_SEED || nd.always_empty) continue;
+            h_tasks[at[2 * nd.depth + (nd.fused ? 1 : 0)]++] = make_uint2((uint32_t)id, (uint32_t)nd.parent);
         }
-    });
-    if (too_many) return GVA_OK;
-    uint32_t nk = 0;
-    for (size_t id = 0; id < nn; ++id) {
-        info[id].child0 = nk;
-        nk += info[id].n_light + info[id].n_fused;
-    }
-    std::vector<uint32_t> kids(nk);
-    pool_run(T, [&](unsigned t) {
-        for (size_t id = nn * t / T; id < nn * (t + 1) / T; ++id) {
-            uint32_t at[2] = {info[id].child0, info[id].child0 + info[id].n_light};
-            for (int c = nodes[id].first_child; c >= 0; c = nodes[c].next_sibling)
-                if (!nodes[c].always_empty) kids[at[nodes[c].fused ? 1 : 0]++] = (uint32_t)c;
+        TaskRef* seeds = (TaskRef*)(h + o_seeds);
+        uint64_t* item1 = (uint64_t*)(h + o_item1);
+        PassState* st = (PassState*)(h + o_state);
+        memset(st, 0, (D + 2) * sizeof(PassState));
+        uint64_t ni = 0;
+        for (uint32_t t = 0; t < n1; ++t) {
+            const Step& sd = *node_steps[h_tasks[first[1] + t].y];
+            const uint64_t rows = sd.always_empty ? 0 : db.seed_off[sd.label + 1] - db.seed_off[sd.label];
+            seeds[t] = TaskRef{h_tasks[first[1] + t].x, 0u, db.seed_verts + (rows ? db.seed_off[sd.label] : 0), rows};
+            if (t == n_light[1]) st[1].ni_light = ni;
+            item1[t] = ni;
+            ni += (rows + R[1] - 1) / R[1];
         }
-    });
-    // the first round's tasks (depth 1, from the seed lists), light class first
-    std::vector<TaskRef> r0;
-    r0.reserve(active.size());
-    uint32_t nt_light0 = 0;
-    for (uint32_t f = 0; f < 2; ++f) {
-        for (const BTask& tk : active) {
-            const BNode& nd = nodes[tk.node];
-            if (nd.always_empty || nd.fused != f || tk.rows == 0) continue;
-            r0.push_back(TaskRef{(uint32_t)tk.node, 0u, tk.in, tk.rows});
-        }
-        if (f == 0) nt_light0 = (uint32_t)r0.size();
+        item1[n1] = st[1].ni = ni;
+        if (n_light[1] == n1) st[1].ni_light = ni;
     }
-    std::vector<uint64_t> i0(r0.size() + 1, 0);
-    uint64_t ni_light0 = 0;
-    for (size_t t = 0; t < r0.size(); ++t) {
-        i0[t + 1] = i0[t] + (r0[t].nrows + R[1] - 1) / R[1];
-        if (t + 1 == nt_light0) ni_light0 = i0[t + 1];
-    }
-    // two frontier regions (a round writes one while its tasks read the other)
+    // two frontier regions (a round reads packed pages from one and writes
+    // scratch pages to the other, which are then packed into the first); rows
+    // of a page = rows of an item of the round that reads it
     uint64_t region = db.round_region_bytes.load();
     if (region == 0) region = 2ull << 30;
     if (2 * region > budget) return GVA_OK;
-    const uint64_t region_words = region / 4;
-    const uint64_t items_cap = std::max<uint64_t>(i0.back(), region_words / 64 + refs_cap) + 1;
-    const uint64_t chunks_cap = items_cap / kScanChunk + 2;
-    // one block for the schedule's small arrays
-    auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    const size_t o_state = 0;
-    const size_t o_refs0 = o_state + al((D + 2) * sizeof(RunState));
-    const size_t o_refs1 = o_refs0 + al((size_t)refs_cap * sizeof(TaskRef));
-    const size_t o_item00 = o_refs1 + al((size_t)refs_cap * sizeof(TaskRef));
-    const size_t o_item01 = o_item00 + al(((size_t)refs_cap + 1) * 8);
-    const size_t o_totals = o_item01 + al(((size_t)refs_cap + 1) * 8);
-    const size_t o_outs = o_totals + al((size_t)refs_cap * 8);
-    const size_t o_wtask = o_outs + al((size_t)refs_cap * 8);
-    const size_t o_witem0 = o_wtask + al((size_t)refs_cap * 4);
-    const size_t o_ntot = o_witem0 + al(((size_t)refs_cap + 1) * 8);
-    const size_t o_info = o_ntot + al(nn * 8);
-    const size_t o_kids = o_info + al(nn * sizeof(NodeRun));
-    const uint32_t nb = (refs_cap + kPlanThreads - 1) / kPlanThreads;
-    const size_t o_flag = o_kids + al(std::max<size_t>(kids.size(), 1) * 4);
-    const size_t o_bsum = o_flag + 256;
-    const size_t o_items = o_bsum + al(((size_t)nb + 1) * kPlanVals * 8);
-    const size_t o_chunks = o_items + al(items_cap * 8);
-    const size_t small_bytes = o_chunks + al((chunks_cap + 1) * 8);
+    uint64_t slot_most = 1;
+    auto page_words = [&](int d) { return (uint64_t)R[d + 1] * wmax[d]; };  // output of depth d
+    auto slot_cap = [&](int d) { return std::min<uint64_t>(region / 4 / page_words(d), (1ull << 32) / R[d + 1] - 2); };  // rows of a node: a word
+    for (int d = 1; d < D; ++d) slot_most = std::max(slot_most, slot_cap(d));
     {
         const int rc = ship_nodes();
         if (rc) return rc;
     }
     lap(0);
-    char* blk = nullptr;
-    void* reg[2] = {nullptr, nullptr};
-    if (cudaMallocAsync((void**)&blk, small_bytes, s) != cudaSuccess) {  // no room: host rounds
-        cudaGetLastError();
+    // one allocation, of nearly the same size in every run: regions, then the
+    // schedule's arrays
+    const size_t region_bytes = al(region);
+    const size_t unit = (size_t)256 << 20, blk_bytes = o_rec + al(slot_most * sizeof(uint4));
+    char* mem = nullptr;
+    cudaMemPool_t pool = round_pool(db.device);
+    if (!pool || cudaMallocFromPoolAsync((void**)&mem, 2 * region_bytes + (blk_bytes + unit - 1) / unit * unit, pool, s) !=
+                     cudaSuccess) {
+        cudaGetLastError();  // no room: counted rounds
         return GVA_OK;
     }
-    if (cudaMallocAsync(&reg[0], region, s) != cudaSuccess || cudaMallocAsync(&reg[1], region, s) != cudaSuccess) {
-        cudaGetLastError();
-        for (void* q : {(void*)blk, reg[0], reg[1]})
-            if (q) cudaFreeAsync(q, s);
-        return GVA_OK;
-    }
-    auto free_all = [&]() {
-        for (void* q : {(void*)blk, reg[0], reg[1]}) cudaFreeAsync(q, s);
-    };
-    RunState* states = (RunState*)(blk + o_state);
-    TaskRef* refs[2] = {(TaskRef*)(blk + o_refs0), (TaskRef*)(blk + o_refs1)};
-    uint64_t* item0[2] = {(uint64_t*)(blk + o_item00), (uint64_t*)(blk + o_item01)};
-    uint64_t* totals = (uint64_t*)(blk + o_totals);
-    uint32_t** outs = (uint32_t**)(blk + o_outs);
-    uint32_t* wtask = (uint32_t*)(blk + o_wtask);
-    uint64_t* witem0 = (uint64_t*)(blk + o_witem0);
-    uint64_t* ntot = (uint64_t*)(blk + o_ntot);
-    NodeRun* d_info = (NodeRun*)(blk + o_info);
-    uint32_t* d_kids = (uint32_t*)(blk + o_kids);
+    struct Free {
+        cudaStream_t s;
+        void* p;
+        ~Free() { cudaFreeAsync(p, s); }
+    } free_mem{s, mem};
+    uint32_t* const packed = (uint32_t*)mem;
+    uint32_t* const scratch = (uint32_t*)(mem + region_bytes);
+    char* const blk = mem + 2 * region_bytes;
+    PassState* states = (PassState*)(blk + o_state);
+    unsigned long long* ntot = (unsigned long long*)(blk + o_ntot);
     uint32_t* d_flag = (uint32_t*)(blk + o_flag);
-    uint64_t* items = (uint64_t*)(blk + o_items);
-    uint64_t* chunks = (uint64_t*)(blk + o_chunks);
-    RunState s1{};
-    s1.ni = i0.back();
-    s1.ni_light = ni_light0;
-    s1.nt = (uint32_t)r0.size();
-    s1.nt_light = nt_light0;
-    // pageable sources: each copy is complete when its call returns
-    GVA_CUDA_B(cudaMemsetAsync(blk + o_state, 0, (D + 2) * sizeof(RunState), s));
-    GVA_CUDA_B(cudaMemsetAsync(ntot, 0, nn * 8, s));
-    GVA_CUDA_B(cudaMemsetAsync(d_flag, 0, 4, s));
-    GVA_CUDA_B(cudaMemcpyAsync(states + 1, &s1, sizeof s1, cudaMemcpyHostToDevice, s));
-    GVA_CUDA_B(cudaMemcpyAsync(d_info, info.data(), nn * sizeof(NodeRun), cudaMemcpyHostToDevice, s));
-    if (!kids.empty()) GVA_CUDA_B(cudaMemcpyAsync(d_kids, kids.data(), kids.size() * 4, cudaMemcpyHostToDevice, s));
-    if (!r0.empty()) GVA_CUDA_B(cudaMemcpyAsync(refs[1], r0.data(), r0.size() * sizeof(TaskRef), cudaMemcpyHostToDevice, s));
-    GVA_CUDA_B(cudaMemcpyAsync(item0[1], i0.data(), i0.size() * 8, cudaMemcpyHostToDevice, s));
-
+    GVA_CUDA_B(cudaMemcpyAsync(blk, h, up_bytes, cudaMemcpyHostToDevice, s));
+    GVA_CUDA_B(cudaMemsetAsync(ntot, 0, o_base - o_ntot, s));  // totals, rows, flag
     BatchCtx ctx{};
     ctx.vgraph = db.vgraph;
     ctx.G = db.num_graphs;
     ctx.words = ctx_words;
     ctx.graph_counts = graph_counts_dev();
     ctx.graph_bits = graph_bits_dev();
-    auto grid = [&](const void* fn, size_t smem) -> uint32_t { return resident_ctas(db.device, fn, smem) * (uint32_t)sms; };
+    auto grid = [&](const void* fn, size_t smem, uint64_t items) -> uint32_t {
+        return (uint32_t)std::max<uint64_t>(
+            1, std::min<uint64_t>(resident_ctas(db.device, fn, smem) * (uint64_t)sms, (items + kRoundWarps - 1) / kRoundWarps));
+    };
     lap(1);
     uint64_t nl = 0;
-    for (int d = 1; d <= D; ++d) {
-        const int b = d & 1;
-        RoundArgs ra{};
-        ra.nodes = (const TaskDesc*)d_nodes;
-        ra.refs = refs[b];
-        ra.item0 = item0[b];
-        ra.rows_per_item = R[d];
-        ra.hub = tune.hub;
-        ra.kmax = kmax[d];
-        ra.items = items;
-        ra.ctx = ctx;
-        ra.dyn = states + d;
-        if (light_at[d]) {
-            const size_t smem = round_smem_bytes(R[d], kmax[d], false, false);
-            round_count_kernel<false><<<grid((const void*)round_count_kernel<false>, smem), kRoundWarps * 32, smem, s>>>(ra);
-            ++nl;
-        }
-        if (fused_at[d]) {
-            const size_t smem = round_smem_bytes(R[d], kmax[d], false, true);
-            round_count_kernel<true><<<grid((const void*)round_count_kernel<true>, smem), kRoundWarps * 32, smem, s>>>(ra);
-            ++nl;
-        }
-        scan_items_local_kernel<<<2 * sms, 1024, 0, s>>>(items, 0, chunks, states + d);
-        scan_items_top_kernel<<<1, 1024, 0, s>>>(chunks, 0, items, 0, item0[b], 0, totals, states + d);
-        PlanArgs pa{};
-        pa.st = states + d;
-        pa.nx = states + d + 1;
-        pa.refs = refs[b];
-        pa.item0 = item0[b];
-        pa.totals = totals;
-        pa.info = d_info;
-        pa.children = d_kids;
+    int done = 0;
+    // items of the coming round; of rounds launched ahead of their planning
+    // only whether there can be any
+    const uint64_t kMany = 1ull << 62;
+    uint64_t items_light = ((PassState*)(h + o_state))[1].ni_light;
+    uint64_t items_fused = ((PassState*)(h + o_state))[1].ni - items_light;
+    for (int d = 1; d <= D && items_light + items_fused; ++d) {
+        ++done;
+        const uint32_t nt = first[d + 1] - first[d];
+        PassArgs pa{};
+        pa.nodes = (const TaskDesc*)d_nodes;
+        pa.tasks = (const uint2*)(blk + o_tasks) + first[d];
+        pa.item0 = (const uint64_t*)(blk + (d == 1 ? o_item1 : o_item0));
+        pa.seeds = d == 1 ? (const TaskRef*)(blk + o_seeds) : nullptr;
+        pa.page_base = (const uint32_t*)(blk + o_base);
+        pa.in_region = packed;
+        pa.out_region = scratch;
+        pa.in_page_words = d > 1 ? (uint32_t)page_words(d - 1) : 0;
+        pa.out_page_words = (uint32_t)page_words(d);
+        pa.out_page_rows = R[d + 1];
+        pa.slot_cap = d < D ? (uint32_t)slot_cap(d) : 0;
+        pa.nt = nt;
+        pa.rows_per_item = R[d];
+        pa.hub = tune.hub;
+        pa.kmax = kmax[d];
+        pa.rec = (uint4*)(blk + o_rec);
+        pa.node_rows = (uint32_t*)(blk + o_nrows);
         pa.node_total = ntot;
-        pa.region = (uint32_t*)reg[b];
-        pa.region_words = region_words;
-        pa.outs = outs;
-        pa.wtask = wtask;
-        pa.witem0 = witem0;
-        pa.next_refs = refs[b ^ 1];
-        pa.next_item0 = item0[b ^ 1];
-        pa.refs_cap = refs_cap;
-        pa.items_cap = items_cap;
-        pa.rows_next = R[d + 1];
-        pa.overflow = d_flag;
-        pa.bsum = (uint64_t*)(blk + o_bsum);
-        pa.nb = nb;
-        plan_sum_kernel<<<nb, kPlanThreads, 0, s>>>(pa);
-        plan_top_kernel<<<1, kPlanThreads, 0, s>>>(pa);
-        plan_write_kernel<<<nb, kPlanThreads, 0, s>>>(pa);
-        nl += 5;
-        if (d < D) {  // the deepest round's tasks have no children
-            RoundArgs wa = ra;
-            wa.wtask = wtask;
-            wa.witem0 = witem0;
-            wa.chunks = chunks;
-            wa.task_out = outs;
-            if (light_at[d]) {
-                const size_t smem = round_smem_bytes(R[d], kmax[d], true, false);
-                round_write_kernel<false><<<grid((const void*)round_write_kernel<false>, smem), kRoundWarps * 32, smem, s>>>(wa);
-                ++nl;
-            }
-            if (fused_at[d]) {
-                const size_t smem = round_smem_bytes(R[d], kmax[d], true, true);
-                round_write_kernel<true><<<grid((const void*)round_write_kernel<true>, smem), kRoundWarps * 32, smem, s>>>(wa);
-                ++nl;
-            }
+        pa.st = states + d;
+        pa.ctx = ctx;
+        if (items_fused) {
+            const size_t smem = pass_smem_bytes(R[d], kmax[d], true);
+            round_pass_kernel<true><<<grid((const void*)round_pass_kernel<true>, smem, items_fused), kRoundWarps * 32, smem, s>>>(pa);
+            ++nl;
+        }
+        if (items_light) {
+            // after the fused class's launch of the same round it may start
+            // before that one's last items are done
+            const size_t smem = pass_smem_bytes(R[d], kmax[d], false);
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(grid((const void*)round_pass_kernel<false>, smem, items_light));
+            cfg.blockDim = dim3(kRoundWarps * 32);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = s;
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at.val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = &at;
+            cfg.numAttrs = items_fused ? 1 : 0;
+            GVA_CUDA_B(cudaLaunchKernelEx(&cfg, round_pass_kernel<false>, pa));
+            ++nl;
+        }
+        if (d == D) continue;  // the deepest round's tasks have no children
+        PlanArgs pl{};
+        pl.st = states + d;
+        pl.nx = states + d + 1;
+        pl.done = pa.tasks;
+        pl.next = pa.tasks + nt;
+        pl.n_done = nt;
+        pl.n_next = first[d + 2] - first[d + 1];
+        pl.n_next_light = n_light[d + 1];
+        pl.slot_cap = pa.slot_cap;
+        pl.page_rows = pa.out_page_rows;
+        pl.page_words = pa.out_page_words;
+        pl.node_rows = pa.node_rows;
+        pl.page_base = (uint32_t*)(blk + o_base);
+        pl.item0 = (uint64_t*)(blk + o_item0);
+        pl.rec = pa.rec;
+        pl.scratch = scratch;
+        pl.packed = packed;
+        pl.overflow = d_flag;
+        pass_plan_kernel<<<kPlanCtas, kPlanThreads, 0, s>>>(pl);
+        pass_pack_kernel<<<8 * sms, 256, 0, s>>>(pl);
+        nl += 2;
+        if (stepped) {
+            PassState* back = (PassState*)(h + o_back);
+            GVA_CUDA_B(cudaMemcpyAsync(back, states + d + 1, sizeof(PassState), cudaMemcpyDeviceToHost, s));
+            const cudaError_t e = wait();
+            if (e != cudaSuccess) return fail(GVA_ERR_CUDA, cudaGetErrorString(e));
+            items_light = back->overflow ? 0 : back->ni_light;
+            items_fused = back->overflow ? 0 : back->ni - back->ni_light;
+        } else {
+            items_light = n_light[d + 1] ? kMany : 0;
+            items_fused = pl.n_next > n_light[d + 1] ? kMany : 0;
         }
     }
     launches += nl;
-    lap(2);
     g_batch_launches += nl;
-    {
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) {
-            free_all();
-            return fail(GVA_ERR_CUDA, std::string("device-scheduled rounds: ") + cudaGetErrorString(e));
-        }
-    }
-    char* h = staging.get(nn * 8 + 16);
-    if (!h) {
-        free_all();
-        return fail(GVA_ERR_NOMEM, "pinned staging allocation failed");
-    }
+    lap(2);
+    GVA_CUDA_B(cudaGetLastError());
     uint64_t* h_tot = (uint64_t*)h;
     uint32_t* h_flag = (uint32_t*)(h + nn * 8);
     GVA_CUDA_B(cudaMemcpyAsync(h_tot, ntot, nn * 8, cudaMemcpyDeviceToHost, s));
     GVA_CUDA_B(cudaMemcpyAsync(h_flag, d_flag, 4, cudaMemcpyDeviceToHost, s));
-    free_all();
     {
-        const auto w0 = std::chrono::steady_clock::now();
-        const cudaError_t e = cudaStreamSynchronize(s);
-        wait_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - w0).count();
+        const cudaError_t e = wait();
         if (e != cudaSuccess) return fail(GVA_ERR_CUDA, cudaGetErrorString(e));
     }
     t_lap = std::chrono::steady_clock::now();
@@ -2325,7 +2546,7 @@ int BatchSession::run_device() {
     } lap_end{lap};
     if (*h_flag) {
         // a round outgrew a region: later runs get regions twice as large, and
-        // this one starts over with host-scheduled rounds
+        // this one starts over with counted rounds
         uint64_t cur = db.round_region_bytes.load();
         while (cur < 2 * region && !db.round_region_bytes.compare_exchange_weak(cur, 2 * region)) {
         }
@@ -2354,8 +2575,8 @@ int BatchSession::run_device() {
         nd.closed = true;
     }
     active.clear();
-    rounds += (uint64_t)D;
-    device_rounds += (uint64_t)D;
+    rounds += (uint64_t)done;
+    if (!stepped) device_rounds += (uint64_t)done;
     return GVA_OK;
 }
 
@@ -2430,7 +2651,7 @@ __global__ void slot_popcount_kernel(const uint32_t* __restrict__ bits, uint32_t
 
 int prepare_batch(DevDB& db, std::vector<std::vector<Step>>&& steps, cudaStream_t s, uint64_t budget,
                   bool per_graph, bool graph_counts, bool profile, PreparedBatch& out, bool presorted,
-                  bool host_rounds) {
+                  RoundsMode rounds, uint32_t pieces) {
     const auto t0 = std::chrono::steady_clock::now();
     GVA_CUDA_B(cudaSetDevice(db.device));
     out.nq = (int)steps.size();
@@ -2439,7 +2660,8 @@ int prepare_batch(DevDB& db, std::vector<std::vector<Step>>&& steps, cudaStream_
     out.ids.clear();
     if (out.nq == 0) return GVA_OK;
     out.ses.reset(new BatchSession(db, s, budget, per_graph ? (uint32_t)out.nq : 0, graph_counts, profile));
-    out.ses->host_rounds = host_rounds;
+    out.ses->host_rounds = rounds == ROUNDS_HOST;
+    out.ses->stepped = rounds == ROUNDS_AUTO && pieces > 1;
     int rc = out.ses->init();
     if (!rc) rc = out.ses->submit(std::move(steps), {}, &out.ids, presorted);
     out.prep_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -2469,7 +2691,7 @@ int finish_batch(DevDB& db, PreparedBatch& pb, uint64_t* counts, uint64_t* graph
     GVA_CUDA_B(cudaEventRecord(tev[dev][0], s));
     int rc = GVA_OK;
     const auto t_loop0 = std::chrono::steady_clock::now();
-    if (!(cancel && *cancel)) rc = ses.run_device();
+    if (!(cancel && *cancel)) rc = ses.run_pages();
     while (!rc && !ses.idle()) {
         if (cancel && *cancel) {
             rc = fail(GVA_ERR_CANCELLED, "cancelled");
@@ -2651,10 +2873,6 @@ int run_batch(DevDB& db, std::vector<std::vector<Step>> steps, cudaStream_t s, u
     // (a profiled run keeps one stream: per-kernel event timings of two
     // overlapping streams would each include the other's kernels)
     const size_t K = n >= 12288 && !profile ? 2 : 1;
-    // two halves hide each other's host round trips: host scheduling there
-    // (no schedule tables or frontier regions per half; the two measure
-    // alike), device scheduling for a run in one piece
-    const bool host_rounds = rounds == ROUNDS_HOST || (rounds == ROUNDS_AUTO && K == 2);
     std::vector<size_t> cut(K + 1);
     for (size_t k = 0; k <= K; ++k) cut[k] = n * k / K;
     const bool per_graph = graph_counts_host || support_host;
@@ -2672,7 +2890,7 @@ int run_batch(DevDB& db, std::vector<std::vector<Step>> steps, cudaStream_t s, u
         std::vector<std::vector<Step>> part(cut[k + 1] - cut[k]);
         for (size_t j = 0; j < part.size(); ++j) part[j] = std::move(steps[order[cut[k] + j]]);
         int r = prepare_batch(db, std::move(part), streams[k], budget, per_graph, graph_counts_host != nullptr,
-                              profile, pb, true, host_rounds);
+                              profile, pb, true, (RoundsMode)rounds, (uint32_t)K);
         const double t_prep = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         // results straight to the caller's arrays, at each plan's index before sorting
         if (!r) r = finish_batch(db, pb, counts, graph_counts_host, support_host, &bss[k], nullptr, order.data() + cut[k]);

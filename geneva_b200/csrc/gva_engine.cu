@@ -456,7 +456,10 @@ int upload_graph(HostGraph& g, int device, DevDB*& out) {
 void free_devdb(DevDB* db) {
     if (!db) return;
     if (db->arena || db->vgraph) cudaSetDevice(db->device);
-    if (db->arena) cudaFree(db->arena);
+    if (db->arena) {
+        cudaFree(db->arena);
+        trim_round_pool(db->device);
+    }
     if (db->vgraph) cudaFree(db->vgraph);
     delete db;
 }

@@ -44,7 +44,7 @@ struct DevDB {
     // frontier budget of batched runs given none: 3/4 of the device memory
     // free when the first such run started (querying it costs a driver call)
     uint64_t default_budget = 0;
-    // device-scheduled rounds (BatchSession::run_device): bytes of each of a
+    // device-scheduled rounds (BatchSession::run_pages): bytes of each of a
     // run's two frontier regions; doubled after a run that overflowed them
     std::atomic<uint64_t> round_region_bytes{0};
 };
@@ -123,6 +123,8 @@ int run_batch(DevDB& db, std::vector<std::vector<Step>> steps, cudaStream_t s, u
               const uint32_t* vgraph, uint32_t G, uint64_t* counts, uint64_t* graph_counts_host,
               uint32_t* support_host, bool profile, BatchStats* stats, int rounds = ROUNDS_AUTO);
 uint64_t batch_kernel_launches();
+// Gives frontier regions that no run holds, beyond the usual size, back to the driver.
+void trim_round_pool(int device);
 
 // Pinned host staging, grown on demand.
 struct Staging {
@@ -182,14 +184,16 @@ public:
         return submit(std::move(copy), tags, ids, presorted);
     }
     int round();
-    // Runs every round of a single-wave session on the device: each round's
-    // planning kernel chooses the writing tasks, places their outputs and
-    // lists the next round's tasks, so the host launches all rounds at once
-    // and synchronises once.  Leaves the session idle with every plan's count
-    // set; or, when the session does not qualify (several waves, profiling,
-    // rounds already run, a budget below the frontier regions) or a round
-    // overflowed its region, leaves the initial tasks active for round().
-    int run_device();
+    // Runs every round of a single-wave session in one pass over its rows,
+    // output going to pages (round_pass_kernel) that a planning kernel orders
+    // for the next round: the host launches all rounds at once and
+    // synchronises once, or (stepped) launches a round after it has read how
+    // many items the one before left.  Leaves the session idle with every
+    // plan's count set; or, when the session does not qualify (several waves,
+    // profiling, rounds already run, a budget below the frontier regions) or
+    // a round overflowed its region, leaves the initial tasks active for
+    // round().
+    int run_pages();
     bool idle() const { return active.empty(); }
     std::vector<int> take_completed();
     const PlanRec& plan(int q) const { return plans[q]; }
@@ -216,8 +220,9 @@ public:
     } tune;
 
     uint64_t rounds = 0, splits = 0, launches = 0;
-    uint64_t device_rounds = 0;  // rounds scheduled on the device (run_device)
-    bool host_rounds = false;    // run_device declines: every round scheduled on the host
+    uint64_t device_rounds = 0;  // rounds scheduled on the device (run_pages)
+    bool host_rounds = false;    // run_pages declines: counted rounds, scheduled on the host
+    bool stepped = false;        // run_pages: a round is launched when the one before has been read
     double submit_ms = 0, round_host_ms = 0, wait_ms = 0;  // host time split
     // round_host_ms by part: task scan + uploads, count launches, totals and
     // budget choice, write launch, next tasks and completion
@@ -289,11 +294,12 @@ struct PreparedBatch {
     bool per_graph = false, graph_counts = false;
     double prep_ms = 0.0;
 };
-// host_rounds: finish_batch schedules every round on the host (else on the
-// device when the session qualifies, BatchSession::run_device)
+// rounds: ROUNDS_HOST = counted rounds scheduled on the host, else
+// BatchSession::run_pages when the session qualifies, stepped by the host for
+// one of several pieces of a run unless ROUNDS_DEVICE
 int prepare_batch(DevDB& db, std::vector<std::vector<Step>>&& steps, cudaStream_t s, uint64_t budget,
                   bool per_graph, bool graph_counts, bool profile, PreparedBatch& out, bool presorted = false,
-                  bool host_rounds = false);
+                  RoundsMode rounds = ROUNDS_AUTO, uint32_t pieces = 1);
 // order (optional): plan q's results go to index order[q] of the arrays
 int finish_batch(DevDB& db, PreparedBatch& pb, uint64_t* counts, uint64_t* graph_counts_host, uint32_t* support_host,
                  BatchStats* stats, const volatile int* cancel = nullptr, const uint32_t* order = nullptr);

@@ -111,6 +111,9 @@ __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* __restrict__
     return lo;
 }
 
+// A row is anything that gives its columns by index: a pointer to its words,
+// or a view of one row of a table kept column by column.
+
 // Candidate range of one row: the (source, label) segment cut below the
 // restriction bound.
 __device__ __forceinline__ void ext_range(const ExtArgs& p, const uint32_t* row, uint32_t& lo, uint32_t& hi) {
@@ -142,7 +145,8 @@ struct GenState {
     uint32_t clo[kMaxChecks], chi[kMaxChecks];  // dir-0 check segments
 };
 
-__device__ __forceinline__ void ext_generator(const ExtArgs& p, const uint32_t* row, GenState& g) {
+template <class Row>
+__device__ __forceinline__ void ext_generator(const ExtArgs& p, Row row, GenState& g) {
     uint32_t slo, shi;
     seg_of(p.off, p.L, row[p.src_col], p.lab, slo, shi);
     g.gadj = p.adj;
@@ -193,7 +197,8 @@ __device__ __forceinline__ bool seg_has(const uint32_t* __restrict__ off, const 
 
 // Whether generated candidate c survives injectivity, the source edge (when
 // the generator is a check segment) and every other check.
-__device__ __forceinline__ bool ext_accept(const ExtArgs& p, const uint32_t* row, uint32_t c, const GenState& g) {
+template <class Row>
+__device__ __forceinline__ bool ext_accept(const ExtArgs& p, Row row, uint32_t c, const GenState& g) {
     for (uint32_t j = 0; j < p.n_eq; ++j)
         if (row[p.eq_cols[j]] == c) return false;
     if (g.which >= 0 && find_in(p.adj, g.slo, g.shi, c) == 0xffffffffu) return false;
@@ -210,9 +215,9 @@ __device__ __forceinline__ bool ext_accept(const ExtArgs& p, const uint32_t* row
 // row's NEQ matched vertices (columns eq_cols), in one pass over the list;
 // the list is ascending, so the walk stops at the bound (no search for it).
 // A vertex in two columns still excludes its candidate once.
-template <int NEQ>
+template <int NEQ, class Row>
 __device__ __forceinline__ uint32_t short_list_count(const uint32_t* __restrict__ adj, uint32_t lo, uint32_t hi,
-                                                     uint64_t b, const uint32_t* row, const uint8_t* eq_cols) {
+                                                     uint64_t b, Row row, const uint8_t* eq_cols) {
     uint32_t eqv[NEQ > 0 ? NEQ : 1];
 #pragma unroll
     for (int e = 0; e < NEQ; ++e) eqv[e] = row[eq_cols[e]];
@@ -231,7 +236,8 @@ __device__ __forceinline__ uint32_t short_list_count(const uint32_t* __restrict_
 // Number of candidates of one row of a plain extension (no fused checks):
 // the segment below the restriction bound minus the already-matched
 // vertices in it.
-__device__ __forceinline__ uint32_t ext_count_plain(const ExtArgs& p, const uint32_t* row) {
+template <class Row>
+__device__ __forceinline__ uint32_t ext_count_plain(const ExtArgs& p, Row row) {
     uint32_t lo, hi;
     seg_of(p.off, p.L, row[p.src_col], p.lab, lo, hi);
     if (lo >= hi) return 0;
@@ -277,7 +283,8 @@ __device__ __forceinline__ uint32_t ext_count_row(const ExtArgs& p, const uint32
     return ext_count_plain(p, row);
 }
 
-__device__ __forceinline__ bool red_keep_row(const RedArgs& p, const uint32_t* row) {
+template <class Row>
+__device__ __forceinline__ bool red_keep_row(const RedArgs& p, Row row) {
     for (uint32_t j = 0; j < p.n_pairs; ++j) {
         const uint32_t s = row[p.rs[j]];
         const uint32_t e = row[p.re[j]];
