@@ -505,8 +505,8 @@ struct WarpSmem {
     uint32_t* tile;
     GenState* gen;
 };
-template <bool WRITE, bool FUSED, class Args>
-__device__ __forceinline__ WarpSmem warp_smem(unsigned char* raw, const Args& a) {
+template <bool WRITE, bool FUSED>
+__device__ __forceinline__ WarpSmem warp_smem(unsigned char* raw, const RoundArgs& a) {
     const int warp = threadIdx.x >> 5;
     WarpSmem w;
     w.d = reinterpret_cast<TaskDesc*>(raw) + warp;
@@ -793,11 +793,21 @@ round_write_kernel(RoundArgs a) {
 // page slots that its output has taken.
 struct PassState {
     unsigned long long heads[2];  // light class, fused class
+    unsigned long long units[2], unit_heads[2];  // long candidate lists: pieces, and their queue heads
     unsigned long long slots;
     uint64_t ni, ni_light;        // items: all, light class (the light class's items come first)
     uint32_t overflow;            // a region was too small: no later round finds work
     uint32_t pad;
 };
+
+// A piece of a long candidate list: candidates [x0, x1) of the group of 32
+// found rows from `base` of a task's item.
+struct Unit {
+    uint64_t item;
+    uint32_t task, base, x0, x1;
+};
+constexpr uint32_t kUnitLen = 256;        // candidates that stay with the warp that found them; of a piece
+constexpr uint32_t kUnitCap = 1u << 19;   // pieces of a round, per class
 
 struct PassArgs {
     const TaskDesc* nodes;
@@ -817,6 +827,7 @@ struct PassArgs {
     uint4* rec;                  // per slot written: (node, place among the node's rows, rows, width)
     uint32_t* node_rows;         // per node: rows written
     unsigned long long* node_total;  // per node: rows
+    Unit* units;                 // kUnitCap per class, light class first (null: no list is long)
     PassState* st;
     BatchCtx ctx;
 };
@@ -882,31 +893,78 @@ struct Pages {
     }
 };
 
-// One page or slice of an extension: 32 rows at a time, their candidate lists
-// end to end are dealt out to the lanes 32 candidates per step, whatever
-// their lengths: rows of a small graph have about one candidate each and up
-// to six (a lane per row left two thirds of the lanes idle), a hub has
-// thousands (they are read as consecutive words).  FEEDS: accepted rows go
+// The rows of an item whose source has a neighbour with the step's label, and
+// where their lists lie.
+struct Found {
+    uint32_t *row, *lo, *hi;
+};
+
+// Looks every row of an item up and lists those with candidates; returns how
+// many.  In the graph databases that is one row in ten (36 million seeds give
+// 3.3 million rows in the first round of a 16,384-pattern list), so whatever
+// follows a lookup is done on full warps of such rows only.
+__device__ __forceinline__ uint32_t pass_find(const ExtArgs& p, const uint32_t* rows_s, uint32_t nr, uint32_t R,
+                                              const Found& f) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t* src = rows_s + p.src_col * R;
+    const uint32_t *off = p.off, L = p.L, lab = p.lab;
+    uint32_t n = 0;
+    for (uint32_t base = 0; base < nr; base += 64) {
+        // two rows per lane: their index records are loaded together
+        const uint32_t r0 = base + lane, r1 = r0 + 32;
+        uint32_t lo0 = 0, hi0 = 0, lo1 = 0, hi1 = 0;
+        if (r0 < nr) seg_of(off, L, src[r0], lab, lo0, hi0);
+        if (r1 < nr) seg_of(off, L, src[r1], lab, lo1, hi1);
+        const uint32_t b0 = __ballot_sync(0xffffffffu, lo0 < hi0), b1 = __ballot_sync(0xffffffffu, lo1 < hi1);
+        const uint32_t below = (1u << lane) - 1u;
+        if (lo0 < hi0) {
+            const uint32_t at = n + __popc(b0 & below);
+            f.row[at] = r0;
+            f.lo[at] = lo0;
+            f.hi[at] = hi0;
+        }
+        n += __popc(b0);
+        if (lo1 < hi1) {
+            const uint32_t at = n + __popc(b1 & below);
+            f.row[at] = r1;
+            f.lo[at] = lo1;
+            f.hi[at] = hi1;
+        }
+        n += __popc(b1);
+    }
+    __syncwarp();
+    return n;
+}
+
+// One page or slice of an extension: the candidate lists of 32 rows end to
+// end are dealt out to the lanes 32 candidates per step, whatever their
+// lengths (a row of a small graph has one to six candidates, under a hub
+// thousands, which are read as consecutive words).  FEEDS: accepted rows go
 // to the node's pages; else (fused class only) they are counted.
+// A group with more than kUnitLen candidates keeps the first of them and
+// queues the others for the round's second launch (`unit`: one of its pieces).
 template <bool FEEDS, bool FUSED>
 __device__ __forceinline__ uint64_t pass_extend(const PassArgs& a, const TaskDesc& d, uint32_t node,
-                                                const uint32_t* rows_s, uint32_t nr, GenState* gen_s, Pages& pg) {
+                                                const uint32_t* rows_s, uint32_t nr, const Found& f, GenState* gen_s,
+                                                Pages& pg, uint32_t task, uint64_t item, const Unit* unit) {
     const ExtArgs& p = d.e;
     const uint32_t lane = threadIdx.x & 31, R = a.rows_per_item;
     const bool graphs = d.mode == MODE_COUNT_GRAPHS || d.mode == MODE_WRITE_AND_GRAPHS;
+    const uint32_t found = pass_find(p, rows_s, nr, R, f);
     uint64_t total = 0;
-    for (uint32_t base = 0; base < nr; base += 32) {
-        uint32_t lo = 0, hi = 0;
-        if (base + lane < nr) {
+    for (uint32_t base = unit ? unit->base : 0; base < (unit ? unit->base + 1 : found); base += 32) {
+        uint32_t lo = 0, mine = 0, r = 0;
+        if (base + lane < found) {
+            r = f.row[base + lane];
+            lo = f.lo[base + lane];
+            uint32_t hi = f.hi[base + lane];
             if (FUSED) {
-                ext_generator(p, Col{rows_s + base + lane, R}, gen_s[lane]);
+                ext_generator_from(p, Col{rows_s + r, R}, lo, hi, gen_s[lane]);
                 lo = gen_s[lane].lo;
                 hi = gen_s[lane].hi;
-            } else {
-                seg_of(p.off, p.L, rows_s[p.src_col * R + base + lane], p.lab, lo, hi);
             }
+            mine = hi > lo ? hi - lo : 0;
         }
-        const uint32_t mine = hi > lo ? hi - lo : 0;
         if (FUSED) __syncwarp();  // generator states written before other lanes read them
         // lists so long that their sum might not fit a word: one row at a time
         const bool huge = __any_sync(0xffffffffu, mine > (1u << 26));
@@ -920,7 +978,23 @@ __device__ __forceinline__ uint64_t pass_extend(const PassArgs& a, const TaskDes
             }
             const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
             const uint32_t shift = lo - (inc - len);  // list position of candidate x: shift + x
-            for (uint32_t x0 = 0; x0 < all; x0 += 32) {
+            uint32_t from = 0, stop = all;
+            if (unit) {
+                from = unit->x0;
+                stop = unit->x1;
+            } else if (a.units && all > kUnitLen && !huge) {
+                const uint32_t np = (all - 1) / kUnitLen;
+                unsigned long long at = 0;
+                if (lane == 0) at = atomicAdd(a.st->units + (FUSED ? 1 : 0), (unsigned long long)np);
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (at + np <= kUnitCap) stop = kUnitLen;  // else the list stays here, and empty pieces there
+                for (uint32_t i = lane; i < np && at + i < kUnitCap; i += 32) {
+                    const uint32_t x = (i + 1) * kUnitLen;
+                    a.units[(FUSED ? kUnitCap : 0) + at + i] =
+                        Unit{item, task, base, x, stop == all ? x : min(all, x + kUnitLen)};
+                }
+            }
+            for (uint32_t x0 = from; x0 < stop; x0 += 32) {
                 const uint32_t x = x0 + lane;
                 uint32_t q = 0;  // the row of candidate x: rows whose lists end at or before it
 #pragma unroll
@@ -929,9 +1003,10 @@ __device__ __forceinline__ uint64_t pass_extend(const PassArgs& a, const TaskDes
                     if (e <= x) q += o;
                 }
                 const uint32_t at = __shfl_sync(0xffffffffu, shift, q) + x;
-                bool ok = x < all;
+                const uint32_t rr = __shfl_sync(0xffffffffu, r, q);
+                bool ok = x < stop;
                 uint32_t c = 0;
-                const Col row{rows_s + base + q, R};
+                const Col row{rows_s + rr, R};
                 if (ok) {
                     if (FUSED) {
                         c = __ldg(gen_s[q].gadj + at);
@@ -946,7 +1021,7 @@ __device__ __forceinline__ uint64_t pass_extend(const PassArgs& a, const TaskDes
                     }
                 }
                 if (FEEDS)
-                    total += pg.put(a, node, ok, rows_s, p.k, true, base + q, c);
+                    total += pg.put(a, node, ok, rows_s, p.k, true, rr, c);
                 else
                     total += __popc(__ballot_sync(0xffffffffu, ok));
                 if (graphs) add_graph_count(a.ctx, d.query, row[0], ok ? 1u : 0u, true);
@@ -959,15 +1034,17 @@ __device__ __forceinline__ uint64_t pass_extend(const PassArgs& a, const TaskDes
 
 // The same for a plain extension that nothing follows: a lane counts its row.
 __device__ __forceinline__ uint64_t pass_count(const PassArgs& a, const TaskDesc& d, const uint32_t* rows_s,
-                                               uint32_t nr) {
+                                               uint32_t nr, const Found& f) {
     const uint32_t lane = threadIdx.x & 31, R = a.rows_per_item;
     const bool graphs = d.mode == MODE_COUNT_GRAPHS;
+    const uint32_t found = pass_find(d.e, rows_s, nr, R, f);
     uint64_t total = 0;
-    for (uint32_t base = 0; base < nr; base += 32) {
-        const bool valid = base + lane < nr;
-        const Col row{rows_s + (valid ? base + lane : 0), R};
+    for (uint32_t base = 0; base < found; base += 32) {
+        const bool valid = base + lane < found;
+        const uint32_t i = valid ? base + lane : 0;
+        const Col row{rows_s + f.row[i], R};
         uint32_t cnt = 0;
-        if (valid) cnt = ext_count_plain(d.e, row);
+        if (valid) cnt = ext_count_range(d.e, row, f.lo[i], f.hi[i]);
         if (graphs) add_graph_count(a.ctx, d.query, row[0], cnt, valid);
         total += cnt;
     }
@@ -1008,22 +1085,40 @@ __device__ __forceinline__ void stage_page(uint32_t* rows_s, const uint32_t* __r
     cp_async_commit();
 }
 
-// Shared memory of one warp: descriptor, row buffers, generator states.
-size_t pass_smem_bytes(uint32_t rows_per_item, uint32_t kmax, bool fused) {
-    return (size_t)kRoundWarps *
-           (sizeof(TaskDesc) + (fused ? kGenBytes : 0) + 4 * round_warp_words(rows_per_item, kmax, false, fused));
+// Shared memory of one warp: descriptor, generator states, row buffers, the
+// rows found.
+__host__ __device__ constexpr size_t pass_warp_words(uint32_t R, uint32_t kmax, bool fused) {
+    return (size_t)row_buffers(fused) * R * kmax + 3 * R;  // a multiple of 32
+}
+size_t pass_smem_bytes(uint32_t R, uint32_t kmax, bool fused) {
+    return (size_t)kRoundWarps * (sizeof(TaskDesc) + (fused ? kGenBytes : 0) + 4 * pass_warp_words(R, kmax, fused));
 }
 
-template <bool FUSED>
-__global__ void __launch_bounds__(kRoundWarps * 32, FUSED ? 4 : 6)
+// UNITS: the second launch of a round on a graph with long lists.  Items are
+// small enough to share out evenly by their rows, but not by their candidates:
+// on an R-MAT graph a page under a hub has a hundred thousand.  Pieces of
+// 2,048 / 512 / 256 / 128 candidates: 61 queries on 2^14 vertices take 1.52 /
+// 0.95 / 0.90 / 1.02 ms, without pieces 2.46.
+//
+// Registers rather than warps: at 6 CTAs per SM (40 registers) the spills took
+// a quarter of the L1 traffic; 4 CTAs (64) are 10-15 % faster.
+template <bool FUSED, bool UNITS>
+__global__ void __launch_bounds__(kRoundWarps * 32, FUSED ? 3 : 4)
 round_pass_kernel(const __grid_constant__ PassArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // the light class's launch may start on the SMs that this one no longer
     // fills; it waits for this one before it ends (below)
-    if (FUSED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (FUSED && !UNITS) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t lane = threadIdx.x & 31, R = a.rows_per_item;
-    const WarpSmem ws = warp_smem<false, FUSED>(smem_raw, a);
-    TaskDesc& d = *ws.d;
+    const uint32_t warp = threadIdx.x >> 5;
+    TaskDesc& d = reinterpret_cast<TaskDesc*>(smem_raw)[warp];
+    unsigned char* const area = smem_raw + kRoundWarps * sizeof(TaskDesc);  // 16-byte aligned
+    GenState* const gen = FUSED ? reinterpret_cast<GenState*>(area) + 32 * warp : nullptr;
+    uint32_t* const buf =
+        reinterpret_cast<uint32_t*>(area + (FUSED ? kRoundWarps * kGenBytes : 0)) + warp * pass_warp_words(R, a.kmax, FUSED);
+    uint32_t* const buf2 = buf + (row_buffers(FUSED) - 1) * R * a.kmax;
+    uint32_t* const lists = buf + row_buffers(FUSED) * R * a.kmax;
+    const Found f{lists, lists + R, lists + 2 * R};
     uint64_t t_lo = 0, t_hi = 0, begin, end, total = 0;
     const uint32_t* in = nullptr;     // first round: the task's seed list; later: its parent's pages
     uint64_t nrows = 0;
@@ -1031,8 +1126,11 @@ round_pass_kernel(const __grid_constant__ PassArgs a) {
     bool ready = false;               // light class: the current item's rows were issued with the previous item
     Pages pg;
     const uint64_t light = a.st->ni_light;
-    const Span sp{FUSED ? light : 0, FUSED ? a.st->ni - light : light, a.st->heads + (FUSED ? 1 : 0),
-                  gridDim.x * kRoundWarps};
+    const Span sp = UNITS ? Span{0, umin64(a.st->units[FUSED ? 1 : 0], kUnitCap), a.st->unit_heads + (FUSED ? 1 : 0),
+                                 gridDim.x * kRoundWarps}
+                          : Span{FUSED ? light : 0, FUSED ? a.st->ni - light : light, a.st->heads + (FUSED ? 1 : 0),
+                                 gridDim.x * kRoundWarps};
+    uint32_t t = 0xffffffffu;
     auto task_done = [&]() {
         pg.close(a, node);
         if (lane == 0 && total) atomicAdd(a.node_total + node, (unsigned long long)total);
@@ -1043,37 +1141,55 @@ round_pass_kernel(const __grid_constant__ PassArgs a) {
     auto stage = [&](uint32_t* rows_s, uint64_t i) {
         stage_page(rows_s, in + i * words, (uint32_t)umin64(R, nrows - i * R), k, R, a.seeds != nullptr);
     };
+    auto open_task = [&](uint32_t task_index) {
+        task_done();
+        t = task_index;
+        t_lo = __ldg(a.item0 + t);
+        t_hi = __ldg(a.item0 + t + 1);
+        const uint2 task = __ldg(a.tasks + t);
+        if (a.seeds) {
+            in = a.seeds[t].in;
+            nrows = a.seeds[t].nrows;
+        } else {
+            in = a.in_region + (uint64_t)a.page_base[task.y] * words;
+            nrows = a.node_rows[task.y];
+        }
+        __syncwarp();
+        load_desc(d, a.nodes + task.x);
+        node = task.x;
+        k = d.kind == STEP_EXT ? d.e.k : d.r.k;
+        pg.width = d.kind == STEP_EXT ? k + 1 : k;
+    };
+    if (UNITS) {
+        while (next_chunk(sp, begin, end)) {
+            for (uint64_t u = begin; u < end; ++u) {
+                const Unit unit = a.units[(FUSED ? kUnitCap : 0) + u];
+                if (unit.x0 >= unit.x1) continue;
+                if (unit.task != t) open_task(unit.task);
+                __syncwarp();
+                stage(buf, unit.item);
+                cp_async_wait_all();
+                __syncwarp();
+                const uint32_t nr = (uint32_t)umin64(R, nrows - unit.item * R);
+                total += d.feeds ? pass_extend<true, FUSED>(a, d, node, buf, nr, f, gen, pg, t, unit.item, &unit)
+                                 : pass_extend<false, FUSED>(a, d, node, buf, nr, f, gen, pg, t, unit.item, &unit);
+                __syncwarp();
+            }
+        }
+    } else
     while (next_chunk(sp, begin, end)) {
         const uint64_t stop = sp.base + end;
         for (uint64_t item = sp.base + begin; item < stop; ++item) {
-            if (item >= t_hi || item < t_lo) {
-                task_done();
-                const uint32_t t = find_slot(a.item0, a.nt + 1, item);
-                t_lo = __ldg(a.item0 + t);
-                t_hi = __ldg(a.item0 + t + 1);
-                const uint2 task = __ldg(a.tasks + t);
-                if (a.seeds) {
-                    in = a.seeds[t].in;
-                    nrows = a.seeds[t].nrows;
-                } else {
-                    in = a.in_region + (uint64_t)a.page_base[task.y] * words;
-                    nrows = a.node_rows[task.y];
-                }
-                __syncwarp();
-                load_desc(d, a.nodes + task.x);
-                node = task.x;
-                k = d.kind == STEP_EXT ? d.e.k : d.r.k;
-                pg.width = d.kind == STEP_EXT ? k + 1 : k;
-            }
+            if (item >= t_hi || item < t_lo) open_task(find_slot(a.item0, a.nt + 1, item));
             const uint64_t i = item - t_lo;
             const uint32_t nr = (uint32_t)umin64(R, nrows - i * R);
-            uint32_t* rows = ws.rows;
+            uint32_t* rows = buf;
             if (FUSED) {
                 __syncwarp();
                 stage(rows, i);
                 cp_async_wait_all();
             } else {
-                rows = cur ? ws.rows2 : ws.rows;
+                rows = cur ? buf2 : buf;
                 if (!ready) {
                     __syncwarp();
                     stage(rows, i);
@@ -1081,7 +1197,7 @@ round_pass_kernel(const __grid_constant__ PassArgs a) {
                 // the next item of the same task and chunk: its rows are copied in meanwhile
                 ready = item + 1 < stop && item + 1 < t_hi;
                 if (ready) {
-                    stage(cur ? ws.rows : ws.rows2, i + 1);
+                    stage(cur ? buf : buf2, i + 1);
                     cp_async_wait_one();
                 } else {
                     cp_async_wait_all();
@@ -1090,18 +1206,18 @@ round_pass_kernel(const __grid_constant__ PassArgs a) {
             }
             __syncwarp();
             if (FUSED)
-                total += d.feeds ? pass_extend<true, true>(a, d, node, rows, nr, ws.gen, pg)
-                                 : pass_extend<false, true>(a, d, node, rows, nr, ws.gen, pg);
+                total += d.feeds ? pass_extend<true, true>(a, d, node, rows, nr, f, gen, pg, t, i, nullptr)
+                                 : pass_extend<false, true>(a, d, node, rows, nr, f, gen, pg, t, i, nullptr);
             else if (d.kind != STEP_EXT)
                 total += pass_reduce(a, d, node, rows, nr, pg);
             else
-                total += d.feeds ? pass_extend<true, false>(a, d, node, rows, nr, nullptr, pg)
-                                 : pass_count(a, d, rows, nr);
+                total += d.feeds ? pass_extend<true, false>(a, d, node, rows, nr, f, nullptr, pg, t, i, nullptr)
+                                 : pass_count(a, d, rows, nr, f);
             __syncwarp();  // every lane done with these rows before the buffer is refilled
         }
     }
     task_done();
-    if (!FUSED) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!FUSED && !UNITS) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Planning of the next round, by one cluster: the finished round's nodes get
@@ -1365,12 +1481,16 @@ int BatchSession::init() {
     if (!smem_set[dev].load(std::memory_order_acquire)) {
         const int most = (int)std::max(round_smem_bytes(kMaxItemRows / 4, kMaxCols, true, true),
                                        round_smem_bytes(kMaxItemRows / 4, kMaxCols, true, false));  // rows per item shrink as rows widen
+        const int pass_most = (int)std::max(std::max(pass_smem_bytes(32, kMaxCols, true), pass_smem_bytes(32, kMaxCols, false)),
+                                            std::max(pass_smem_bytes(kMaxItemRows, 6, true), pass_smem_bytes(kMaxItemRows, 6, false)));
         GVA_CUDA_B(cudaFuncSetAttribute(round_count_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
         GVA_CUDA_B(cudaFuncSetAttribute(round_count_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
         GVA_CUDA_B(cudaFuncSetAttribute(round_write_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
         GVA_CUDA_B(cudaFuncSetAttribute(round_write_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-        GVA_CUDA_B(cudaFuncSetAttribute(round_pass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-        GVA_CUDA_B(cudaFuncSetAttribute(round_pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        GVA_CUDA_B(cudaFuncSetAttribute(round_pass_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, pass_most));
+        GVA_CUDA_B(cudaFuncSetAttribute(round_pass_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, pass_most));
+        GVA_CUDA_B(cudaFuncSetAttribute(round_pass_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, pass_most));
+        GVA_CUDA_B(cudaFuncSetAttribute(round_pass_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, pass_most));
         smem_set[dev].store(true, std::memory_order_release);
     }
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -2359,8 +2479,11 @@ int BatchSession::run_pages() {
     if (!h) return fail(GVA_ERR_NOMEM, "pinned staging allocation failed");
     std::vector<uint32_t> R(D + 2, 32);
     for (int d = 1; d <= D; ++d) {
-        R[d] = std::min<uint32_t>(tune.rows_per_item, std::max<uint32_t>(32, (768 / kmax[d]) & ~31u));
-        if (R[d] == 96) R[d] = 64;  // a power of two (stage_page)
+        // twice the tuned rows (128 by default): a tenth of them is left after
+        // the lookups.  64 / 128 rows, per call: 16,384 patterns 9.1 / 8.2 ms,
+        // 1,501 texts 2.04 / 1.96 ms, 16 patterns 458 / 447 us
+        R[d] = std::min<uint32_t>(2 * tune.rows_per_item, std::max<uint32_t>(32, (768 / kmax[d]) & ~31u));
+        R[d] = R[d] >= 128 ? 128 : R[d] >= 64 ? 64 : 32;  // a power of two (stage_page)
     }
     uint2* h_tasks = (uint2*)(h + o_tasks);
     {
@@ -2406,9 +2529,12 @@ int BatchSession::run_pages() {
     }
     lap(0);
     // one allocation, of nearly the same size in every run: regions, then the
-    // schedule's arrays
+    // schedule's arrays; on a graph with long lists also the queues of their
+    // pieces
+    const bool long_lists = db.max_degree > kUnitLen;
+    const size_t o_units = o_rec + al(slot_most * sizeof(uint4));
     const size_t region_bytes = al(region);
-    const size_t unit = (size_t)256 << 20, blk_bytes = o_rec + al(slot_most * sizeof(uint4));
+    const size_t unit = (size_t)256 << 20, blk_bytes = o_units + (long_lists ? 2 * (size_t)kUnitCap * sizeof(Unit) : 0);
     char* mem = nullptr;
     cudaMemPool_t pool = round_pool(db.device);
     if (!pool || cudaMallocFromPoolAsync((void**)&mem, 2 * region_bytes + (blk_bytes + unit - 1) / unit * unit, pool, s) !=
@@ -2469,11 +2595,13 @@ int BatchSession::run_pages() {
         pa.rec = (uint4*)(blk + o_rec);
         pa.node_rows = (uint32_t*)(blk + o_nrows);
         pa.node_total = ntot;
+        pa.units = long_lists ? (Unit*)(blk + o_units) : nullptr;
         pa.st = states + d;
         pa.ctx = ctx;
         if (items_fused) {
             const size_t smem = pass_smem_bytes(R[d], kmax[d], true);
-            round_pass_kernel<true><<<grid((const void*)round_pass_kernel<true>, smem, items_fused), kRoundWarps * 32, smem, s>>>(pa);
+            round_pass_kernel<true, false>
+                <<<grid((const void*)round_pass_kernel<true, false>, smem, items_fused), kRoundWarps * 32, smem, s>>>(pa);
             ++nl;
         }
         if (items_light) {
@@ -2481,7 +2609,7 @@ int BatchSession::run_pages() {
             // before that one's last items are done
             const size_t smem = pass_smem_bytes(R[d], kmax[d], false);
             cudaLaunchConfig_t cfg{};
-            cfg.gridDim = dim3(grid((const void*)round_pass_kernel<false>, smem, items_light));
+            cfg.gridDim = dim3(grid((const void*)round_pass_kernel<false, false>, smem, items_light));
             cfg.blockDim = dim3(kRoundWarps * 32);
             cfg.dynamicSmemBytes = smem;
             cfg.stream = s;
@@ -2490,7 +2618,19 @@ int BatchSession::run_pages() {
             at.val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = &at;
             cfg.numAttrs = items_fused ? 1 : 0;
-            GVA_CUDA_B(cudaLaunchKernelEx(&cfg, round_pass_kernel<false>, pa));
+            GVA_CUDA_B(cudaLaunchKernelEx(&cfg, round_pass_kernel<false, false>, pa));
+            ++nl;
+        }
+        if (long_lists && items_fused) {
+            const size_t smem = pass_smem_bytes(R[d], kmax[d], true);
+            round_pass_kernel<true, true>
+                <<<grid((const void*)round_pass_kernel<true, true>, smem, kMany), kRoundWarps * 32, smem, s>>>(pa);
+            ++nl;
+        }
+        if (long_lists && items_light && d < D) {  // tasks that nothing follows are counted without walking their lists
+            const size_t smem = pass_smem_bytes(R[d], kmax[d], false);
+            round_pass_kernel<false, true>
+                <<<grid((const void*)round_pass_kernel<false, true>, smem, kMany), kRoundWarps * 32, smem, s>>>(pa);
             ++nl;
         }
         if (d == D) continue;  // the deepest round's tasks have no children

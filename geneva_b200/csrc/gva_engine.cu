@@ -409,6 +409,14 @@ int upload_graph(HostGraph& g, int device, DevDB*& out) {
     db->packed = packed;
     db->labels = g.labels;
     db->seed_off = seed_off;
+    for (uint32_t l = 0; l < L; ++l) {  // the first of each label's group by degree
+        if (seed_off[l] == seed_off[l + 1]) continue;
+        const uint64_t v = seed_deg[seed_off[l]];
+        uint64_t deg = 0;
+        for (const HostPartition& p : g.parts)
+            if (!p.off.empty()) deg += p.off[v * L + L] - p.off[v * L];
+        db->max_degree = std::max(db->max_degree, deg);
+    }
     db->arena = arena;
     db->arena_bytes = bytes;
     char* cur = (char*)arena;

@@ -36,6 +36,7 @@ struct DevDB {
     void* arena = nullptr;
     size_t arena_bytes = 0;
     uint64_t n_adj = 0;
+    uint64_t max_degree = 0;              // the most neighbours of one vertex, over all partitions
     HostGraph meta;                       // labels/partition presence for lowering (no adjacency)
     uint32_t* vgraph = nullptr;           // optional vertex -> graph id map (graph databases)
     uint32_t num_graphs = 0;

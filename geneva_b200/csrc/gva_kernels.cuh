@@ -146,9 +146,7 @@ struct GenState {
 };
 
 template <class Row>
-__device__ __forceinline__ void ext_generator(const ExtArgs& p, Row row, GenState& g) {
-    uint32_t slo, shi;
-    seg_of(p.off, p.L, row[p.src_col], p.lab, slo, shi);
+__device__ __forceinline__ void ext_generator_from(const ExtArgs& p, Row row, uint32_t slo, uint32_t shi, GenState& g) {
     g.gadj = p.adj;
     g.which = -1;
     if (slo >= shi) {  // no candidate from the source: nothing else to look up
@@ -186,6 +184,13 @@ __device__ __forceinline__ void ext_generator(const ExtArgs& p, Row row, GenStat
             g.which = i;
         }
     }
+}
+
+template <class Row>
+__device__ __forceinline__ void ext_generator(const ExtArgs& p, Row row, GenState& g) {
+    uint32_t slo, shi;
+    seg_of(p.off, p.L, row[p.src_col], p.lab, slo, shi);
+    ext_generator_from(p, row, slo, shi, g);
 }
 
 __device__ __forceinline__ bool seg_has(const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj, uint32_t L,
@@ -233,14 +238,11 @@ __device__ __forceinline__ uint32_t short_list_count(const uint32_t* __restrict_
     return m;
 }
 
-// Number of candidates of one row of a plain extension (no fused checks):
-// the segment below the restriction bound minus the already-matched
-// vertices in it.
+// Number of candidates of one row of a plain extension (no fused checks) in
+// its source's segment [lo, hi), which holds at least one vertex: those below
+// the restriction bound minus the already-matched vertices.
 template <class Row>
-__device__ __forceinline__ uint32_t ext_count_plain(const ExtArgs& p, Row row) {
-    uint32_t lo, hi;
-    seg_of(p.off, p.L, row[p.src_col], p.lab, lo, hi);
-    if (lo >= hi) return 0;
+__device__ __forceinline__ uint32_t ext_count_range(const ExtArgs& p, Row row, uint32_t lo, uint32_t hi) {
     const uint32_t n_eq = p.n_eq;
     if (hi - lo <= 8 && n_eq <= 8) {
         const uint64_t b = p.bound_col >= 0 ? (uint64_t)row[p.bound_col] + p.bound_incl : ~0ull;
@@ -269,6 +271,13 @@ __device__ __forceinline__ uint32_t ext_count_plain(const ExtArgs& p, Row row) {
         if (!dup && find_in(p.adj, lo, hi, w) != 0xffffffffu) --n;
     }
     return n;
+}
+
+template <class Row>
+__device__ __forceinline__ uint32_t ext_count_plain(const ExtArgs& p, Row row) {
+    uint32_t lo, hi;
+    seg_of(p.off, p.L, row[p.src_col], p.lab, lo, hi);
+    return lo < hi ? ext_count_range(p, row, lo, hi) : 0;
 }
 
 // Number of candidates of one row, plain or with fused checks.

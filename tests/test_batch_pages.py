@@ -68,3 +68,50 @@ def test_stepped_halves(native):
     assert st["device_rounds"] == 0 and st["rounds"] > 0
     assert [int(c) for c in counts] == list(want) * reps
     db.close()
+
+
+@pytest.mark.parametrize("m", [7, 12, 13, 16])
+def test_wide_rows(native, m):
+    """Rows wide enough for pages of 64 and 32 rows: paths of m vertices along
+    one long path whose labels repeat 1, 2, 3."""
+    n = 3 * 500
+    labels = np.array([0] + [1 + i % 3 for i in range(n)], np.uint32)
+    a = np.arange(1, n, dtype=np.uint32)
+    db = gv.Database.from_edges(labels, a, a + 1, np.ones(n - 1, np.uint32))
+    texts = ["".join(f"v {i} {1 + (i + s) % 3}\n" for i in range(m)) + "".join(f"e {i} {i + 1} 1\n" for i in range(m - 1))
+             for s in range(3)]
+    counts, _, st = gv.batch_count(db, gv.Plan.batch_from_texts(texts))
+    assert st["device_rounds"] > 0
+    assert [int(c) for c in counts] == [len(range(s, n - m + 1, 3)) for s in range(3)]
+    db.close()
+
+
+@pytest.mark.parametrize("hubs,n", [(1, 300), (3, 2100), (2, 4097)])
+def test_long_lists(native, hubs, n):
+    """Lists cut into pieces: hubs joined in a path, their leaves paired, so
+    that extensions with and without fused checks walk thousands of
+    candidates per row."""
+    labels, edges, first = [0], [], []
+    for h in range(hubs):
+        labels.append(1)
+        hub = len(labels) - 1
+        first.append(hub)
+        leaf = list(range(len(labels), len(labels) + n))
+        labels += [2] * n
+        edges += [(hub, v) for v in leaf] + [(leaf[i], leaf[i + 1]) for i in range(0, n - 1, 2)]
+        if h:
+            edges.append((first[-2], hub))
+    e = np.array(edges, np.uint32)
+    db = gv.Database.from_edges(np.array(labels, np.uint32), e[:, 0], e[:, 1], np.ones(len(e), np.uint32))
+    pairs = n // 2
+    texts = ["v 0 1\nv 1 2\nv 2 2\ne 0 1 1\ne 0 2 1\ne 1 2 1\n",              # triangles
+             "v 0 1\nv 1 2\nv 2 2\ne 0 1 1\ne 0 2 1\n",                       # two leaves of a hub
+             "v 0 2\nv 1 1\nv 2 1\nv 3 2\ne 0 1 1\ne 1 2 1\ne 2 3 1\n",       # leaf, hub, hub, leaf
+             "v 0 1\nv 1 2\nv 2 2\nv 3 2\ne 0 1 1\ne 0 2 1\ne 1 2 1\ne 0 3 1\n"]  # triangle and a leaf
+    want = [hubs * pairs, hubs * n * (n - 1) // 2, (hubs - 1) * n * n, hubs * pairs * (n - 2)]
+    for R in (32, 64):
+        db.set_tuning(R, 32)
+        counts, _, st = gv.batch_count(db, gv.Plan.batch_from_texts(texts))
+        assert st["device_rounds"] > 0
+        assert [int(c) for c in counts] == want
+    db.close()
