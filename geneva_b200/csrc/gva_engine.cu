@@ -14,6 +14,7 @@
 // Label segments come from a dense (vertex, label) offset table, one load per
 // lookup, replacing the warp bisection with vLabel gathers of the reference
 // (FIND_LABEL_LIMIT, include/common.h:18-66).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -54,10 +55,98 @@ __global__ void __launch_bounds__(kThreads) red_count_kernel(RedArgs p, uint64_t
     store_block_sum(c, block_sums);
 }
 
-// Block b expands rows [256b, 256b + 256): every thread produces one output
-// row per tile, so a block's work is balanced however the candidates are
-// spread over its rows.
-__global__ void __launch_bounds__(kThreads) ext_write_kernel(ExtArgs p, const uint64_t* __restrict__ block_off) {
+// The outputs of an extension are shared out to CTAs by an ordinal that
+// counts both the rows read and the rows written: block b (256 input rows)
+// takes kBlockWork for its prologue (lookups and a scan) and then one for each
+// of its output rows.  A CTA takes `chunk` consecutive ordinals, so that a
+// block under a hub is written by as many CTAs as its rows need and a run of
+// blocks without output costs one.  (With a CTA per block, 910 blocks wrote
+// the 24 million rows of one step on an R-MAT graph of 2^18 vertices in 830
+// us, most of them waiting for a few hub blocks.)
+constexpr uint64_t kBlockWork = 1024;
+constexpr uint64_t kEvenDegree = 256;  // up to this degree a CTA takes a block
+
+__device__ __forceinline__ uint64_t block_key(const uint64_t* __restrict__ block_off, uint64_t b) {
+    return __ldg(block_off + b) + b * kBlockWork;
+}
+
+// Last block b in [0, nb) with block_key(b) <= x, found by the first warp, 32
+// pivots per step.
+__device__ __forceinline__ uint64_t find_block(const uint64_t* __restrict__ block_off, uint64_t nb, uint64_t x) {
+    __shared__ uint64_t found;
+    if (threadIdx.x < 32) {
+        uint64_t lo = 0, len = nb;
+        while (len > 1) {
+            const uint64_t step = (len + 31) / 32, at = threadIdx.x * step;
+            const uint32_t m = __ballot_sync(0xffffffffu, at < len && block_key(block_off, lo + at) <= x);
+            const uint64_t k = (31 - __clz(m)) * step;  // block 0's key is 0
+            lo += k;
+            len = len - k < step ? len - k : step;
+        }
+        if (threadIdx.x == 0) found = lo;
+    }
+    __syncthreads();
+    const uint64_t b = found;
+    __syncthreads();
+    return b;
+}
+
+// The part [first, last) of block b's output rows that ordinals [k0, k1) hold.
+__device__ __forceinline__ void block_part(const uint64_t* __restrict__ block_off, uint64_t b, uint64_t k0, uint64_t k1,
+                                           uint64_t& first, uint64_t& last) {
+    const uint64_t base = block_key(block_off, b) + kBlockWork, n = __ldg(block_off + b + 1) - __ldg(block_off + b);
+    first = k0 > base ? k0 - base : 0;
+    last = k1 > base ? umin64(k1 - base, n) : 0;
+}
+
+// One row of a block: its candidate list and the positions in it of matched
+// vertices (ascending, each once); returns its output rows.
+__device__ __forceinline__ uint32_t block_row(const ExtArgs& p, const uint32_t* row, uint32_t* coll, uint32_t& lo,
+                                              uint32_t& nc) {
+    uint32_t hi;
+    ext_range(p, row, lo, hi);
+    nc = 0;
+    if (lo >= hi) return 0;
+    for (uint32_t j = 0; j < p.n_eq; ++j) {
+        const uint32_t pos = find_in(p.adj, lo, hi, row[p.eq_cols[j]]);
+        if (pos == 0xffffffffu) continue;
+        bool dup = false;
+        for (uint32_t i = 0; i < nc; ++i) dup |= (coll[i] == pos);
+        if (dup) continue;
+        uint32_t i = nc++;  // insertion sort, ascending
+        while (i > 0 && coll[i - 1] > pos) {
+            coll[i] = coll[i - 1];
+            --i;
+        }
+        coll[i] = pos;
+    }
+    return hi - lo - nc;
+}
+
+// List position of a row's u-th output row.
+__device__ __forceinline__ uint32_t nth_candidate(uint32_t lo, const uint32_t* coll, uint32_t nc, uint32_t u) {
+    uint32_t j = lo + u;
+    for (uint32_t c = 0; c < nc; ++c) j += (coll[c] <= j) ? 1u : 0u;
+    return j;
+}
+
+// Largest r in [0, nr) with offs[r] <= o.
+__device__ __forceinline__ int row_of(const uint64_t* offs, int nr, uint64_t o) {
+    int a = 0, b = nr - 1;
+    while (a < b) {
+        const int m = (a + b + 1) >> 1;
+        if (offs[m] <= o)
+            a = m;
+        else
+            b = m - 1;
+    }
+    return a;
+}
+
+// Every thread produces one output row per tile of 256, so a CTA's work is
+// balanced however the candidates are spread over its rows.
+__global__ void __launch_bounds__(kThreads) ext_write_kernel(ExtArgs p, const uint64_t* __restrict__ block_off,
+                                                             uint64_t nb, uint64_t chunk) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint64_t* offs_s = reinterpret_cast<uint64_t*>(smem_raw);           // 257
     uint32_t* rows_s = reinterpret_cast<uint32_t*>(offs_s + kRowsPerBlock + 1);  // 256 * k
@@ -65,75 +154,214 @@ __global__ void __launch_bounds__(kThreads) ext_write_kernel(ExtArgs p, const ui
     uint32_t* ncol_s = lo_s + kRowsPerBlock;                              // 256
     uint32_t* coll_s = ncol_s + kRowsPerBlock;                            // 256 * n_eq
     uint32_t* out_s = coll_s + kRowsPerBlock * p.n_eq;                    // 256 * (k + 1)
-
-    const uint64_t row0 = (uint64_t)blockIdx.x * kRowsPerBlock;
-    const uint32_t nr = (uint32_t)umin64((uint64_t)kRowsPerBlock, p.nrows - row0);
     const uint32_t k = p.k, k1 = p.k + 1;
+    const uint64_t o0 = blockIdx.x * chunk, o1 = o0 + chunk;
+    for (uint64_t b = chunk ? find_block(block_off, nb, o0) : blockIdx.x;; ++b) {
+        uint64_t first = 0, last = 0;
+        if (chunk) {
+            if (b >= nb || block_key(block_off, b) >= o1) break;
+            block_part(block_off, b, o0, o1, first, last);
+            if (first >= last) continue;
+        }
+        const uint64_t row0 = b * kRowsPerBlock;
+        const uint32_t nr = (uint32_t)umin64((uint64_t)kRowsPerBlock, p.nrows - row0);
 
-    // coalesced load of this block's rows
-    const uint32_t* gin = p.in + row0 * k;
-    for (uint32_t w = threadIdx.x; w < nr * k; w += kThreads) rows_s[w] = gin[w];
-    __syncthreads();
+        // coalesced load of this block's rows
+        const uint32_t* gin = p.in + row0 * k;
+        for (uint32_t w = threadIdx.x; w < nr * k; w += kThreads) rows_s[w] = gin[w];
+        __syncthreads();
+        uint64_t cnt = 0;
+        if (threadIdx.x < nr)
+            cnt = block_row(p, rows_s + threadIdx.x * k, coll_s + threadIdx.x * p.n_eq, lo_s[threadIdx.x],
+                            ncol_s[threadIdx.x]);
+        uint64_t total;
+        offs_s[threadIdx.x] = block_exclusive_scan(cnt, &total);
+        if (threadIdx.x == 0) offs_s[nr] = total;
+        __syncthreads();
+        if (!chunk) last = total;
 
-    uint64_t cnt = 0;
-    if (threadIdx.x < nr) {
+        const uint64_t out0 = __ldg(block_off + b);
+        for (uint64_t base = first; base < last; base += kThreads) {
+            const uint64_t o = base + threadIdx.x;
+            if (o < last) {
+                const int a = row_of(offs_s, (int)nr, o);
+                const uint32_t j = nth_candidate(lo_s[a], coll_s + a * p.n_eq, ncol_s[a], (uint32_t)(o - offs_s[a]));
+                uint32_t* dst = out_s + threadIdx.x * k1;
+                const uint32_t* src = rows_s + a * k;
+                for (uint32_t c = 0; c < k; ++c) dst[c] = src[c];
+                dst[k] = __ldg(p.adj + j);
+            }
+            __syncthreads();
+            const uint32_t n_tile = (uint32_t)umin64((uint64_t)kThreads, last - base);
+            uint32_t* gout = p.out + (out0 + base) * k1;
+            for (uint32_t w = threadIdx.x; w < n_tile * k1; w += kThreads) gout[w] = out_s[w];
+            __syncthreads();
+        }
+        if (!chunk) break;
+    }
+}
+
+// First index >= at in [at, hi) with adj[index] >= x (hi if none), looked for
+// from `at` outwards.
+__device__ __forceinline__ uint32_t gallop(const uint32_t* __restrict__ adj, uint32_t at, uint32_t hi, uint32_t x) {
+    uint32_t step = 1;
+    while (hi - at > step && __ldg(adj + at + step) < x) {
+        at += step;
+        step <<= 1;
+    }
+    return lower_bound_u32(adj, at, hi - at > step ? at + step : hi, x);
+}
+
+// An extension and the reduction after it in one: the extension's output rows
+// (counted, and placed in block_off, but never written) are tested as they
+// are generated, and only those that pass are written.  A row's candidates
+// come from the shorter of its list and the checked vertices' lists, cut to
+// the vertices between its first and last candidate of this chunk: the rows
+// kept, and their order, are those of the two steps.  A thread tests eight
+// consecutive candidates, searching the other list from where it found the
+// last one.  The count pass keeps its verdicts (a byte per eight candidates,
+// `mask_cap` per CTA) for the write pass.
+//
+// What bounds it: the loads of those searches.  24 million extension rows,
+// 1.2 million of them kept, on an R-MAT graph of 2^18 vertices: written,
+// counted and written again in 830 + 474 + 608 us as two steps.
+constexpr uint32_t kTestRun = 8;
+template <bool WRITE>
+__global__ void __launch_bounds__(kThreads) ext_red_kernel(ExtArgs p, const uint64_t* __restrict__ block_off,
+                                                           uint64_t nb, uint64_t chunk, uint64_t* __restrict__ sums,
+                                                           uint8_t* __restrict__ masks, uint32_t mask_cap) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    uint64_t* offs_s = reinterpret_cast<uint64_t*>(smem_raw);                  // 257
+    const uint32_t** gadj_s = reinterpret_cast<const uint32_t**>(offs_s + kRowsPerBlock + 1);  // 256
+    uint32_t* rows_s = reinterpret_cast<uint32_t*>(gadj_s + kRowsPerBlock);    // 256 * k
+    uint32_t* glo_s = rows_s + kRowsPerBlock * p.k;                            // 256: the candidates' list
+    uint32_t* ghi_s = glo_s + kRowsPerBlock;                                   // 256
+    uint32_t* slo_s = ghi_s + kRowsPerBlock;                                   // 256: the list searched
+    uint32_t* shi_s = slo_s + kRowsPerBlock;                                   // 256
+    int* which_s = reinterpret_cast<int*>(shi_s + kRowsPerBlock);              // 256: check of the candidates' list
+    int* other_s = which_s + kRowsPerBlock;                                    // 256: check of the list searched
+    uint32_t* coll_s = reinterpret_cast<uint32_t*>(other_s + kRowsPerBlock);   // 256 * n_eq
+    constexpr int kSource = -1, kNone_ = -2;
+    const uint32_t k = p.k, k1 = p.k + 1;
+    const uint64_t o0 = blockIdx.x * chunk, o1 = o0 + chunk;
+    uint8_t* mask = masks + (uint64_t)blockIdx.x * mask_cap;
+    uint64_t done = 0;  // rows kept so far: by this thread (count), by the CTA (write)
+    for (uint64_t b = find_block(block_off, nb, o0); b < nb && block_key(block_off, b) < o1; ++b) {
+        uint64_t first, last;
+        block_part(block_off, b, o0, o1, first, last);
+        if (first >= last) continue;
+        const uint64_t row0 = b * kRowsPerBlock;
+        const uint32_t nr = (uint32_t)umin64((uint64_t)kRowsPerBlock, p.nrows - row0);
+        const uint32_t* gin = p.in + row0 * k;
+        for (uint32_t w = threadIdx.x; w < nr * k; w += kThreads) rows_s[w] = gin[w];
+        __syncthreads();
         const uint32_t* row = rows_s + threadIdx.x * k;
-        uint32_t lo, hi;
-        ext_range(p, row, lo, hi);
-        uint32_t nc = 0;
-        uint32_t* mine = coll_s + threadIdx.x * p.n_eq;
-        if (lo < hi) {
-            for (uint32_t j = 0; j < p.n_eq; ++j) {
-                const uint32_t pos = find_in(p.adj, lo, hi, row[p.eq_cols[j]]);
-                if (pos == 0xffffffffu) continue;
-                bool dup = false;
-                for (uint32_t i = 0; i < nc; ++i) dup |= (mine[i] == pos);
-                if (dup) continue;
-                uint32_t i = nc++;  // insertion sort, ascending
-                while (i > 0 && mine[i - 1] > pos) {
-                    mine[i] = mine[i - 1];
-                    --i;
+        uint32_t* coll = coll_s + threadIdx.x * p.n_eq;
+        uint32_t lo = 0, nc = 0;
+        uint64_t cnt = 0, total;
+        if (threadIdx.x < nr) cnt = block_row(p, row, coll, lo, nc);
+        const uint64_t before = block_exclusive_scan(cnt, &total);
+        // this row's part of the chunk, as list positions [slo, shi); its
+        // candidates are those of the shortest list
+        uint32_t slo = 0, shi = 0, glo = 0, ghi = 0;
+        int which = kSource, other = kNone_;
+        const uint32_t* gadj = p.adj;
+        if (cnt && before < last && before + cnt > first) {
+            const uint32_t u0 = first > before ? (uint32_t)(first - before) : 0;
+            const uint32_t u1 = (uint32_t)umin64(cnt, last - before);
+            glo = nth_candidate(lo, coll, nc, u0);
+            ghi = nth_candidate(lo, coll, nc, u1 - 1) + 1;
+            const uint32_t v0 = __ldg(p.adj + glo);
+            const uint64_t v1 = (uint64_t)__ldg(p.adj + ghi - 1) + 1;
+            for (uint32_t i = 0; i < p.n_chk; ++i) {
+                if (p.chk_dir[i]) continue;
+                uint32_t cl, ch;
+                seg_of(p.chk_off[i], p.L, row[p.chk_col[i]], p.chk_lab[i], cl, ch);
+                cl = lower_bound_u32(p.chk_adj[i], cl, ch, v0);
+                ch = lower_bound_u32(p.chk_adj[i], cl, ch, v1);
+                if (ch - cl < ghi - glo) {  // the new shortest; the old one is searched
+                    slo = glo;
+                    shi = ghi;
+                    other = which;
+                    glo = cl;
+                    ghi = ch;
+                    gadj = p.chk_adj[i];
+                    which = (int)i;
+                } else if (other == kNone_) {
+                    slo = cl;
+                    shi = ch;
+                    other = (int)i;
                 }
-                mine[i] = pos;
             }
-            cnt = hi - lo - nc;
         }
-        lo_s[threadIdx.x] = lo;
-        ncol_s[threadIdx.x] = nc;
-    }
-    uint64_t total;
-    const uint64_t before = block_exclusive_scan(cnt, &total);
-    offs_s[threadIdx.x] = before;
-    if (threadIdx.x == 0) offs_s[nr] = total;
-    __syncthreads();
-
-    const uint64_t out0 = block_off[blockIdx.x];
-    for (uint64_t base = 0; base < total; base += kThreads) {
-        const uint64_t o = base + threadIdx.x;
-        if (o < total) {
-            // largest r with offs_s[r] <= o; rows with no candidate are skipped
-            int a = 0, b = (int)nr - 1;
-            while (a < b) {
-                const int m = (a + b + 1) >> 1;
-                if (offs_s[m] <= o)
-                    a = m;
-                else
-                    b = m - 1;
+        slo_s[threadIdx.x] = slo;
+        shi_s[threadIdx.x] = shi;
+        glo_s[threadIdx.x] = glo;
+        ghi_s[threadIdx.x] = ghi;
+        gadj_s[threadIdx.x] = gadj;
+        which_s[threadIdx.x] = which;
+        other_s[threadIdx.x] = other;
+        offs_s[threadIdx.x] = block_exclusive_scan((ghi - glo + kTestRun - 1) / kTestRun, &total);
+        __syncthreads();
+        for (uint64_t base = 0; base < total; base += kThreads) {
+            const uint64_t o = base + threadIdx.x;
+            uint32_t m = 0, x = 0;
+            int a = 0;
+            if (o < total) {
+                a = row_of(offs_s, kRowsPerBlock, o);
+                x = glo_s[a] + (uint32_t)(o - offs_s[a]) * kTestRun;
+                if (WRITE) m = mask[o];
             }
-            uint32_t j = lo_s[a] + (uint32_t)(o - offs_s[a]);
-            const uint32_t* mine = coll_s + a * p.n_eq;
-            for (uint32_t c = 0; c < ncol_s[a]; ++c) j += (mine[c] <= j) ? 1u : 0u;
-            uint32_t* dst = out_s + threadIdx.x * k1;
-            const uint32_t* src = rows_s + a * k;
-            for (uint32_t c = 0; c < k; ++c) dst[c] = src[c];
-            dst[k] = __ldg(p.adj + j);
+            if (!WRITE && o < total) {
+                const uint32_t* r = rows_s + a * k;
+                const uint32_t* g = gadj_s[a];
+                const int wh = which_s[a], ot = other_s[a];
+                const uint32_t* oadj = ot >= 0 ? p.chk_adj[ot] : p.adj;
+                const uint32_t n = min(kTestRun, ghi_s[a] - x), oh = shi_s[a];
+                uint32_t at = slo_s[a];
+                for (uint32_t i = 0; i < n; ++i) {
+                    const uint32_t c = __ldg(g + x + i);
+                    bool ok = true;
+                    for (uint32_t j = 0; j < p.n_eq && ok; ++j) ok = r[p.eq_cols[j]] != c;
+                    if (ok && ot != kNone_) {
+                        at = i ? gallop(oadj, at, oh, c) : lower_bound_u32(oadj, at, oh, c);
+                        ok = at < oh && __ldg(oadj + at) == c;
+                    }
+                    for (int j = 0; j < (int)p.n_chk && ok; ++j) {
+                        if (j == wh || j == ot) continue;
+                        ok = p.chk_dir[j] ? seg_has(p.chk_off[j], p.chk_adj[j], p.L, c, p.chk_lab[j], r[p.chk_col[j]])
+                                          : seg_has(p.chk_off[j], p.chk_adj[j], p.L, r[p.chk_col[j]], p.chk_lab[j], c);
+                    }
+                    // with three lists or more the source's may be neither
+                    if (ok && wh != kSource && ot != kSource) {
+                        uint32_t sl, sh;
+                        ext_range(p, r, sl, sh);
+                        ok = find_in(p.adj, sl, sh, c) != 0xffffffffu;
+                    }
+                    if (ok) m |= 1u << i;
+                }
+                mask[o] = (uint8_t)m;
+                done += __popc(m);
+            }
+            if (WRITE) {
+                uint64_t kept;
+                const uint64_t at = block_exclusive_scan(__popc(m), &kept);
+                uint32_t* dst = p.out + (sums[blockIdx.x] + done + at) * k1;
+                const uint32_t* r = rows_s + a * k;
+                while (m) {
+                    const uint32_t i = __ffs(m) - 1;
+                    m &= m - 1;
+                    for (uint32_t j = 0; j < k; ++j) dst[j] = r[j];
+                    dst[k] = __ldg(gadj_s[a] + x + i);
+                    dst += k1;
+                }
+                done += kept;
+            }
         }
-        __syncthreads();
-        const uint32_t n_tile = (uint32_t)umin64((uint64_t)kThreads, total - base);
-        uint32_t* gout = p.out + (out0 + base) * k1;
-        for (uint32_t w = threadIdx.x; w < n_tile * k1; w += kThreads) gout[w] = out_s[w];
-        __syncthreads();
+        mask += total;
+        __syncthreads();  // every thread done with this block's rows
     }
+    if (!WRITE) store_block_sum(done, sums);
 }
 
 __global__ void __launch_bounds__(kThreads) red_write_kernel(RedArgs p, const uint64_t* __restrict__ block_off) {
@@ -157,10 +385,64 @@ __global__ void __launch_bounds__(kThreads) red_write_kernel(RedArgs p, const ui
     for (uint32_t w = threadIdx.x; w < (uint32_t)total * k; w += kThreads) gout[w] = out_s[w];
 }
 
+// The same scan as scan_block_sums_kernel by one cluster: every thread takes a
+// contiguous share, the CTAs exchange their sums through distributed shared
+// memory.  94,578 sums: 93 us with one CTA.
+constexpr int kScanCtas = 8;
+__global__ void __cluster_dims__(kScanCtas, 1, 1) __launch_bounds__(kScanThreads)
+scan_cluster_kernel(uint64_t* __restrict__ sums, uint64_t n) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    __shared__ uint64_t ws[32];
+    __shared__ uint64_t mine;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint64_t all = (uint64_t)kScanCtas * kScanThreads, per = (n + all - 1) / all;
+    const uint64_t me = (uint64_t)blockIdx.x * kScanThreads + threadIdx.x;
+    const uint64_t b = umin64(n, me * per), e = umin64(n, b + per);
+    uint64_t v = 0;
+    for (uint64_t i = b; i < e; ++i) v += sums[i];
+    uint64_t inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    if (lane == 31) ws[wid] = inc;
+    __syncthreads();
+    if (wid == 0) {
+        uint64_t w = ws[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t y = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += y;
+        }
+        ws[lane] = w;
+        if (lane == 31) mine = w;
+    }
+    cl.sync();
+    uint64_t at = (wid > 0 ? ws[wid - 1] : 0) + inc - v, total = 0;
+    for (uint32_t r = 0; r < kScanCtas; ++r) {
+        const uint64_t x = *cl.map_shared_rank(&mine, r);
+        if (r < cl.block_rank()) at += x;
+        total += x;
+    }
+    for (uint64_t i = b; i < e; ++i) {
+        const uint64_t x = sums[i];
+        sums[i] = at;
+        at += x;
+    }
+    if (me == 0) sums[n] = total;
+    cl.sync();  // no CTA leaves while another reads its sum
+}
+
 size_t ext_smem_bytes(uint32_t k, uint32_t n_eq) {
     return sizeof(uint64_t) * (kRowsPerBlock + 1) +
            sizeof(uint32_t) * ((size_t)kRowsPerBlock * k + 2 * kRowsPerBlock + (size_t)kRowsPerBlock * n_eq +
                                (size_t)kRowsPerBlock * (k + 1));
+}
+size_t ext_red_smem_bytes(uint32_t k, uint32_t n_eq) {
+    return sizeof(uint64_t) * (2 * kRowsPerBlock + 1) +
+           sizeof(uint32_t) * ((size_t)kRowsPerBlock * k + 6 * kRowsPerBlock + (size_t)kRowsPerBlock * n_eq);
 }
 size_t red_smem_bytes(uint32_t k) { return sizeof(uint32_t) * 2 * (size_t)kRowsPerBlock * k; }
 
@@ -173,6 +455,9 @@ int set_smem_limits() {
     if (dev < 64 && done[dev].load(std::memory_order_acquire)) return GVA_OK;
     GVA_CUDA(cudaFuncSetAttribute(ext_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)ext_smem_bytes(kMaxCols - 1, kMaxCols)));
+    for (const void* fn : {(const void*)ext_red_kernel<false>, (const void*)ext_red_kernel<true>})
+        GVA_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)ext_red_smem_bytes(kMaxCols - 1, kMaxCols)));
     GVA_CUDA(cudaFuncSetAttribute(red_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)red_smem_bytes(kMaxCols)));
     if (dev < 64) done[dev].store(true, std::memory_order_release);
@@ -215,6 +500,47 @@ void fill_red(RedArgs& a, const DevDB& db, const Step& st, const uint32_t* in, u
     }
 }
 
+// Ordinals of one CTA of an extension's write (block_key): about 24 CTAs per
+// SM, at least a block's worth and at most 32,768.  On a graph without long
+// lists the blocks' outputs are alike and a CTA takes its block without a
+// search (chunk 0; 6.0 against 8.6 us for 1,144 blocks).
+uint64_t chunk_of(uint64_t total, uint64_t nb) {
+    const uint64_t all = total + nb * kBlockWork;
+    return std::min<uint64_t>(std::max<uint64_t>((all + 148 * 24 - 1) / (148 * 24), kBlockWork + 256), 32768);
+}
+uint64_t num_chunks(uint64_t total, uint64_t nb) {
+    const uint64_t c = chunk_of(total, nb);
+    return (total + nb * kBlockWork + c - 1) / c;
+}
+
+// Verdict bytes of one CTA of ext_red_kernel: one per eight candidates, and
+// per row of the blocks that a chunk meets a started one and its matched
+// vertices' (n_eq candidates more than output rows).
+uint32_t mask_cap(uint64_t chunk, uint32_t n_eq) {
+    return (uint32_t)(chunk / kTestRun + (kRowsPerBlock + kRowsPerBlock / kTestRun * n_eq) * (chunk / kBlockWork + 2));
+}
+
+// Exclusive scan of n block sums in place, their total in sums[n].
+void launch_scan(uint64_t* sums, uint64_t n, cudaStream_t s) {
+    if (n <= 4096)
+        scan_block_sums_kernel<<<1, kScanThreads, 0, s>>>(sums, n);
+    else
+        scan_cluster_kernel<<<kScanCtas, kScanThreads, 0, s>>>(sums, n);
+}
+
+// Whether reduction `r` only checks edges of the vertex that extension `e`
+// adds, so that ext_red_kernel can run both.
+bool can_fuse(const DevDB& db, const Step& e, const Step& r) {
+    if (db.max_degree <= kEvenDegree) return false;  // frontiers are small: the two steps are as fast
+    if (e.kind != STEP_EXT || r.kind != STEP_REDUCE || e.always_empty || r.always_empty) return false;
+    if (r.n_pairs == 0 || r.n_pairs > (uint32_t)kMaxChecks || r.width_in != e.width_in + 1) return false;
+    for (const Step* st : {&e, &r})
+        if (st->part == 0 || st->part > db.parts.size() || !db.parts[st->part - 1].off) return false;
+    for (uint32_t i = 0; i < r.n_pairs; ++i)
+        if ((r.rs_col[i] == e.width_in) == (r.re_col[i] == e.width_in)) return false;
+    return true;
+}
+
 // count + scan; leaves exclusive block offsets in sums[0..nb) and the total in sums[nb]
 int launch_count(const DevDB& db, const Step& st, const uint32_t* in, uint64_t nrows, uint64_t* sums,
                  cudaStream_t s, Profiler* prof) {
@@ -240,7 +566,7 @@ int launch_count(const DevDB& db, const Step& st, const uint32_t* in, uint64_t n
     GVA_CUDA(cudaGetLastError());
     const double sbytes = 16.0 * (double)nb;
     if (prof) prof->begin(K_SCAN, sbytes, s, ev);
-    scan_block_sums_kernel<<<1, kScanThreads, 0, s>>>(sums, nb);
+    launch_scan(sums, nb, s);
     if (prof) prof->end(ev, K_SCAN, sbytes, s, (double)nb);
     GVA_CUDA(cudaGetLastError());
     g_launches += 2;
@@ -259,7 +585,11 @@ int launch_write(const DevDB& db, const Step& st, const uint32_t* in, uint64_t n
         fill_ext(a, db, st, in, nrows, out);
         const double bytes = (4.0 * k + 8.0) * (double)nrows + (4.0 + 4.0 * (k + 1)) * (double)nout;
         if (prof) prof->begin(K_EXT_WRITE, bytes, s, ev);
-        ext_write_kernel<<<(unsigned)nb, kThreads, ext_smem_bytes(a.k, a.n_eq), s>>>(a, sums);
+        const bool even = db.max_degree <= kEvenDegree;
+        const uint64_t nch = even ? nb : num_chunks(nout, nb);
+        if (nch > 0x7fffffffull) return fail(GVA_ERR_UNSUPPORTED, "frontier too large for one launch");
+        ext_write_kernel<<<(unsigned)nch, kThreads, ext_smem_bytes(a.k, a.n_eq), s>>>(a, sums, nb,
+                                                                                      even ? 0 : chunk_of(nout, nb));
         if (prof) prof->end(ev, K_EXT_WRITE, bytes, s, (double)nrows);
     } else {
         RedArgs a;
@@ -271,6 +601,56 @@ int launch_write(const DevDB& db, const Step& st, const uint32_t* in, uint64_t n
     }
     GVA_CUDA(cudaGetLastError());
     g_launches += 1;
+    return GVA_OK;
+}
+
+// The counted rows of extension `st` (offsets in sums, `total` rows) that pass
+// reduction `rd`: counted per CTA into csums and scanned (out null), or
+// written to out at the scanned offsets.
+int launch_ext_red(const DevDB& db, const Step& st, const Step& rd, const uint32_t* in, uint64_t nrows, uint64_t total,
+                   const uint64_t* sums, uint64_t* csums, uint8_t* masks, uint32_t* out, uint64_t kept, cudaStream_t s,
+                   Profiler* prof) {
+    int rc = set_smem_limits();
+    if (rc) return rc;
+    const uint64_t nb = (nrows + kRowsPerBlock - 1) / kRowsPerBlock, nch = num_chunks(total, nb);
+    if (nch > 0x7fffffffull) return fail(GVA_ERR_UNSUPPORTED, "frontier too large for one launch");
+    ExtArgs a;
+    fill_ext(a, db, st, in, nrows, out);
+    const DevPart& P = db.parts[rd.part - 1];
+    a.n_chk = rd.n_pairs;
+    for (uint32_t i = 0; i < rd.n_pairs; ++i) {
+        // the new vertex on the right: it must lie in the partner's segment;
+        // on the left: the partner in the new vertex's
+        a.chk_dir[i] = rd.rs_col[i] == st.width_in ? 1 : 0;
+        a.chk_col[i] = a.chk_dir[i] ? rd.re_col[i] : rd.rs_col[i];
+        a.chk_lab[i] = rd.re_label[i];
+        a.chk_off[i] = P.off;
+        a.chk_adj[i] = P.adj;
+    }
+    const double k = st.width_in;
+    cudaEvent_t ev = nullptr;
+    const size_t smem = ext_red_smem_bytes(a.k, a.n_eq);
+    if (!out) {
+        const double bytes = (4.0 * k + 8.0) * (double)nrows + (4.0 + 8.0 * rd.n_pairs) * (double)total;
+        if (prof) prof->begin(K_RED_COUNT, bytes, s, ev);
+        ext_red_kernel<false><<<(unsigned)nch, kThreads, smem, s>>>(a, sums, nb, chunk_of(total, nb), csums, masks,
+                                                                        mask_cap(chunk_of(total, nb), a.n_eq));
+        if (prof) prof->end(ev, K_RED_COUNT, bytes, s, (double)total);
+        GVA_CUDA(cudaGetLastError());
+        if (prof) prof->begin(K_SCAN, 16.0 * (double)nch, s, ev);
+        launch_scan(csums, nch, s);
+        if (prof) prof->end(ev, K_SCAN, 16.0 * (double)nch, s, (double)nch);
+        g_launches += 2;
+    } else {
+        const double bytes = (4.0 * k + 8.0) * (double)nrows + (4.0 + 8.0 * rd.n_pairs) * (double)total +
+                             4.0 * (k + 1) * (double)kept;
+        if (prof) prof->begin(K_RED_WRITE, bytes, s, ev);
+        ext_red_kernel<true><<<(unsigned)nch, kThreads, smem, s>>>(a, sums, nb, chunk_of(total, nb), csums, masks,
+                                                                        mask_cap(chunk_of(total, nb), a.n_eq));
+        if (prof) prof->end(ev, K_RED_WRITE, bytes, s, (double)total);
+        g_launches += 1;
+    }
+    GVA_CUDA(cudaGetLastError());
     return GVA_OK;
 }
 
@@ -569,7 +949,57 @@ int run_match(DevDB& db, const Plan& plan, const std::vector<Step>& steps, cudaS
             ce = cudaMemcpyAsync(total_h, sums + nb, 8, cudaMemcpyDeviceToHost, s);
             if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
             if (ce != cudaSuccess) { status = fail(GVA_ERR_CUDA, cudaGetErrorString(ce)); break; }
-            const uint64_t total = *total_h;
+            uint64_t total = *total_h;
+            if (total > 0 && !last && can_fuse(db, st, steps[i + 1])) {
+                // this extension's rows are only needed by the reduction
+                // after it: tested as they are generated, never written
+                if (total * out_w * 4ull > budget) {
+                    status = fail(GVA_ERR_NOMEM, "frontier of " + std::to_string(total) + " rows exceeds the memory budget");
+                    break;
+                }
+                if (st.phase_end >= 0) res.phase_rows[st.phase_end] = total;
+                const Step& rd = steps[i + 1];
+                const uint64_t nch = num_chunks(total, nb);
+                uint64_t* csums = nullptr;
+                ce = cudaMallocAsync((void**)&csums, (nch + 1) * 8 + nch * mask_cap(chunk_of(total, nb), st.n_eq), s);
+                if (ce != cudaSuccess) { status = fail(GVA_ERR_NOMEM, "scratch allocation failed"); break; }
+                uint8_t* masks = (uint8_t*)(csums + nch + 1);
+                status = launch_ext_red(db, st, rd, cur, rows, total, sums, csums, masks, nullptr, 0, s, prof);
+                uint64_t kept = 0;
+                if (!status) {
+                    ce = cudaMemcpyAsync(total_h, csums + nch, 8, cudaMemcpyDeviceToHost, s);
+                    if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
+                    if (ce != cudaSuccess) status = fail(GVA_ERR_CUDA, cudaGetErrorString(ce));
+                    kept = *total_h;
+                }
+                uint32_t* out = nullptr;
+                const bool only_count = i + 2 == steps.size() && count_only;
+                if (!status && kept && !only_count) {
+                    if (kept * out_w * 4ull > budget) {
+                        status = fail(GVA_ERR_NOMEM, "frontier of " + std::to_string(kept) + " rows exceeds the memory budget");
+                    } else if (cudaMallocAsync((void**)&out, kept * out_w * 4ull, s) != cudaSuccess) {
+                        out = nullptr;
+                        status = fail(GVA_ERR_NOMEM, "frontier allocation failed");
+                    } else {
+                        status = launch_ext_red(db, st, rd, cur, rows, total, sums, csums, masks, out, kept, s, prof);
+                        if (status) cudaFreeAsync(out, s);
+                    }
+                }
+                cudaFreeAsync(csums, s);
+                if (status) break;
+                if (out) {
+                    if (owned) cudaFreeAsync(owned, s);
+                    owned = out;
+                    cur = out;
+                }
+                rows = kept;
+                counted_only = only_count;
+                width = out_w;
+                if (rd.phase_end >= 0) res.phase_rows[rd.phase_end] = rows;
+                ++i;
+                if (rows == 0) break;
+                continue;
+            }
             if (last && count_only) {
                 rows = total;
                 counted_only = true;

@@ -1,0 +1,75 @@
+"""gva_match on lists far longer than a CTA's share of an extension's output:
+rows, their order and the phase counts against the oracle."""
+import numpy as np
+import pytest
+
+import geneva_b200 as gv
+
+pytestmark = pytest.mark.gpu
+
+
+def hub_graph(leaves, hubs, seed):
+    """Hubs (label 1) joined to all of their own `leaves` leaves (labels 2 and
+    3), random edges among leaves of neighbouring hubs, hubs in a path."""
+    rng = np.random.default_rng(seed)
+    n = hubs * (1 + leaves)
+    labels = np.zeros(n + 1, np.uint32)
+    labels[1:] = rng.integers(2, 4, n)
+    edges = set()
+    hub_ids = [1 + h * (1 + leaves) for h in range(hubs)]
+    for h, hub in enumerate(hub_ids):
+        labels[hub] = 1
+        edges |= {(hub, hub + 1 + i) for i in range(leaves)}
+        if h:
+            edges.add((hub_ids[h - 1], hub))
+    while len(edges) < n + 2 * leaves:
+        a, b = sorted(int(x) for x in rng.integers(1, n + 1, 2))
+        if a != b and labels[a] != 1 and labels[b] != 1:
+            edges.add((a, b))
+    e = np.array(sorted(edges), np.uint32)
+    return labels, e[:, 0], e[:, 1], np.ones(len(e), np.uint32)
+
+
+QUERIES = [
+    "v 0 1\nv 1 2\nv 2 3\ne 0 1 1\ne 0 2 1\n",                               # no reduction
+    "v 0 1\nv 1 2\nv 2 3\ne 0 1 1\ne 0 2 1\ne 1 2 1\n",                       # a triangle
+    "v 0 1\nv 1 2\nv 2 2\ne 0 1 1\ne 0 2 1\ne 1 2 1\n",                       # with a restriction
+    "v 0 1\nv 1 2\nv 2 3\nv 3 3\ne 0 1 1\ne 0 2 1\ne 1 2 1\ne 0 3 1\n",       # and a tail
+    "v 0 1\nv 1 2\nv 2 3\nv 3 2\ne 0 1 1\ne 1 2 1\ne 2 3 1\ne 0 3 1\n",       # a square
+    "v 0 1\nv 1 1\nv 2 2\ne 0 1 1\ne 0 2 1\n",
+]
+
+
+@pytest.mark.parametrize("leaves,hubs", [(3, 2), (255, 1), (1300, 2), (5000, 1)])
+def test_rows_against_oracle(native, oracle, leaves, hubs):
+    labels, src, dst, el = hub_graph(leaves, hubs, leaves)
+    db = gv.Database.from_edges(labels, src, dst, el)
+    og = oracle.from_edges(labels, src, dst, el)
+    for text in QUERIES:
+        want, phases = oracle.match(og, text)
+        for mode in (gv.MODE_DV, gv.MODE_SV):
+            plan = gv.Plan.from_text(text, mode)
+            res = gv.match(db, plan)
+            rows = res.rows()
+            if mode == gv.MODE_DV:
+                assert res.phase_rows == phases, text
+            # every step takes its rows in order and their candidates ascending
+            assert np.array_equal(rows, want[np.lexsort(want.T[::-1])]), text
+            counted = gv.match(db, plan, count_only=True)
+            assert counted.num_rows == len(want) and counted.phase_rows == res.phase_rows
+    oracle.free(og)
+    db.close()
+
+
+def test_budget_still_refuses_the_extension(native):
+    """An extension whose rows exceed the budget is refused although the
+    reduction after it means that they are never written."""
+    labels, src, dst, el = hub_graph(1300, 2, 7)
+    db = gv.Database.from_edges(labels, src, dst, el)
+    plan = gv.Plan.from_text(QUERIES[1])
+    res = gv.match(db, plan)
+    assert res.num_rows > 0
+    kept = 12 * res.num_rows
+    with pytest.raises(gv.GenevaError):
+        gv.match(db, plan, budget_bytes=2 * kept)
+    db.close()
