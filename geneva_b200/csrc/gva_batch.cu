@@ -2390,12 +2390,12 @@ static uint32_t resident_ctas(int device, const void* fn, size_t smem) {
 // Freed memory stays in it for the next run; what is more than the regions of
 // two runs side by side at their first size (9 GiB) goes back to the driver
 // when a database is freed.
-static cudaMemPool_t round_pool(int device) {
+static cudaMemPool_t round_pool(int device, bool make = true) {
     static std::mutex mu;
     static cudaMemPool_t pools[64] = {};
     if (device < 0 || device >= 64) return nullptr;
     std::lock_guard<std::mutex> lk(mu);
-    if (!pools[device]) {
+    if (!pools[device] && make) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -2413,7 +2413,7 @@ static cudaMemPool_t round_pool(int device) {
 }
 
 void trim_round_pool(int device) {
-    cudaMemPool_t pool = round_pool(device);
+    cudaMemPool_t pool = round_pool(device, false);
     if (pool) cudaMemPoolTrimTo(pool, (size_t)9 << 30);
 }
 

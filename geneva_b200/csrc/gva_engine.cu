@@ -385,6 +385,214 @@ __global__ void __launch_bounds__(kThreads) red_write_kernel(RedArgs p, const ui
     for (uint32_t w = threadIdx.x; w < (uint32_t)total * k; w += kThreads) gout[w] = out_s[w];
 }
 
+// ------------------------------------------------------- steps in a chain ---
+// On a graph without long lists a query's steps are launched one after another
+// without a look at their totals: a step counts, places and writes its rows in
+// one pass (tiles of 256 input rows, taken in order from a counter; a tile's
+// place is the sum of the tiles before it, looked back for while they run),
+// takes its input's length from the step before it, and the host reads all
+// totals at the end.  Rows and order are those of the counted steps.
+//
+// What bounds it: latency.  A query of three steps on a 1,000-graph database
+// has 30 us of kernels; the host's look at every total (copy, wait, allocate,
+// launch) made it 112 us, the chain takes 48.  (Looking back by the whole CTA,
+// 256 tiles at a time, was slower: 18 against 16 us for 1,144 tiles.)
+struct Chain {
+    const uint64_t* n_in;            // rows of the input (null: p.nrows)
+    uint64_t cap_in, cap_out;        // rows that the input / output has room for
+    unsigned long long* tiles;       // next tile
+    unsigned long long* status;      // per tile: 1 << 62 | rows, then 2 << 62 | rows up to here
+    uint64_t* n_out;                 // rows of the output
+    uint64_t* host_out;              // the same, in host memory
+    uint32_t* failed;                // 1: an output has no room, 2: a wait ran out
+    uint32_t* host_failed;
+};
+constexpr uint32_t kWaitPolls = 1u << 20;  // of a tile for the ones before it, then the chain fails
+
+__device__ __forceinline__ void chain_fail(const Chain& c, uint32_t why) {
+    *(volatile uint32_t*)c.failed = why;
+    *(volatile uint32_t*)c.host_failed = why;
+    __threadfence_system();
+}
+
+// Rows of a step's input: none once a step has failed (its rows were not all
+// written).  A CTA that starts late may find its own step's failure; the CTAs
+// that found none take all of its tiles, so that the total is known.
+__device__ __forceinline__ uint64_t chain_rows(const Chain& c, uint64_t nrows) {
+    __shared__ uint64_t n;
+    if (threadIdx.x == 0)
+        n = *(volatile uint32_t*)c.failed ? 0 : c.n_in ? umin64(*c.n_in, c.cap_in) : nrows;
+    __syncthreads();
+    return n;
+}
+
+// Whether the CTAs with lower numbers are as many as the tiles: this one need
+// take none.
+__device__ __forceinline__ bool chain_idle(uint64_t n) { return (uint64_t)blockIdx.x * kRowsPerBlock >= n; }
+
+// The next tile, for every thread of the CTA.
+__device__ __forceinline__ uint64_t chain_tile(const Chain& c) {
+    __shared__ uint64_t tile;
+    __syncthreads();  // the last one was read by every thread
+    if (threadIdx.x == 0) tile = atomicAdd(c.tiles, 1ull);
+    __syncthreads();
+    return tile;
+}
+
+// Rows before `tile`, whose own number is `total`; ~0: the wait ran out.
+// Tiles are taken in order, so the ones waited for are done or running.
+__device__ __forceinline__ uint64_t chain_place(const Chain& c, uint64_t tile, uint64_t total) {
+    __shared__ uint64_t place;
+    constexpr unsigned long long kHas = 1ull << 62, kDone = 2ull << 62, kMask = kHas - 1;
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        volatile unsigned long long* status = c.status;
+        uint64_t sum = 0;
+        bool ok = true;
+        if (tile > 0) {
+            if (lane == 0) status[tile] = kHas | total;
+            uint32_t polls = 0;
+            for (int64_t at = (int64_t)tile - 1; ok;) {
+                const int64_t i = at - lane;
+                const unsigned long long w = i >= 0 ? status[i] : kDone;
+                const uint32_t done = __ballot_sync(0xffffffffu, (w >> 62) == 2);
+                const uint32_t none = __ballot_sync(0xffffffffu, (w >> 62) == 0);
+                // lanes up to the nearest finished prefix
+                const uint32_t upto = done ? (done & -done) | ((done & -done) - 1) : 0xffffffffu;
+                if (none & upto) {
+                    ok = ++polls < kWaitPolls;
+                    continue;
+                }
+                sum += __shfl_sync(0xffffffffu, warp_sum((upto >> lane & 1) ? (uint64_t)(w & kMask) : 0), 0);
+                if (done) break;
+                at -= 32;
+            }
+        }
+        if (lane == 0) {
+            if (ok)
+                status[tile] = kDone | (sum + total);
+            else
+                chain_fail(c, 2);
+            place = ok ? sum : ~0ull;
+        }
+    }
+    __syncthreads();
+    return place;
+}
+
+// The tile's rows are placed: the last one tells the total.  Returns whether
+// they may be written.
+__device__ __forceinline__ bool chain_end(const Chain& c, uint64_t tile, uint64_t n, uint64_t place, uint64_t total) {
+    const bool room = place + total <= c.cap_out;
+    if (threadIdx.x == 0) {
+        if (!room) chain_fail(c, 1);
+        if ((tile + 1) * kRowsPerBlock >= n) {
+            *c.n_out = place + total;
+            *(volatile uint64_t*)c.host_out = place + total;
+        }
+    }
+    return room;
+}
+
+__global__ void __launch_bounds__(kThreads) chain_ext_kernel(ExtArgs p, Chain c) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    uint64_t* offs_s = reinterpret_cast<uint64_t*>(smem_raw);           // 257
+    uint32_t* rows_s = reinterpret_cast<uint32_t*>(offs_s + kRowsPerBlock + 1);  // 256 * k
+    uint32_t* lo_s = rows_s + kRowsPerBlock * p.k;                        // 256
+    uint32_t* ncol_s = lo_s + kRowsPerBlock;                              // 256
+    uint32_t* coll_s = ncol_s + kRowsPerBlock;                            // 256 * n_eq
+    uint32_t* out_s = coll_s + kRowsPerBlock * p.n_eq;                    // 256 * (k + 1)
+    const uint32_t k = p.k, k1 = p.k + 1;
+    const uint64_t n = chain_rows(c, p.nrows);
+    if (chain_idle(n)) return;
+    for (;;) {
+        const uint64_t tile = chain_tile(c), row0 = tile * kRowsPerBlock;
+        if (row0 >= n) return;
+        const uint32_t nr = (uint32_t)umin64((uint64_t)kRowsPerBlock, n - row0);
+        const uint32_t* gin = p.in + row0 * k;
+        for (uint32_t w = threadIdx.x; w < nr * k; w += kThreads) rows_s[w] = gin[w];
+        __syncthreads();
+        uint64_t cnt = 0, total;
+        if (threadIdx.x < nr)
+            cnt = block_row(p, rows_s + threadIdx.x * k, coll_s + threadIdx.x * p.n_eq, lo_s[threadIdx.x],
+                            ncol_s[threadIdx.x]);
+        offs_s[threadIdx.x] = block_exclusive_scan(cnt, &total);
+        const uint64_t place = chain_place(c, tile, total);
+        if (place == ~0ull) return;
+        if (!chain_end(c, tile, n, place, total)) continue;  // counted only
+        for (uint64_t base = 0; base < total; base += kThreads) {
+            const uint64_t o = base + threadIdx.x;
+            if (o < total) {
+                const int a = row_of(offs_s, (int)nr, o);
+                const uint32_t j = nth_candidate(lo_s[a], coll_s + a * p.n_eq, ncol_s[a], (uint32_t)(o - offs_s[a]));
+                uint32_t* dst = out_s + threadIdx.x * k1;
+                const uint32_t* src = rows_s + a * k;
+                for (uint32_t i = 0; i < k; ++i) dst[i] = src[i];
+                dst[k] = __ldg(p.adj + j);
+            }
+            __syncthreads();
+            const uint32_t n_tile = (uint32_t)umin64((uint64_t)kThreads, total - base);
+            uint32_t* gout = p.out + (place + base) * k1;
+            for (uint32_t w = threadIdx.x; w < n_tile * k1; w += kThreads) gout[w] = out_s[w];
+            __syncthreads();
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) chain_red_kernel(RedArgs p, Chain c) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    uint32_t* rows_s = reinterpret_cast<uint32_t*>(smem_raw);
+    uint32_t* out_s = rows_s + kRowsPerBlock * p.k;
+    const uint32_t k = p.k;
+    const uint64_t n = chain_rows(c, p.nrows);
+    if (chain_idle(n)) return;
+    for (;;) {
+        const uint64_t tile = chain_tile(c), row0 = tile * kRowsPerBlock;
+        if (row0 >= n) return;
+        const uint32_t nr = (uint32_t)umin64((uint64_t)kRowsPerBlock, n - row0);
+        const uint32_t* gin = p.in + row0 * k;
+        for (uint32_t w = threadIdx.x; w < nr * k; w += kThreads) rows_s[w] = gin[w];
+        __syncthreads();
+        const bool keep = threadIdx.x < nr && red_keep_row(p, rows_s + threadIdx.x * k);
+        uint64_t total;
+        const uint64_t before = block_exclusive_scan(keep ? 1 : 0, &total);
+        const uint64_t place = chain_place(c, tile, total);
+        if (place == ~0ull) return;
+        if (!chain_end(c, tile, n, place, total)) continue;  // counted only
+        if (keep)
+            for (uint32_t i = 0; i < k; ++i) out_s[before * k + i] = rows_s[threadIdx.x * k + i];
+        __syncthreads();
+        uint32_t* gout = p.out + place * k;
+        for (uint32_t w = threadIdx.x; w < (uint32_t)total * k; w += kThreads) gout[w] = out_s[w];
+    }
+}
+
+// The last step of a counted query: only its total.  c.status[0] counts the
+// CTAs that have added theirs.
+template <class Args>
+__global__ void __launch_bounds__(kThreads) chain_count_kernel(Args p, Chain c) {
+    const uint64_t n = chain_rows(c, p.nrows);
+    uint64_t v = 0;
+    for (uint64_t r = (uint64_t)blockIdx.x * kThreads + threadIdx.x; r < n; r += (uint64_t)gridDim.x * kThreads) {
+        if constexpr (sizeof(Args) == sizeof(ExtArgs))
+            v += ext_count_plain(p, p.in + r * p.k);
+        else
+            v += red_keep_row(p, p.in + r * p.k) ? 1 : 0;
+    }
+    __shared__ uint64_t ws[kThreads / 32];
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < kThreads / 32; ++i) v += ws[i];
+        if (v) atomicAdd((unsigned long long*)c.n_out, (unsigned long long)v);
+        __threadfence();
+        if (atomicAdd(c.status, 1ull) + 1 == gridDim.x)
+            *(volatile uint64_t*)c.host_out = atomicAdd((unsigned long long*)c.n_out, 0ull);
+    }
+}
+static_assert(sizeof(ExtArgs) != sizeof(RedArgs), "told apart by their sizes");
+
 // The same scan as scan_block_sums_kernel by one cluster: every thread takes a
 // contiguous share, the CTAs exchange their sums through distributed shared
 // memory.  94,578 sums: 93 us with one CTA.
@@ -455,6 +663,10 @@ int set_smem_limits() {
     if (dev < 64 && done[dev].load(std::memory_order_acquire)) return GVA_OK;
     GVA_CUDA(cudaFuncSetAttribute(ext_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)ext_smem_bytes(kMaxCols - 1, kMaxCols)));
+    GVA_CUDA(cudaFuncSetAttribute(chain_ext_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)ext_smem_bytes(kMaxCols - 1, kMaxCols)));
+    GVA_CUDA(cudaFuncSetAttribute(chain_red_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)red_smem_bytes(kMaxCols)));
     for (const void* fn : {(const void*)ext_red_kernel<false>, (const void*)ext_red_kernel<true>})
         GVA_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)ext_red_smem_bytes(kMaxCols - 1, kMaxCols)));
@@ -667,11 +879,175 @@ int host_stage(int device, HostStage*& out) {
     if (device < 0 || device >= 64) return fail(GVA_ERR_ARG, "device index out of range");
     HostStage& h = stages[device];
     if (!h.pinned) {
-        GVA_CUDA(cudaMallocHost(&h.pinned, 64));
+        GVA_CUDA(cudaMallocHost(&h.pinned, 1024));
         GVA_CUDA(cudaEventCreate(&h.ev0));
         GVA_CUDA(cudaEventCreate(&h.ev1));
     }
     out = &h;
+    return GVA_OK;
+}
+
+// Rows of the first step's input up to which a query runs as a chain, and the
+// room of its result (a larger one is written by a second launch of the last
+// step).
+constexpr uint64_t kChainRows = 1ull << 22;
+constexpr size_t kChainResult = 256u << 10;
+constexpr size_t kChainSteps = 64;
+
+// Runs every step of a query at once (Chain).  `done` is set when the query is
+// finished: res and the totals are as run_match leaves them, `final` the last
+// step's rows.  Not set: the query does not qualify or an output had no room;
+// nothing is kept.
+int run_chain(DevDB& db, const std::vector<Step>& steps, cudaStream_t s, uint64_t budget, bool count_only,
+              HostStage* hs, std::vector<uint64_t>& totals, uint32_t*& final, bool& done) {
+    done = false;
+    final = nullptr;
+    const size_t n = steps.size();
+    if (db.max_degree > kEvenDegree || n < 2 || n > kChainSteps || steps[0].kind != STEP_SEED) return GVA_OK;
+    for (const Step& st : steps)
+        if (st.always_empty) return GVA_OK;
+    uint32_t wmax = 1;
+    for (size_t i = 1; i < n; ++i) {
+        const Step& st = steps[i];
+        if (st.kind == STEP_SEED || st.part == 0 || st.part > db.parts.size() || !db.parts[st.part - 1].off) return GVA_OK;
+        wmax = std::max(wmax, st.kind == STEP_EXT ? st.width_in + 1 : st.width_in);
+    }
+    const uint64_t rows0 = db.seed_off[steps[0].label + 1] - db.seed_off[steps[0].label];
+    if (rows0 == 0 || rows0 > kChainRows) return GVA_OK;
+    // room for four times the seeds in every step: the frontiers of labelled
+    // queries on such graphs mostly shrink
+    const uint64_t cap = 4 * rows0 + 65536;
+    const size_t bytes = cap * wmax * 4;
+    if (bytes > budget) return GVA_OK;
+    int rc = set_smem_limits();
+    if (rc) return rc;
+    const uint64_t most_tiles = (cap + kRowsPerBlock - 1) / kRowsPerBlock;
+    // control: failed | tile counters | totals | statuses (one step more, for
+    // the last step's second launch)
+    const size_t o_tiles = 8, o_tot = o_tiles + 8 * (n + 1), o_status = o_tot + 8 * (n + 1);
+    std::vector<size_t> status_at(n + 1);
+    size_t ctl = o_status;
+    for (size_t i = 1; i <= n; ++i) {
+        status_at[i] = ctl;
+        ctl += 8 * (i == 1 ? (rows0 + kRowsPerBlock - 1) / kRowsPerBlock : most_tiles);
+    }
+    const bool keep_rows = !count_only;
+    const size_t o_buf = align256(ctl), o_buf2 = o_buf + align256(bytes);
+    char* mem = nullptr;
+    uint32_t* fin = nullptr;
+    if (cudaMallocAsync((void**)&mem, o_buf2 + align256(bytes), s) != cudaSuccess) {
+        cudaGetLastError();
+        return GVA_OK;
+    }
+    struct Free {
+        char* mem;
+        cudaStream_t s;
+        ~Free() { cudaFreeAsync(mem, s); }
+    } free_mem{mem, s};
+    if (keep_rows && cudaMallocAsync((void**)&fin, kChainResult, s) != cudaSuccess) {
+        cudaGetLastError();
+        return GVA_OK;
+    }
+    auto drop = [&]() {
+        if (fin) cudaFreeAsync(fin, s);
+        fin = nullptr;
+    };
+    volatile uint64_t* h_tot = hs->pinned + 8;
+    volatile uint32_t* h_failed = (volatile uint32_t*)(hs->pinned + 7);
+    for (size_t i = 0; i < n; ++i) h_tot[i] = 0;
+    *h_failed = 0;
+    auto launch = [&](size_t i, size_t slot, uint32_t* out, uint64_t cap_out) {
+        const Step& st = steps[i];
+        Chain c{};
+        c.n_in = i == 1 ? nullptr : (uint64_t*)(mem + o_tot) + (i - 1);
+        c.cap_in = cap;
+        c.cap_out = cap_out;
+        c.tiles = (unsigned long long*)(mem + o_tiles) + slot;
+        c.status = (unsigned long long*)(mem + status_at[slot]);
+        c.n_out = (uint64_t*)(mem + o_tot) + slot;
+        c.host_out = const_cast<uint64_t*>(h_tot) + (i == slot ? i : 0);
+        c.failed = (uint32_t*)mem;
+        c.host_failed = const_cast<uint32_t*>(h_failed);
+        const uint32_t* in = i == 1 ? db.seed_verts + db.seed_off[steps[0].label] : (uint32_t*)(mem + (i & 1 ? o_buf2 : o_buf));
+        // a CTA per tile of the seeds while they fit the chip at once (a tile
+        // waits for the ones before it); later steps mostly have fewer, and a
+        // CTA that finds none costs a launch slot: 1,184 CTAs for 228 tiles
+        // took 16 us, 444 take 11
+        const uint64_t tiles = (rows0 + kRowsPerBlock - 1) / kRowsPerBlock;
+        const unsigned grid = (unsigned)(i == 1 ? std::min<uint64_t>(tiles, 148 * 8)
+                                                : std::min<uint64_t>(std::max<uint64_t>(2 * tiles, 64), 148 * 3));
+        const bool counts = count_only && i + 1 == n;
+        if (st.kind == STEP_EXT) {
+            ExtArgs a;
+            fill_ext(a, db, st, in, rows0, out);
+            if (counts)
+                chain_count_kernel<ExtArgs><<<grid, kThreads, 0, s>>>(a, c);
+            else
+                chain_ext_kernel<<<grid, kThreads, ext_smem_bytes(a.k, a.n_eq), s>>>(a, c);
+        } else {
+            RedArgs a;
+            fill_red(a, db, st, in, rows0, out);
+            if (counts)
+                chain_count_kernel<RedArgs><<<grid, kThreads, 0, s>>>(a, c);
+            else
+                chain_red_kernel<<<grid, kThreads, red_smem_bytes(a.k), s>>>(a, c);
+        }
+        g_launches += 1;
+    };
+    // from here on errors of the driver end the query
+    cudaError_t e = cudaMemsetAsync(mem, 0, ctl, s);
+    const uint32_t w_last = steps[n - 1].kind == STEP_EXT ? steps[n - 1].width_in + 1 : steps[n - 1].width_in;
+    for (size_t i = 1; i < n; ++i) {
+        const bool last = i + 1 == n;
+        uint32_t* out = last ? fin : (uint32_t*)(mem + (i & 1 ? o_buf : o_buf2));
+        launch(i, i, out, last ? kChainResult / 4 / w_last : cap);
+    }
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaEventRecord(hs->ev1, s);
+    if (e == cudaSuccess) e = cudaEventSynchronize(hs->ev1);
+    if (e != cudaSuccess) {
+        drop();
+        return fail(GVA_ERR_CUDA, cudaGetErrorString(e));
+    }
+    totals.assign(n, 0);
+    totals[0] = rows0;
+    bool reached = true;  // the last step's total is known
+    for (size_t i = 1; i < n; ++i) totals[i] = h_tot[i];
+    for (size_t i = 1; i + 1 < n; ++i) reached = reached && totals[i] <= cap;
+    const bool big = keep_rows && *h_failed == 1 && reached && totals[n - 1] * w_last * 4 > kChainResult;
+    if (*h_failed && !big) {  // an output had no room (or a wait ran out): counted steps
+        drop();
+        return GVA_OK;
+    }
+    // as the counted steps check it: every frontier that is written
+    for (size_t i = 1; i < n; ++i) {
+        const uint32_t w = steps[i].kind == STEP_EXT ? steps[i].width_in + 1 : steps[i].width_in;
+        if (i + 1 == n && count_only) break;
+        if (totals[i] * w * 4ull > budget) {
+            drop();
+            return fail(GVA_ERR_NOMEM, "frontier of " + std::to_string(totals[i]) + " rows exceeds the memory budget");
+        }
+    }
+    if (keep_rows && totals[n - 1] == 0) drop();
+    if (big) {
+        drop();
+        if (cudaMallocAsync((void**)&fin, totals[n - 1] * w_last * 4, s) != cudaSuccess) {
+            fin = nullptr;
+            return fail(GVA_ERR_NOMEM, "frontier allocation failed");
+        }
+        *h_failed = 0;
+        e = cudaMemsetAsync(mem, 0, 8, s);  // the failure mark
+        launch(n - 1, n, fin, totals[n - 1]);
+        if (e == cudaSuccess) e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaEventRecord(hs->ev1, s);
+        if (e == cudaSuccess) e = cudaEventSynchronize(hs->ev1);
+        if (e != cudaSuccess || *h_failed) {
+            drop();
+            return fail(GVA_ERR_CUDA, e != cudaSuccess ? cudaGetErrorString(e) : "a tile of the last step did not end");
+        }
+    }
+    final = fin;
+    done = true;
     return GVA_OK;
 }
 
@@ -915,6 +1291,29 @@ int run_match(DevDB& db, const Plan& plan, const std::vector<Step>& steps, cudaS
     cudaEvent_t ev0 = hs->ev0, ev1 = hs->ev1;
     GVA_CUDA(cudaEventRecord(ev0, s));
 
+    if (!profile) {
+        std::vector<uint64_t> totals;
+        uint32_t* final = nullptr;
+        bool done = false;
+        rc = run_chain(db, steps, s, budget, count_only, hs, totals, final, done);
+        if (rc) return rc;
+        if (done) {
+            float ms = 0.f;
+            cudaEventElapsedTime(&ms, ev0, ev1);
+            res.gpu_ms = ms;
+            res.rows = totals.back();
+            for (size_t i = 0; i < steps.size(); ++i) {
+                if (steps[i].phase_end >= 0) res.phase_rows[steps[i].phase_end] = totals[i];
+                if (totals[i] == 0) {
+                    res.rows = 0;
+                    break;
+                }
+            }
+            res.width = (uint32_t)plan.columns.size();
+            res.rows_dev = final;
+            return GVA_OK;
+        }
+    }
     const uint32_t* cur = nullptr;
     uint32_t* owned = nullptr;  // frontier we must free
     uint64_t rows = 0;

@@ -73,3 +73,53 @@ def test_budget_still_refuses_the_extension(native):
     with pytest.raises(gv.GenevaError):
         gv.match(db, plan, budget_bytes=2 * kept)
     db.close()
+
+
+def small_graphs(copies, extra, seed):
+    """`copies` graphs of 24 vertices (labels 1..3, two edge labels), each a
+    cycle and `extra` chords."""
+    rng = np.random.default_rng(seed)
+    labels, edges = [0], set()
+    for c in range(copies):
+        v0 = len(labels)
+        labels += rng.integers(1, 4, 24).tolist()
+        edges |= {(v0 + i, v0 + (i + 1) % 24) for i in range(24)}
+        while len(edges) < (c + 1) * (24 + extra):
+            a, b = sorted(int(x) for x in rng.integers(v0, v0 + 24, 2))
+            if a != b and (a, b) not in edges and (b, a) not in edges:
+                edges.add((a, b))
+    e = np.array(sorted(edges), np.uint32)
+    return np.array(labels, np.uint32), e[:, 0], e[:, 1], rng.integers(1, 3, len(e)).astype(np.uint32)
+
+
+CHAIN_QUERIES = QUERIES + [
+    "v 0 1\nv 1 2\ne 0 1 1\n",
+    "v 0 1\nv 1 1\nv 2 1\nv 3 1\nv 4 1\ne 0 1 1\ne 1 2 2\ne 2 3 1\ne 3 4 2\n",
+    "v 0 1\nv 1 2\nv 2 1\nv 3 2\nv 4 3\ne 0 1 1\ne 1 2 1\ne 2 3 2\ne 0 3 1\ne 3 4 1\n",
+    "v 0 2\nv 1 9\ne 0 1 1\n",   # a label that the data lack
+    "v 0 2\nv 1 2\nv 2 2\nv 3 2\ne 0 1 2\ne 1 2 2\ne 2 3 2\ne 0 3 2\ne 0 2 2\ne 1 3 2\n",  # likely none
+]
+
+
+# extra chords: 4 keeps frontiers small; 130 makes them outgrow the chain's
+# room (dense graphs: degree about 13) and its result buffer
+@pytest.mark.parametrize("copies,extra", [(1, 0), (11, 4), (32, 4), (700, 6), (40, 130), (1500, 130)])
+def test_chain_against_oracle(native, oracle, copies, extra):
+    """Queries on graphs without long lists, whose steps run as a chain: one
+    tile, several, as many as there are seeds, outputs without room."""
+    labels, src, dst, el = small_graphs(copies, extra, copies + extra)
+    db = gv.Database.from_edges(labels, src, dst, el)
+    og = oracle.from_edges(labels, src, dst, el)
+    for text in CHAIN_QUERIES:
+        want, phases = oracle.match(og, text)
+        plan = gv.Plan.from_text(text)
+        res = gv.match(db, plan)
+        assert res.phase_rows == phases, text
+        rows = res.rows()
+        assert np.array_equal(rows, want[np.lexsort(want.T[::-1])]), text
+        counted = gv.match(db, plan, count_only=True)
+        assert counted.num_rows == len(want) and counted.phase_rows == phases, text
+        # the same rows as the steps that are counted one by one
+        assert np.array_equal(gv.match(db, plan, profile=True).rows(), rows), text
+    oracle.free(og)
+    db.close()
