@@ -170,12 +170,12 @@ __device__ __forceinline__ bool next_chunk(const Span& a, uint64_t& begin, uint6
 // warp: 32 pivots per step, so three dependent loads find one of 32,768
 // tasks (a binary search takes 15, about half of what a small round's only
 // item per warp waits for).
-__device__ __forceinline__ uint32_t find_slot(const uint64_t* __restrict__ pfx, uint32_t n, uint64_t x) {
+__device__ __forceinline__ uint32_t find_slot(const uint64_t* pfx, uint32_t n, uint64_t x) {
     const uint32_t lane = threadIdx.x & 31;
     uint32_t lo = 0, len = n;
     while (len > 1) {
         const uint32_t step = (len + 31) / 32, at = lane * step;
-        const uint32_t m = __ballot_sync(0xffffffffu, at < len && __ldg(pfx + lo + at) <= x);
+        const uint32_t m = __ballot_sync(0xffffffffu, at < len && pfx[lo + at] <= x);
         const uint32_t k = (31 - __clz(m)) * step;  // lane 0's pivot always qualifies
         lo += k;
         len = min(step, len - k);
@@ -824,7 +824,8 @@ struct PassArgs {
     uint32_t rows_per_item;      // rows of an input page; of a slice of a seed list
     uint32_t hub;
     uint32_t kmax;
-    uint4* rec;                  // per slot written: (node, place among the node's rows, rows, width)
+    uint32_t second;             // light class: launched after the fused class's of the same round
+    uint4* rec;                  // per slot written: (task, place among its node's rows, rows, width)
     uint32_t* node_rows;         // per node: rows written
     unsigned long long* node_total;  // per node: rows
     Unit* units;                 // kUnitCap per class, light class first (null: no list is long)
@@ -844,12 +845,12 @@ constexpr uint32_t kNoPage = 0xffffffffu, kLostPage = 0xfffffffeu;
 
 // Where a warp's output of one node goes: the open page and its rows.
 struct Pages {
-    uint32_t slot = kNoPage, fill = 0, width = 0;
+    uint32_t slot = kNoPage, fill = 0, width = 0, task = 0;
 
     // Lists the open page among the node's rows.
     __device__ __forceinline__ void close(const PassArgs& a, uint32_t node) {
         if (slot < kLostPage && (threadIdx.x & 31) == 0)
-            a.rec[slot] = make_uint4(node, atomicAdd(a.node_rows + node, fill), fill, width);
+            a.rec[slot] = make_uint4(task, atomicAdd(a.node_rows + node, fill), fill, width);
         slot = kNoPage;
         fill = 0;
     }
@@ -1106,9 +1107,12 @@ template <bool FUSED, bool UNITS>
 __global__ void __launch_bounds__(kRoundWarps * 32, FUSED ? 3 : 4)
 round_pass_kernel(const __grid_constant__ PassArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    // the light class's launch may start on the SMs that this one no longer
-    // fills; it waits for this one before it ends (below)
-    if (FUSED && !UNITS) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // A launch may start while the one before it ends: the first of a round
+    // waits here for the round before it, and only then lets the next start;
+    // the light class's, after the fused class's of the same round, fills the
+    // SMs which that one no longer does and waits for it before it ends.
+    if (!UNITS && (FUSED || !a.second)) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!UNITS) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t lane = threadIdx.x & 31, R = a.rows_per_item;
     const uint32_t warp = threadIdx.x >> 5;
     TaskDesc& d = reinterpret_cast<TaskDesc*>(smem_raw)[warp];
@@ -1144,8 +1148,8 @@ round_pass_kernel(const __grid_constant__ PassArgs a) {
     auto open_task = [&](uint32_t task_index) {
         task_done();
         t = task_index;
-        t_lo = __ldg(a.item0 + t);
-        t_hi = __ldg(a.item0 + t + 1);
+        t_lo = a.item0[t];  // plain loads of what the planning wrote: this launch may have started before it
+        t_hi = a.item0[t + 1];
         const uint2 task = __ldg(a.tasks + t);
         if (a.seeds) {
             in = a.seeds[t].in;
@@ -1159,6 +1163,7 @@ round_pass_kernel(const __grid_constant__ PassArgs a) {
         node = task.x;
         k = d.kind == STEP_EXT ? d.e.k : d.r.k;
         pg.width = d.kind == STEP_EXT ? k + 1 : k;
+        pg.task = t;
     };
     if (UNITS) {
         while (next_chunk(sp, begin, end)) {
@@ -1217,7 +1222,7 @@ round_pass_kernel(const __grid_constant__ PassArgs a) {
         }
     }
     task_done();
-    if (!FUSED && !UNITS) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!FUSED && !UNITS && a.second) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Planning of the next round, by one cluster: the finished round's nodes get
@@ -1283,6 +1288,8 @@ __device__ __forceinline__ uint64_t cluster_scan(uint64_t v, uint64_t& sum) {
 }
 
 __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanThreads) pass_plan_kernel(PlanArgs p) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     constexpr uint32_t kAll = kPlanCtas * kPlanThreads;
     const uint32_t me = blockIdx.x * kPlanThreads + threadIdx.x;
     const bool lost = p.st->overflow || p.st->slots > p.slot_cap;  // the same in every CTA
@@ -1324,21 +1331,111 @@ __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanThreads
     }
 }
 
+// Slot s's rows to their places: `first` is the first packed page of its node.
+__device__ __forceinline__ void pack_slot(const PlanArgs& p, uint32_t s, const uint4& r, uint64_t first) {
+    const uint32_t R = p.page_rows;
+    const uint32_t* src = p.scratch + (uint64_t)s * p.page_words;
+    for (uint32_t i = threadIdx.x & 31; i < r.z; i += 32) {
+        const uint32_t at = r.y + i, page = at / R;
+        uint32_t* dst = p.packed + (first + page) * p.page_words + (at - page * R);
+        for (uint32_t c = 0; c < r.w; ++c) dst[c * R] = src[c * R + i];
+    }
+}
+
 // The scratch pages' rows to their places in the packed pages, a warp per
 // page.  Bound by memory: every row is read and written once.
 __global__ void __launch_bounds__(256) pass_pack_kernel(PlanArgs p) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (p.nx->overflow) return;
-    const uint32_t lane = threadIdx.x & 31, R = p.page_rows, slots = (uint32_t)p.st->slots;
-    const uint32_t warps = gridDim.x * 8;
+    const uint32_t slots = (uint32_t)p.st->slots, warps = gridDim.x * 8;
     for (uint32_t s = blockIdx.x * 8 + (threadIdx.x >> 5); s < slots; s += warps) {
-        const uint4 r = __ldg(p.rec + s);
-        const uint32_t* src = p.scratch + (uint64_t)s * p.page_words;
-        const uint64_t first = (uint64_t)__ldg(p.page_base + r.x) * p.page_words;
-        for (uint32_t i = lane; i < r.z; i += 32) {
-            const uint32_t at = r.y + i, page = at / R;
-            uint32_t* dst = p.packed + first + (uint64_t)page * p.page_words + (at - page * R);
-            for (uint32_t c = 0; c < r.w; ++c) dst[c * R] = __ldg(src + c * R + i);
+        const uint4 r = p.rec[s];
+        pack_slot(p, s, r, p.page_base[p.done[r.x].x]);
+    }
+}
+
+// Planning and packing in one launch, for rounds of few tasks: every CTA
+// prefixes the finished round's nodes for itself, the first one also tells
+// the next round.  A round of 16 patterns spent 13 us on the two launches
+// and the gap between them, as long as its round kernels took; with one launch
+// that starts while the round's last items run, nine rounds take 361 instead
+// of 436 us per call.
+constexpr uint32_t kSmallDone = 2048, kSmallNext = 8192;  // most tasks: finished round, next round
+constexpr int kSmallThreads = 512;
+__global__ void __launch_bounds__(kSmallThreads) pass_small_kernel(PlanArgs p) {
+    __shared__ uint32_t base_s[kSmallDone];
+    __shared__ uint64_t ws[kSmallThreads / 32];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    if (p.st->overflow || p.st->slots > p.slot_cap) {  // the same in every CTA
+        if (blockIdx.x == 0 && tid == 0) {
+            p.nx->overflow = 1;
+            *p.overflow = 1;
         }
+        return;
+    }
+    auto pages = [&](uint32_t node) { return (p.node_rows[node] + p.page_rows - 1) / p.page_rows; };
+    auto scan = [&](uint64_t v, uint64_t& sum) {  // exclusive, over the CTA
+        uint64_t inc = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= (uint32_t)o) inc += y;
+        }
+        __syncthreads();  // ws read by every thread before
+        if (lane == 31) ws[wid] = inc;
+        __syncthreads();
+        uint64_t before = inc - v;
+        sum = 0;
+        for (uint32_t j = 0; j < kSmallThreads / 32; ++j) {
+            if (j < wid) before += ws[j];
+            sum += ws[j];
+        }
+        return before;
+    };
+    uint64_t sum;
+    {
+        uint32_t n[kSmallDone / kSmallThreads];
+        const uint32_t per = (p.n_done + kSmallThreads - 1) / kSmallThreads, b = tid * per;
+        uint64_t v = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < kSmallDone / kSmallThreads; ++j) {
+            n[j] = j < per && b + j < p.n_done ? pages(p.done[b + j].x) : 0;
+            v += n[j];
+        }
+        uint64_t at = scan(v, sum);
+#pragma unroll
+        for (uint32_t j = 0; j < kSmallDone / kSmallThreads; ++j) {
+            if (j >= per || b + j >= p.n_done) break;
+            base_s[b + j] = (uint32_t)at;
+            if (blockIdx.x == 0) p.page_base[p.done[b + j].x] = (uint32_t)at;
+            at += n[j];
+        }
+    }
+    if (blockIdx.x == 0) {
+        const uint32_t per = (p.n_next + kSmallThreads - 1) / kSmallThreads;
+        const uint32_t b = min(p.n_next, tid * per), e = min(p.n_next, b + per);
+        uint64_t v = 0;
+        for (uint32_t t = b; t < e; ++t) v += pages(p.next[t].y);
+        uint64_t at = scan(v, sum);
+        if (tid == 0) {
+            p.item0[p.n_next] = sum;
+            p.nx->ni = sum;
+            if (p.n_next_light == p.n_next) p.nx->ni_light = sum;
+        }
+        for (uint32_t t = b; t < e; ++t) {
+            p.item0[t] = at;
+            if (t == p.n_next_light) p.nx->ni_light = at;
+            at += pages(p.next[t].y);
+        }
+    }
+    __syncthreads();
+    const uint32_t slots = (uint32_t)p.st->slots, warps = gridDim.x * (kSmallThreads / 32);
+    for (uint32_t s = blockIdx.x + gridDim.x * wid; s < slots; s += warps) {  // the first CTA is the last to start
+        const uint4 r = p.rec[s];
+        pack_slot(p, s, r, base_s[r.x]);
     }
 }
 
@@ -2565,6 +2662,23 @@ int BatchSession::run_pages() {
         return (uint32_t)std::max<uint64_t>(
             1, std::min<uint64_t>(resident_ctas(db.device, fn, smem) * (uint64_t)sms, (items + kRoundWarps - 1) / kRoundWarps));
     };
+    // a launch that may start before the one before it has ended (the kernels
+    // wait for it themselves); rounds that the host steps through leave nothing
+    // to overlap
+    const bool early = !stepped;
+    auto launch = [&](auto kernel, uint32_t ctas, int threads, size_t smem, bool overlap, auto args) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(ctas);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = overlap ? 1 : 0;
+        return cudaLaunchKernelEx(&cfg, kernel, args);
+    };
     lap(1);
     uint64_t nl = 0;
     int done = 0;
@@ -2600,25 +2714,16 @@ int BatchSession::run_pages() {
         pa.ctx = ctx;
         if (items_fused) {
             const size_t smem = pass_smem_bytes(R[d], kmax[d], true);
-            round_pass_kernel<true, false>
-                <<<grid((const void*)round_pass_kernel<true, false>, smem, items_fused), kRoundWarps * 32, smem, s>>>(pa);
+            GVA_CUDA_B(launch(round_pass_kernel<true, false>, grid((const void*)round_pass_kernel<true, false>, smem, items_fused),
+                              kRoundWarps * 32, smem, early && d > 1, pa));
             ++nl;
         }
         if (items_light) {
-            // after the fused class's launch of the same round it may start
-            // before that one's last items are done
             const size_t smem = pass_smem_bytes(R[d], kmax[d], false);
-            cudaLaunchConfig_t cfg{};
-            cfg.gridDim = dim3(grid((const void*)round_pass_kernel<false, false>, smem, items_light));
-            cfg.blockDim = dim3(kRoundWarps * 32);
-            cfg.dynamicSmemBytes = smem;
-            cfg.stream = s;
-            cudaLaunchAttribute at{};
-            at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            at.val.programmaticStreamSerializationAllowed = 1;
-            cfg.attrs = &at;
-            cfg.numAttrs = items_fused ? 1 : 0;
-            GVA_CUDA_B(cudaLaunchKernelEx(&cfg, round_pass_kernel<false, false>, pa));
+            pa.second = items_fused ? 1 : 0;
+            GVA_CUDA_B(launch(round_pass_kernel<false, false>,
+                              grid((const void*)round_pass_kernel<false, false>, smem, items_light), kRoundWarps * 32, smem,
+                              items_fused || (early && d > 1), pa));
             ++nl;
         }
         if (long_lists && items_fused) {
@@ -2652,9 +2757,14 @@ int BatchSession::run_pages() {
         pl.scratch = scratch;
         pl.packed = packed;
         pl.overflow = d_flag;
-        pass_plan_kernel<<<kPlanCtas, kPlanThreads, 0, s>>>(pl);
-        pass_pack_kernel<<<8 * sms, 256, 0, s>>>(pl);
-        nl += 2;
+        if (pl.n_done <= kSmallDone && pl.n_next <= kSmallNext) {
+            GVA_CUDA_B(launch(pass_small_kernel, 2 * sms, kSmallThreads, 0, early, pl));
+            nl += 1;
+        } else {
+            GVA_CUDA_B(launch(pass_plan_kernel, kPlanCtas, kPlanThreads, 0, early, pl));
+            GVA_CUDA_B(launch(pass_pack_kernel, 8 * sms, 256, 0, early, pl));
+            nl += 2;
+        }
         if (stepped) {
             PassState* back = (PassState*)(h + o_back);
             GVA_CUDA_B(cudaMemcpyAsync(back, states + d + 1, sizeof(PassState), cudaMemcpyDeviceToHost, s));

@@ -418,8 +418,12 @@ __device__ __forceinline__ void chain_fail(const Chain& c, uint32_t why) {
 // Rows of a step's input: none once a step has failed (its rows were not all
 // written).  A CTA that starts late may find its own step's failure; the CTAs
 // that found none take all of its tiles, so that the total is known.
+// A step's launch may start while the one before it runs and waits for it
+// here (its rows and totals are read with plain loads).
 __device__ __forceinline__ uint64_t chain_rows(const Chain& c, uint64_t nrows) {
     __shared__ uint64_t n;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (threadIdx.x == 0)
         n = *(volatile uint32_t*)c.failed ? 0 : c.n_in ? umin64(*c.n_in, c.cap_in) : nrows;
     __syncthreads();
@@ -956,6 +960,7 @@ int run_chain(DevDB& db, const std::vector<Step>& steps, cudaStream_t s, uint64_
     volatile uint32_t* h_failed = (volatile uint32_t*)(hs->pinned + 7);
     for (size_t i = 0; i < n; ++i) h_tot[i] = 0;
     *h_failed = 0;
+    cudaError_t e = cudaSuccess;
     auto launch = [&](size_t i, size_t slot, uint32_t* out, uint64_t cap_out) {
         const Step& st = steps[i];
         Chain c{};
@@ -977,25 +982,39 @@ int run_chain(DevDB& db, const std::vector<Step>& steps, cudaStream_t s, uint64_
         const unsigned grid = (unsigned)(i == 1 ? std::min<uint64_t>(tiles, 148 * 8)
                                                 : std::min<uint64_t>(std::max<uint64_t>(2 * tiles, 64), 148 * 3));
         const bool counts = count_only && i + 1 == n;
+        auto start = [&](auto kernel, size_t smem, auto args) {
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(grid);
+            cfg.blockDim = dim3(kThreads);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = s;
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at.val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = &at;
+            cfg.numAttrs = i > 1 && slot == i ? 1 : 0;
+            const cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, args, c);
+            if (e == cudaSuccess) e = le;
+        };
         if (st.kind == STEP_EXT) {
             ExtArgs a;
             fill_ext(a, db, st, in, rows0, out);
             if (counts)
-                chain_count_kernel<ExtArgs><<<grid, kThreads, 0, s>>>(a, c);
+                start(chain_count_kernel<ExtArgs>, 0, a);
             else
-                chain_ext_kernel<<<grid, kThreads, ext_smem_bytes(a.k, a.n_eq), s>>>(a, c);
+                start(chain_ext_kernel, ext_smem_bytes(a.k, a.n_eq), a);
         } else {
             RedArgs a;
             fill_red(a, db, st, in, rows0, out);
             if (counts)
-                chain_count_kernel<RedArgs><<<grid, kThreads, 0, s>>>(a, c);
+                start(chain_count_kernel<RedArgs>, 0, a);
             else
-                chain_red_kernel<<<grid, kThreads, red_smem_bytes(a.k), s>>>(a, c);
+                start(chain_red_kernel, red_smem_bytes(a.k), a);
         }
         g_launches += 1;
     };
     // from here on errors of the driver end the query
-    cudaError_t e = cudaMemsetAsync(mem, 0, ctl, s);
+    e = cudaMemsetAsync(mem, 0, ctl, s);
     const uint32_t w_last = steps[n - 1].kind == STEP_EXT ? steps[n - 1].width_in + 1 : steps[n - 1].width_in;
     for (size_t i = 1; i < n; ++i) {
         const bool last = i + 1 == n;
