@@ -1491,6 +1491,58 @@ char* Staging::get(size_t need) {
 }
 Staging::~Staging() { pin_give(p, cap); }
 
+// Large results to the caller's memory through pinned memory, the host's
+// cores taking pieces as they arrive: a copy into pageable memory runs on one
+// core of the driver's, and memory that the caller has never touched is
+// faulted in page by page on the one that writes.  The workers are woken once
+// per 64 MiB (once per piece cost more than it gave).
+int copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+    constexpr size_t kWindow = 64u << 20, kPiece = 2u << 20;
+    const unsigned T = pool_width();
+    if (bytes < 4 * kPiece || T < 4) {
+        GVA_CUDA_B(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
+        GVA_CUDA_B(cudaStreamSynchronize(s));
+        return GVA_OK;
+    }
+    Staging stage;
+    char* from = stage.get(std::min(bytes, kWindow));
+    if (!from) return fail(GVA_ERR_NOMEM, "pinned staging allocation failed");
+    std::vector<cudaEvent_t> ev;
+    cudaError_t e = cudaSuccess;
+    for (size_t at = 0; at < bytes && e == cudaSuccess; at += kWindow) {
+        const size_t len = std::min(kWindow, bytes - at), n = (len + kPiece - 1) / kPiece;
+        for (size_t i = 0; i < n && e == cudaSuccess; ++i) {
+            const size_t o = i * kPiece;
+            if (i == ev.size()) {
+                ev.push_back(nullptr);
+                e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
+            }
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(from + o, (const char*)src + at + o, std::min(kPiece, len - o), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaEventRecord(ev[i], s);
+        }
+        if (e != cudaSuccess) break;
+        std::atomic<int> bad{cudaSuccess};
+        pool_run(T, [&](unsigned t) {
+            for (size_t i = 0; i < n; ++i) {
+                const cudaError_t we = cudaEventSynchronize(ev[i]);
+                if (we != cudaSuccess) {
+                    bad = (int)we;
+                    return;
+                }
+                const size_t o = i * kPiece, m = std::min(kPiece, len - o), b = m * t / T;
+                memcpy((char*)dst + at + o + b, from + o + b, m * (t + 1) / T - b);
+            }
+        });
+        e = (cudaError_t)bad.load();
+    }
+    if (e != cudaSuccess) cudaStreamSynchronize(s);  // no copy lands in memory that is given back
+    for (cudaEvent_t x : ev)
+        if (x) cudaEventDestroy(x);
+    if (e != cudaSuccess) return fail(GVA_ERR_CUDA, cudaGetErrorString(e));
+    return GVA_OK;
+}
+
 // ---------------------------------------------------------------------------
 // BatchSession: the persistent form of the batched engine.  Plans are
 // submitted in waves (plans of one wave share their common step prefixes);
@@ -2983,11 +3035,17 @@ int finish_batch(DevDB& db, PreparedBatch& pb, uint64_t* counts, uint64_t* graph
             }
             if (!rc)
                 rc = cudaStreamSynchronize(s) == cudaSuccess ? GVA_OK : fail(GVA_ERR_CUDA, "result read-back failed");
-            for (int q = 0; q < nq && !rc; ++q) {
-                const int sl = ses.plan(ses.first_peer(ids[q])).slot;
-                if (support_host) support_host[at(q)] = pop[sl];
-                if (gc) std::copy(gc + (size_t)sl * G, gc + (size_t)(sl + 1) * G, graph_counts_host + at(q) * G);
-            }
+            // the rows on the host's cores: the caller's memory is often fresh
+            // (4,096 x 1,000 counts, 33 MB: 4.4 ms on one core)
+            const unsigned T = gc && (size_t)nq * G >= (1u << 18) ? pool_width() : 1u;
+            if (!rc)
+                pool_run(T, [&](unsigned t) {
+                    for (int q = (int)((int64_t)nq * t / T); q < (int)((int64_t)nq * (t + 1) / T); ++q) {
+                        const int sl = ses.plan(ses.first_peer(ids[q])).slot;
+                        if (support_host) support_host[at(q)] = pop[sl];
+                        if (gc) std::copy(gc + (size_t)sl * G, gc + (size_t)(sl + 1) * G, graph_counts_host + at(q) * G);
+                    }
+                });
         }
     }
     if (stats) {

@@ -389,11 +389,7 @@ int gva_result_copy_rows(const gva_result* res, uint32_t* host_dst, uint64_t fir
     if (!res->r.rows_dev) return fail(GVA_ERR_ARG, "result holds counts only");
     cudaSetDevice(res->r.device);
     const size_t w = res->r.width;
-    cudaError_t e = cudaMemcpyAsync(host_dst, res->r.rows_dev + first_row * w, num_rows * w * 4,
-                                    cudaMemcpyDeviceToHost, res->r.stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(res->r.stream);
-    if (e != cudaSuccess) return fail(GVA_ERR_CUDA, cudaGetErrorString(e));
-    return GVA_OK;
+    return copy_to_host(host_dst, res->r.rows_dev + first_row * w, num_rows * w * 4, res->r.stream);
 }
 
 int gva_result_write_text(const gva_result* res, const char* path) {

@@ -135,6 +135,10 @@ struct Staging {
     ~Staging();
 };
 
+// `bytes` of device memory to the caller's (pageable) memory, complete on
+// return.
+int copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s);
+
 // Persistent batched engine (gva_batch.cu).  Plans are submitted in waves;
 // round() advances every active task one step; completed plans are reported
 // by take_completed().  Per-graph results need slots > 0 (one per live plan).

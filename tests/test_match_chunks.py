@@ -123,3 +123,23 @@ def test_chain_against_oracle(native, oracle, copies, extra):
         assert np.array_equal(gv.match(db, plan, profile=True).rows(), rows), text
     oracle.free(og)
     db.close()
+
+
+@pytest.mark.parametrize("leaves", [900, 1183, 1184, 2100])
+def test_large_read_back(native, leaves):
+    """Rows read back in pieces (from 8 MiB on; 1,184 leaves give the first
+    such size) equal the closed form, whole and from any row on."""
+    labels = np.array([0, 1] + [2] * leaves, np.uint32)
+    leaf = np.arange(2, 2 + leaves, dtype=np.uint32)
+    db = gv.Database.from_edges(labels, np.ones(leaves, np.uint32), leaf, np.ones(leaves, np.uint32))
+    res = gv.match(db, gv.Plan.from_text("v 0 1\nv 1 2\nv 2 2\ne 0 1 1\ne 0 2 1\n"))
+    rows = res.rows()
+    assert len(rows) == leaves * (leaves - 1) // 2
+    i, j = np.tril_indices(leaves, -1)
+    pairs = np.sort(rows[:, 1:], axis=1) if (rows[:, 0] == 1).all() else None
+    assert pairs is not None
+    want = np.stack([leaf[j], leaf[i]], axis=1)
+    assert np.array_equal(pairs[np.lexsort(pairs.T[::-1])], want[np.lexsort(want.T[::-1])])
+    for first, count in ((0, 1), (1, len(rows) - 1), (len(rows) // 3, len(rows) // 2)):
+        assert np.array_equal(res.rows(first, count), rows[first:first + count])
+    db.close()
