@@ -520,7 +520,7 @@ def batch_count(db: Database, plans: Sequence[Plan], stream: Optional[int] = Non
     n = len(plans)
     arr = _plan_handles(plans)
     counts = np.zeros(n, dtype=np.uint64)
-    gc = np.zeros((n, db.num_graphs), dtype=np.uint64) if graph_counts else None
+    gc = np.empty((n, db.num_graphs), dtype=np.uint64) if graph_counts else None  # every entry is written by the call
     sup = np.zeros(n, dtype=np.uint32) if support else None
     o = _BatchOpts(stream or None, budget_bytes, 1 if profile else 0,
                    (BATCH_HOST_ROUNDS if host_rounds else 0) | (BATCH_DEVICE_ROUNDS if device_rounds else 0))
@@ -557,7 +557,7 @@ def batch_count_texts(db: Database, texts: Sequence[str], mode: int = MODE_DV, s
     n = len(texts)
     buf, arr = _text_array(texts)
     counts = np.zeros(n, dtype=np.uint64)
-    gc = np.zeros((n, db.num_graphs), dtype=np.uint64) if graph_counts else None
+    gc = np.empty((n, db.num_graphs), dtype=np.uint64) if graph_counts else None  # every entry is written by the call
     sup = np.zeros(n, dtype=np.uint32) if support else None
     status = np.zeros(max(n, 1), dtype=np.int32)
     o = _BatchOpts(stream or None, budget_bytes, 1 if profile else 0, BATCH_PLAN_ON_DEVICE if plan_on_device else 0)
