@@ -19,11 +19,10 @@
 //           the candidates are the shortest segment among the already matched
 //           neighbours, each filtered by injectivity and by binary search in
 //           the other matched neighbours' segments, the first survivor taken.
-//           Each lane first searches its own seed for up to 64 candidates (32
-//           independent searches per warp keep many loads in flight); seeds
-//           still undecided are searched by the whole warp, 32 candidates per
-//           step, one seed at a time; what a warp leaves undecided after a
-//           few steps is cut into pieces that all warps share (MniWork)
+//           Each lane first searches its own seed for up to 96 candidates (32
+//           independent searches per warp keep many loads in flight); what
+//           they leave undecided is cut into pieces that all warps share
+//           (MniWork), a warp to a piece, 32 candidates per step
 //   stop    a task stops once its count reaches the cap (default: the minimum
 //           support, which decides frequency) or the smallest exhausted orbit
 //           of its pattern, so the support returned is min(MNI, cap) exactly
@@ -285,12 +284,11 @@ __device__ bool put_pieces(const MniHard& H, int q, const Dfs& s, int base, int 
 // their dependent loads overlap; most roots of frequent patterns succeed or
 // fail within a few candidates.
 __device__ int lane_dfs(const MniTask& T, const PartPtr* __restrict__ parts, uint32_t L, uint32_t root,
-                        uint32_t budget, unsigned long long* cnt) {
-    Dfs s;
+                        uint32_t budget, Dfs& s, int& i, unsigned long long* cnt) {
     const int n = (int)T.n;
     s.f[0] = root;
     if (n <= 1) return 1;
-    int i = 1;
+    i = 1;
     dfs_open(T, parts, L, s, 1);
     cnt[P_OPENS] += 1;
     uint32_t steps = 0;
@@ -329,10 +327,53 @@ __device__ int lane_dfs(const MniTask& T, const PartPtr* __restrict__ parts, uin
     }
 }
 
-constexpr uint32_t kLaneBudget = 64;  // candidates a lane search may take before the warp search decides
-// Steps of 32 candidates that a warp may take on a root before what is left
-// is cut into pieces for every warp, and on a piece before it is cut again.
-constexpr uint32_t kWarpBudget = 32, kPieceBudget = 128;
+// Candidates a lane may take on its root before what is left becomes pieces
+// for every warp, and steps of 32 candidates a warp may take on a piece before
+// it is cut again: [1] with several items for every warp, [0] with fewer, when
+// a lane's candidates are what the round waits for.  Lane budgets 16 / 32 / 64
+// / 96 / 128, device ms on R-MAT graphs: 1,200 patterns capped at 1,000 (many)
+// 17 / 5.4 / 2.7 / 2.4 / 2.5 (below 64 the queue runs over), 37 exact
+// patterns (few) 0.94 / 0.87 / 1.02 / - / -; 2.9 and 1.4 when the warp searched
+// 32 steps on each such root, one after another, before it gave it away.
+constexpr uint32_t kLaneBudget[2] = {16, 96}, kPieceBudget[2] = {64, 128};
+
+// What the lanes with `mine` have left of their searches (levels 1 .. i of s)
+// into queue 0, a piece per open level; false: no room, nothing was put there.
+__device__ bool put_lanes(const MniHard& H, bool mine, const Dfs& s, int i, uint32_t task, uint32_t cap, uint32_t lane) {
+    uint32_t n = 0;
+    if (mine)
+        for (int j = 1; j <= i; ++j) n += s.pos[j] < s.end[j] ? 1 : 0;
+    uint32_t inc = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (uint32_t)o) inc += y;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, inc, 31), voters = __ballot_sync(0xffffffffu, mine);
+    unsigned long long at = 0, root = 0;
+    if (lane == 0) {
+        root = reserve(H.state + 4, __popc(voters), H.cap_roots);
+        at = root < H.cap_roots ? reserve(H.state, total, H.cap_work) : H.cap_work;
+    }
+    at = __shfl_sync(0xffffffffu, at, 0);
+    root = __shfl_sync(0xffffffffu, root, 0) + __popc(voters & ((1u << lane) - 1u));
+    if (at >= H.cap_work) return total == 0;
+    at += inc - n;
+    if (mine)
+        for (int j = 1; j <= i; ++j) {
+            if (s.pos[j] >= s.end[j]) continue;
+            MniWork& w = H.queue[0][at++];
+            w.hard = (uint32_t)root;
+            w.task = task;
+            w.cap = cap;
+            w.level = (uint32_t)j;
+            w.pos = s.pos[j];
+            w.end = s.end[j];
+            w.gsel = s.gsel[j];
+            for (int k = 0; k < kMniMaxVertices - 1; ++k) w.f[k] = k < j ? s.f[k] : 0u;
+        }
+    return true;
+}
 
 __device__ __forceinline__ void load_task(MniTask& T, const MniTask* __restrict__ src, uint32_t lane) {
     __syncwarp();
@@ -352,8 +393,8 @@ __device__ __forceinline__ void add_prof(unsigned long long* prof, const unsigne
 
 // Persistent: every warp pulls 128-seed items; per 32 seeds it checks the
 // task's count against its cap, filters roots by neighbour-label degrees and
-// runs one search per surviving root.  A root that neither a lane nor the
-// warp decides within its budget goes to the pieces of mni_piece_kernel.
+// runs one search per surviving root.  A root that its lane does not decide
+// within its budget goes to the pieces of mni_piece_kernel.
 //
 // Why: nearly every root is decided within a few candidates, but one without
 // an embedding under a hub can take millions of steps (pairs of a hub's
@@ -369,7 +410,8 @@ mni_search_kernel(const MniTask* __restrict__ tasks, const MniSlot* __restrict__
                   const uint64_t* __restrict__ item0, const uint32_t* __restrict__ item_slot, uint64_t nitems,
                   const uint32_t* __restrict__ seeds, uint32_t item_len,
                   const PartPtr* __restrict__ parts, uint32_t L, uint32_t* __restrict__ counts,
-                  unsigned long long* __restrict__ queue, MniHard H, unsigned long long* __restrict__ prof) {
+                  unsigned long long* __restrict__ queue, MniHard H, uint32_t lane_budget,
+                  unsigned long long* __restrict__ prof) {
     __shared__ MniTask tsh[kMniWarps];
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     MniTask& T = tsh[w];
@@ -402,30 +444,24 @@ mni_search_kernel(const MniTask* __restrict__ tasks, const MniSlot* __restrict__
             }
             const uint32_t roots = __ballot_sync(0xffffffffu, ok);  // all lanes vote
             if (lane == 0) cnt[P_ROOTS] += __popc(roots);
-            // every lane searches its own root; roots whose search ran out of
-            // budget are decided by the whole warp, one after another
-            int verdict = 0;
-            if (ok) verdict = lane_dfs(T, parts, L, v, kLaneBudget, cnt);
+            // every lane searches its own root; what a search has left when
+            // it runs out of budget is shared out
+            int verdict = 0, i = 0;
+            Dfs st;
+            if (ok) verdict = lane_dfs(T, parts, L, v, lane_budget, st, i, cnt);
             uint32_t found = __popc(__ballot_sync(0xffffffffu, verdict == 1));
             uint32_t m = __ballot_sync(0xffffffffu, verdict < 0);
-            while (m) {
-                const int l = __ffs(m) - 1;
-                m &= m - 1;
-                Dfs st;
-                st.f[0] = __shfl_sync(0xffffffffu, v, l);
-                int i = 1;
-                dfs_open(T, parts, L, st, 1);
-                cnt[P_OPENS] += lane == 0 ? 1 : 0;
-                int r = warp_search(T, parts, L, st, 1, i, kWarpBudget, lane, cnt);
-                if (r < 0) {
-                    unsigned long long hard = 0;
-                    if (lane == 0) hard = reserve(H.state + 4, 1, H.cap_roots);
-                    hard = __shfl_sync(0xffffffffu, hard, 0);
-                    if (hard >= H.cap_roots ||
-                        !put_pieces(H, 0, st, 1, i, (uint32_t)hard, sl.task, sl.cap, lane))
-                        r = warp_search(T, parts, L, st, 1, i, 0xffffffffu, lane, cnt);  // no room: to its end here
+            if (m && !put_lanes(H, verdict < 0, st, i, sl.task, sl.cap, lane)) {
+                while (m) {  // no room: to their ends here, by the whole warp
+                    const int l = __ffs(m) - 1;
+                    m &= m - 1;
+                    Dfs all;
+                    all.f[0] = __shfl_sync(0xffffffffu, v, l);
+                    int k = 1;
+                    dfs_open(T, parts, L, all, 1);
+                    cnt[P_OPENS] += lane == 0 ? 1 : 0;
+                    if (warp_search(T, parts, L, all, 1, k, 0xffffffffu, lane, cnt) > 0) ++found;
                 }
-                if (r > 0) ++found;
             }
             if (found && lane == 0) atomicAdd(counts + sl.task, found);
             if (lane == 0) cnt[P_FOUND] += found;
@@ -435,13 +471,14 @@ mni_search_kernel(const MniTask* __restrict__ tasks, const MniSlot* __restrict__
 }
 
 // The pieces of queue q, one per warp at a time: each is searched for up to
-// kPieceBudget steps and what is left goes, cut again, to the other queue (a
+// `piece_budget` steps and what is left goes, cut again, to the other queue (a
 // search thus spreads over the chip within two or three launches).  The first
 // embedding of a root counts it; the root's other pieces are then skipped, as
 // are pieces of a task at its cap.
 __global__ void __launch_bounds__(kMniWarps * 32, 6)
 mni_piece_kernel(const MniTask* __restrict__ tasks, const PartPtr* __restrict__ parts, uint32_t L,
-                 uint32_t* __restrict__ counts, MniHard H, int q, unsigned long long* __restrict__ prof) {
+                 uint32_t* __restrict__ counts, MniHard H, int q, uint32_t piece_budget,
+                 unsigned long long* __restrict__ prof) {
     __shared__ MniTask tsh[kMniWarps];
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     MniTask& T = tsh[w];
@@ -474,7 +511,7 @@ mni_piece_kernel(const MniTask* __restrict__ tasks, const PartPtr* __restrict__ 
         s.gsel[base] = field(6);
         s.gadj[base] = parts[T.part[base][s.gsel[base]] - 1].adj;
         int i = base;
-        int r = warp_search(T, parts, L, s, base, i, kPieceBudget, lane, cnt);
+        int r = warp_search(T, parts, L, s, base, i, piece_budget, lane, cnt);
         if (r < 0 && !put_pieces(H, q ^ 1, s, base, i, hard, task, cap, lane))
             r = warp_search(T, parts, L, s, base, i, 0xffffffffu, lane, cnt);
         if (r > 0 && lane == 0 && atomicExch(H.found + hard, 1u) == 0) {
@@ -869,6 +906,7 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
                                          ? slots_all
                                          : std::max<uint64_t>(1, slots_all * sm_percent / 100);
             const uint64_t grid = std::min<uint64_t>(cta_cap, (nitems + kMniWarps - 1) / kMniWarps);
+            const int many = nitems > 4 * cta_cap * kMniWarps;
             cudaEvent_t ev = nullptr;
             const double rows = (double)total;
             mni_expand_kernel<<<(unsigned)std::min<uint64_t>((ns + 255) / 256, 4096), 256, 0, s>>>(d_item0, ns,
@@ -876,7 +914,7 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
             if (profile) prof.begin(K_MNI, 0.0, s, ev);
             mni_search_kernel<<<(unsigned)std::max<uint64_t>(grid, 1), kMniWarps * 32, 0, s>>>(
                 d_tasks, d_slots, d_item0, d_item_slot, nitems, db.seed_by_degree, (uint32_t)item_len, d_parts, db.kernel_L(),
-                d_counts, d_queue, H, profile ? d_prof : nullptr);
+                d_counts, d_queue, H, kLaneBudget[many], profile ? d_prof : nullptr);
             if (profile) prof.end(ev, K_MNI, 0.0, s, rows);
             st.launches += 2;
             g_mni_launches += 2;
@@ -909,7 +947,7 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
                     cudaMemsetAsync(H.state + 2 * (q ^ 1), 0, 16, s);  // taken by the launch before
                     if (profile) prof.begin(K_MNI, 0.0, s, ev);
                     mni_piece_kernel<<<(unsigned)cta_cap, kMniWarps * 32, 0, s>>>(
-                        d_tasks, d_parts, db.kernel_L(), d_counts, H, q, profile ? d_prof : nullptr);
+                        d_tasks, d_parts, db.kernel_L(), d_counts, H, q, kPieceBudget[many], profile ? d_prof : nullptr);
                     if (profile) prof.end(ev, K_MNI, 0.0, s, 0.0);
                 }
                 st.launches += 4;
