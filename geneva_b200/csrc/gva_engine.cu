@@ -224,10 +224,12 @@ __device__ __forceinline__ uint32_t gallop(const uint32_t* __restrict__ adj, uin
 //
 // What bounds it: the loads of those searches.  24 million extension rows,
 // 1.2 million of them kept, on an R-MAT graph of 2^18 vertices: written,
-// counted and written again in 830 + 474 + 608 us as two steps.
+// counted and written again in 830 + 474 + 608 us as two steps, counted and
+// written in 425 + 71 us here (490 with 48 registers and five CTAs per SM
+// instead of 32 and eight: more searches in flight).
 constexpr uint32_t kTestRun = 8;
 template <bool WRITE>
-__global__ void __launch_bounds__(kThreads) ext_red_kernel(ExtArgs p, const uint64_t* __restrict__ block_off,
+__global__ void __launch_bounds__(kThreads, 8) ext_red_kernel(ExtArgs p, const uint64_t* __restrict__ block_off,
                                                            uint64_t nb, uint64_t chunk, uint64_t* __restrict__ sums,
                                                            uint8_t* __restrict__ masks, uint32_t mask_cap) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
