@@ -2626,12 +2626,16 @@ int BatchSession::run_pages() {
     const size_t o_back = al(std::max(up_bytes, nn * 8 + 64));  // staging: a round's state read back (stepped)
     char* h = staging.get(o_back + sizeof(PassState));
     if (!h) return fail(GVA_ERR_NOMEM, "pinned staging allocation failed");
+    const bool long_lists = db.max_degree > kUnitLen;
     std::vector<uint32_t> R(D + 2, 32);
     for (int d = 1; d <= D; ++d) {
-        // twice the tuned rows (128 by default): a tenth of them is left after
-        // the lookups.  64 / 128 rows, per call: 16,384 patterns 9.1 / 8.2 ms,
-        // 1,501 texts 2.04 / 1.96 ms, 16 patterns 458 / 447 us
-        R[d] = std::min<uint32_t>(2 * tune.rows_per_item, std::max<uint32_t>(32, (768 / kmax[d]) & ~31u));
+        // twice the tuned rows (128 by default) where a tenth of them is left
+        // after the lookups.  64 / 128 rows, per call: 16,384 patterns 9.1 /
+        // 8.2 ms, 1,501 texts 2.04 / 1.96 ms, 16 patterns 458 / 447 us.  With
+        // long lists nearly all are left, items differ more, and every piece
+        // stages its whole item: 32 / 64 / 128 rows, 61 queries on an R-MAT
+        // graph 604 / 570 / 621 us
+        R[d] = std::min<uint32_t>((long_lists ? 1 : 2) * tune.rows_per_item, std::max<uint32_t>(32, (768 / kmax[d]) & ~31u));
         R[d] = R[d] >= 128 ? 128 : R[d] >= 64 ? 64 : 32;  // a power of two (stage_page)
     }
     uint2* h_tasks = (uint2*)(h + o_tasks);
@@ -2680,7 +2684,6 @@ int BatchSession::run_pages() {
     // one allocation, of nearly the same size in every run: regions, then the
     // schedule's arrays; on a graph with long lists also the queues of their
     // pieces
-    const bool long_lists = db.max_degree > kUnitLen;
     const size_t o_units = o_rec + al(slot_most * sizeof(uint4));
     const size_t region_bytes = al(region);
     const size_t unit = (size_t)256 << 20, blk_bytes = o_units + (long_lists ? 2 * (size_t)kUnitCap * sizeof(Unit) : 0);
