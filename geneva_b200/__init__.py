@@ -253,8 +253,8 @@ class Database:
                 "round_region_mb": int(t.round_region_mb)}
 
     def set_tuning(self, rows_per_item: int, hub: int, round_region_mb: int = 0) -> None:
-        """round_region_mb: MiB of each frontier region of device-scheduled
-        rounds (0 keeps the current size)."""
+        """round_region_mb: MiB of each frontier region of one-pass rounds
+        (0 keeps the current size)."""
         t = _Tuning(rows_per_item, hub, 0.0, 0.0, 0, round_region_mb)
         _check(library().gva_db_set_tuning(self._h, ctypes.byref(t)))
 
@@ -513,10 +513,11 @@ def batch_count(db: Database, plans: Sequence[Plan], stream: Optional[int] = Non
 
     Returns (counts[n] uint64, per_graph, stats) where per_graph is the
     [n, num_graphs] uint64 count matrix when graph_counts, else the [n]
-    uint32 supporting-graph counts when support, else None.  host_rounds /
-    device_rounds: schedule every round on the host / on the device
-    (GVA_BATCH_HOST_ROUNDS / GVA_BATCH_DEVICE_ROUNDS; default: on the device
-    for a run in one piece, on the host for one split in halves)."""
+    uint32 supporting-graph counts when support, else None.  host_rounds:
+    counted rounds, scheduled on the host; device_rounds: one-pass rounds
+    launched at once (GVA_BATCH_HOST_ROUNDS / GVA_BATCH_DEVICE_ROUNDS;
+    default: one-pass rounds, launched at once for a run in one piece and one
+    after another for a run split in halves)."""
     n = len(plans)
     arr = _plan_handles(plans)
     counts = np.zeros(n, dtype=np.uint64)

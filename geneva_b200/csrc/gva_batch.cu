@@ -1,16 +1,14 @@
 // Batched engine: many query patterns advance together.
 //
 // A task is (query, slice of that query's frontier, next step).  One round
-// advances every active task by one step:
-//   count   one launch over the 256-row blocks of all tasks (per-task step
-//           parameters from a descriptor array); final steps in count mode
-//           also add their rows into per-(query, graph) counters and graph
-//           bitmaps here and never write rows
-//   scan    exclusive scan of all block totals
-//   totals  per-task output rows
-//   write   persistent kernel: blocks pull 256-row items from an atomic work
-//           queue (load balance across SMs however uneven the tasks are) and
-//           expand / compact them into the round's output buffer
+// advances every active task by one step, by persistent kernels whose warps
+// pull items (slices of up to 128 rows) from an atomic work queue, so the SMs
+// stay evenly loaded however uneven the tasks are.  Counted rounds:
+//   count   all tasks' items (step parameters from a descriptor array); final
+//           steps in count mode also add their rows into per-(query, graph)
+//           counters and graph bitmaps here and never write rows
+//   scan    exclusive scan of the items' totals; per-task output rows
+//   write   the items again, expanded / compacted into the round's output
 // A task whose output does not fit the memory budget is split in half (its
 // input rows) and retried next round, so any frontier is processed in
 // budget-sized pieces, deepest tasks first.  This replaces the reference's
@@ -822,7 +820,6 @@ struct PassArgs {
     uint32_t slot_cap;           // slots of either region
     uint32_t nt;
     uint32_t rows_per_item;      // rows of an input page; of a slice of a seed list
-    uint32_t hub;
     uint32_t kmax;
     uint32_t second;             // light class: launched after the fused class's of the same round
     uint4* rec;                  // per slot written: (task, place among its node's rows, rows, width)
@@ -1508,7 +1505,8 @@ int copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s) {
     char* from = stage.get(std::min(bytes, kWindow));
     if (!from) return fail(GVA_ERR_NOMEM, "pinned staging allocation failed");
     std::vector<cudaEvent_t> ev;
-    cudaError_t e = cudaSuccess;
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
     for (size_t at = 0; at < bytes && e == cudaSuccess; at += kWindow) {
         const size_t len = std::min(kWindow, bytes - at), n = (len + kPiece - 1) / kPiece;
         for (size_t i = 0; i < n && e == cudaSuccess; ++i) {
@@ -1524,6 +1522,7 @@ int copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s) {
         if (e != cudaSuccess) break;
         std::atomic<int> bad{cudaSuccess};
         pool_run(T, [&](unsigned t) {
+            cudaSetDevice(device);  // a worker's calls stay on the caller's GPU
             for (size_t i = 0; i < n; ++i) {
                 const cudaError_t we = cudaEventSynchronize(ev[i]);
                 if (we != cudaSuccess) {
@@ -2094,7 +2093,7 @@ int BatchSession::submit(std::vector<std::vector<Step>>&& wave, const std::vecto
     }
     }
     // the new nodes' descriptors, on the host's cores, into the staging that
-    // the next round (or device-scheduled run) ships; only descriptors not
+    // the next round (or one-pass run) ships; only descriptors not
     // yet shipped are kept.  An initialised session stages them in pinned
     // memory (an asynchronous copy), one never initialised in host memory
     // (tries built without a device make no device call).
@@ -2512,7 +2511,7 @@ int BatchSession::ship_nodes() {
 
 // Resident CTAs per SM of a round kernel at a dynamic shared memory size,
 // cached per (device, kernel, size): the occupancy query is a driver call
-// and a device-scheduled run makes several per round.
+// and a one-pass run makes several per round.
 static uint32_t resident_ctas(int device, const void* fn, size_t smem) {
     static std::mutex mu;
     static std::map<std::tuple<int, const void*, size_t>, uint32_t> known;
@@ -2581,7 +2580,7 @@ int BatchSession::run_pages() {
         }
     } timer{t_start, round_host_ms, wait_ms, wait_before};
     auto t_lap = t_start;
-    auto lap = [&](int k) {  // phase_ms: schedule tables, uploads, launches, -, results
+    auto lap = [&](int k) {  // phase_ms
         const auto now = std::chrono::steady_clock::now();
         phase_ms[k] += std::chrono::duration<double, std::milli>(now - t_lap).count();
         t_lap = now;
@@ -2759,7 +2758,6 @@ int BatchSession::run_pages() {
         pa.slot_cap = d < D ? (uint32_t)slot_cap(d) : 0;
         pa.nt = nt;
         pa.rows_per_item = R[d];
-        pa.hub = tune.hub;
         pa.kmax = kmax[d];
         pa.rec = (uint4*)(blk + o_rec);
         pa.node_rows = (uint32_t*)(blk + o_nrows);

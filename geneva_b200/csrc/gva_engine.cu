@@ -1,19 +1,22 @@
 // CUDA engine for sm_100a: device database, phase kernels, phase executor.
 //
 // Frontiers are row-major uint32 tables (one column per matched query
-// vertex).  Every extension or reduction runs as
+// vertex).  An extension or reduction by itself runs as
 //   count  (thread per row)            -> per-256-row block totals
-//   scan   (one block)                 -> exclusive block offsets + total
-//   write  (block per 256 rows)        -> rows staged in shared memory,
-//                                         outputs balanced across the block,
+//   scan   (one CTA or one cluster)    -> exclusive block offsets + total
+//   write  (CTA per block; with long lists per share of the outputs)
+//                                      -> rows staged in shared memory,
+//                                         outputs balanced across the CTA,
 //                                         flushed with coalesced stores
 // so the output size is known before it is written (no device-side overflow
-// protocol, unlike src/miningPattern.cu:3325-3343) and output order is
-// deterministic (input-row order, candidates ascending).
+// protocol, unlike src/miningPattern.cu:3325-3343).  A query's steps run
+// either as a chain of one-pass kernels (graphs without long lists, run_chain)
+// or counted, an extension and its reduction fused (ext_red_kernel).  Output
+// order is deterministic on every path (input-row order, candidates ascending).
 //
-// Label segments come from a dense (vertex, label) offset table, one load per
-// lookup, replacing the warp bisection with vLabel gathers of the reference
-// (FIND_LABEL_LIMIT, include/common.h:18-66).
+// Label segments come from an index (packed records or a dense (vertex, label)
+// offset table), one load per lookup, replacing the warp bisection with vLabel
+// gathers of the reference (FIND_LABEL_LIMIT, include/common.h:18-66).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 

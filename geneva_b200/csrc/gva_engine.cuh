@@ -45,7 +45,7 @@ struct DevDB {
     // frontier budget of batched runs given none: 3/4 of the device memory
     // free when the first such run started (querying it costs a driver call)
     uint64_t default_budget = 0;
-    // device-scheduled rounds (BatchSession::run_pages): bytes of each of a
+    // one-pass rounds (BatchSession::run_pages): bytes of each of a
     // run's two frontier regions; doubled after a run that overflowed them
     std::atomic<uint64_t> round_region_bytes{0};
 };
@@ -117,8 +117,9 @@ size_t step_key_bytes(const Step& st, uint8_t* buf);
 // 64-bit hash of the same fields, never 0 (a sort key: equal keys hash equal)
 uint64_t step_key_hash(const Step& st);
 
-// Round scheduling of run_batch: ROUNDS_AUTO = on the device when the run is
-// one piece, on the host when it runs as two halves
+// Round scheduling of run_batch: ROUNDS_AUTO = one-pass rounds, launched at
+// once when the run is one piece and stepped by the host when it runs as two
+// halves; ROUNDS_DEVICE = launched at once; ROUNDS_HOST = counted rounds
 enum RoundsMode { ROUNDS_AUTO = 0, ROUNDS_HOST = 1, ROUNDS_DEVICE = 2 };
 int run_batch(DevDB& db, std::vector<std::vector<Step>> steps, cudaStream_t s, uint64_t budget,
               const uint32_t* vgraph, uint32_t G, uint64_t* counts, uint64_t* graph_counts_host,
@@ -217,20 +218,23 @@ public:
     uint32_t* graph_bits_dev() const;
 
     // Launch shape of the round kernels: rows per work item (a multiple of
-    // 32, at most 128; fewer when rows are wide) and the candidate-list length
-    // above which a row's candidates are shared by its whole warp.
+    // 32, at most 128; fewer when rows are wide) and, for counted rounds, the
+    // candidate-list length above which a row's candidates are shared by its
+    // whole warp.
     struct Tuning {
         uint32_t rows_per_item = 64;
         uint32_t hub = 32;
     } tune;
 
     uint64_t rounds = 0, splits = 0, launches = 0;
-    uint64_t device_rounds = 0;  // rounds scheduled on the device (run_pages)
+    uint64_t device_rounds = 0;  // one-pass rounds launched at once (run_pages)
     bool host_rounds = false;    // run_pages declines: counted rounds, scheduled on the host
     bool stepped = false;        // run_pages: a round is launched when the one before has been read
     double submit_ms = 0, round_host_ms = 0, wait_ms = 0;  // host time split
-    // round_host_ms by part: task scan + uploads, count launches, totals and
-    // budget choice, write launch, next tasks and completion
+    // round_host_ms by part.  Counted rounds: task scan + uploads, count
+    // launches, totals and budget choice, write launch, next tasks and
+    // completion; run_pages: descriptors, memory and uploads, launches, -,
+    // completion
     double phase_ms[5] = {0, 0, 0, 0, 0};
     KernelStat kstat[K_NUM];
 

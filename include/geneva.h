@@ -165,9 +165,11 @@ void gva_result_free(gva_result* res);
 
 /* ---- batched form ----------------------------------------------------------
  * Many plans in shared rounds: each round advances every (plan, frontier
- * slice) task by one step with one count, scan, totals and one persistent
- * write launch fed by a device work queue; a task whose output exceeds
- * budget_bytes is split.  Replaces running the gpumine driver once per query
+ * slice) task by one step with persistent launches fed by a device work queue.
+ * A round walks its rows once, into pages of two frontier regions; where
+ * these don't fit budget_bytes or run over, rounds are counted before they
+ * are written, and a task whose output exceeds budget_bytes is split.
+ * Replaces running the gpumine driver once per query
  * (src/gpumine.cpp:866-1072).  Results are counts: the final step of every
  * plan only counts. */
 typedef struct gva_batch_opts {
@@ -180,17 +182,17 @@ typedef struct gva_batch_opts {
  * planner, one query per thread; queries of up to 16 vertices and 32 edge
  * lines, DV mode), the others on the host */
 #define GVA_BATCH_PLAN_ON_DEVICE 1
-/* Round scheduling.  On the device, a planning kernel per round chooses the
- * writing tasks, places their outputs and lists the next round's tasks, so
- * the host launches every round at once and synchronises once (when the
- * budget holds two frontier regions; a round that outgrows its region makes
- * the run start over on the host).  On the host, each round's task totals
- * are read back and the host chooses the writes (splitting tasks larger than
- * the budget) and the next round's tasks.  By default a run in one piece is
- * scheduled on the device, and a run of 12,288 plans or more, which runs as
- * two halves whose round trips hide behind each other's kernels, on the
- * host (no schedule tables or frontier regions per half; the two measured
- * alike there).  The flags force one or the other; they exclude each other. */
+/* Round scheduling.  One-pass rounds: each walks its rows once, a planning
+ * kernel places what they gave and lists the next round's items.  A run in
+ * one piece launches every round at once and synchronises once; a run of
+ * 12,288 plans or more, which runs as two halves whose round trips hide
+ * behind each other's kernels, reads each round's size back and launches the
+ * next one sized to it (GVA_BATCH_DEVICE_ROUNDS: at once there too).  They
+ * need two frontier regions within the budget; a round that outgrows its
+ * region makes the run start over with counted rounds.  Counted rounds
+ * (GVA_BATCH_HOST_ROUNDS; profiled runs): each round's task totals are read
+ * back and the host chooses the writes (splitting tasks larger than the
+ * budget) and the next round's tasks.  The two flags exclude each other. */
 #define GVA_BATCH_HOST_ROUNDS 2
 #define GVA_BATCH_DEVICE_ROUNDS 4
 
@@ -203,8 +205,10 @@ typedef struct gva_batch_stats {
      * rounds' host work (task lists, launches, budget choice), waiting for
      * the device, session set-up / read-back / tear-down */
     double lower_ms, submit_ms, round_host_ms, wait_ms, session_ms;
-    /* round_host_ms by part: task list and uploads, count launches, totals
-     * and budget choice, write launch, next tasks and completion */
+    /* round_host_ms by part.  Counted rounds: task list and uploads, count
+     * launches, totals and budget choice, write launch, next tasks and
+     * completion.  One-pass rounds: node descriptors, memory and uploads,
+     * launches (with the read-backs between them), -, completion */
     double round_phase_ms[5];
     /* wall-clock marks of the run (ms from the call's start of the batched
      * run): plans ordered; then for each of up to two halves (a run of
@@ -212,8 +216,8 @@ typedef struct gva_batch_stats {
      * prepared, its rounds done, its results read back and its session freed
      * (0 for an absent half) */
     double timeline_ms[9];
-    /* rounds scheduled on the device: the run's rounds were launched at
-     * once, each round's planning kernel choosing the next round's tasks */
+    /* one-pass rounds that were launched at once, without a read-back
+     * between them */
     uint64_t device_rounds;
 } gva_batch_stats;
 
@@ -241,9 +245,11 @@ int gva_batch_count_texts(gva_db* db, const char* const* query_texts, int n, int
                           gva_batch_stats* stats);
 
 /* Launch shape of the batched engine's round kernels on one database: rows
- * per work item (32, 64 or 128; fewer when rows are wide) and the candidate
- * list length above which a frontier row's candidates are shared by a whole
- * warp instead of walked by one lane.  Defaults 64 / 32.  The reference's
+ * per work item (32, 64 or 128; fewer when rows are wide; one-pass rounds
+ * take twice as many on databases without adjacency lists above 256 entries,
+ * a page) and, in counted rounds, the candidate list length above which a
+ * frontier row's candidates are shared by a whole warp instead of walked by
+ * one lane.  Defaults 64 / 32.  The reference's
  * launch shape is fixed (a persistent grid of GPU_SM_NUM blocks,
  * src/miningPattern.cu:3350-3377); here it is chosen per database. */
 typedef struct gva_tuning {
@@ -252,7 +258,7 @@ typedef struct gva_tuning {
     double ms;          /* gva_db_autotune: calibration time of the chosen shape */
     double default_ms;  /* gva_db_autotune: calibration time of the default shape */
     uint32_t tried;     /* gva_db_autotune: shapes timed */
-    /* MiB of each of the two frontier regions of device-scheduled rounds
+    /* MiB of each of the two frontier regions of one-pass rounds
      * (0: unchanged by gva_db_set_tuning; default 2048); doubled after a run
      * whose round outgrew it */
     uint32_t round_region_mb;
