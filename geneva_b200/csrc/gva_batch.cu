@@ -911,8 +911,14 @@ __device__ __forceinline__ uint32_t pass_find(const ExtArgs& p, const uint32_t* 
         // two rows per lane: their index records are loaded together
         const uint32_t r0 = base + lane, r1 = r0 + 32;
         uint32_t lo0 = 0, hi0 = 0, lo1 = 0, hi1 = 0;
-        if (r0 < nr) seg_of(off, L, src[r0], lab, lo0, hi0);
-        if (r1 < nr) seg_of(off, L, src[r1], lab, lo1, hi1);
+        if (L & kPackedSeg) {
+            const SegRec a = seg_record(off, r0 < nr ? src[r0] : 0), b = seg_record(off, r1 < nr ? src[r1] : 0);
+            if (r0 < nr) seg_in_record(a, off, lab, lo0, hi0);
+            if (r1 < nr) seg_in_record(b, off, lab, lo1, hi1);
+        } else {
+            if (r0 < nr) seg_of(off, L, src[r0], lab, lo0, hi0);
+            if (r1 < nr) seg_of(off, L, src[r1], lab, lo1, hi1);
+        }
         const uint32_t b0 = __ballot_sync(0xffffffffu, lo0 < hi0), b1 = __ballot_sync(0xffffffffu, lo1 < hi1);
         const uint32_t below = (1u << lane) - 1u;
         if (lo0 < hi0) {
