@@ -32,7 +32,7 @@
 // queue (SM-level load balance however skewed the seeds' degrees are).  With
 // many tasks an item is a task's whole quota, scanned by one warp in seed
 // order and stopped as soon as the count reaches the cap; with few, quotas
-// are cut into items of down to 128 seeds so that every warp has work.  The
+// are cut into items of down to 32 seeds so that every warp has work.  The
 // host retires capped and exhausted tasks between rounds.
 // The batched form puts every task of many patterns in one round; the plain
 // form runs the same rounds one pattern at a time.
@@ -63,7 +63,12 @@ namespace {
     } while (0)
 
 constexpr int kMniWarps = 8;       // warps per block
-constexpr uint32_t kMniItem = 128; // smallest work item (seeds); rounds with few tasks use it
+// Smallest work item (seeds), of rounds with few tasks: one group.  128 left
+// nine of ten warps of the chip idle in a round of 250,000 seeds (37 patterns on
+// an R-MAT graph of 2^16 vertices; its search launches 250 + 130 + 27 us with
+// 128, 200 + 58 + 12 us with 32).
+constexpr uint32_t kMniItem = 32;
+constexpr uint32_t kMniManySeeds = 128;  // seeds per resident warp, times 4: from there on there are many
 constexpr uint32_t kMniFirst = 2048;  // seeds per task in the first round (doubles every round)
 
 struct PartPtr {
@@ -375,6 +380,19 @@ __device__ bool put_lanes(const MniHard& H, bool mine, const Dfs& s, int i, uint
     return true;
 }
 
+// A warp's first item is that of its number, the others come from the queue's
+// head: 7,104 warps asking one counter at once took 10 us, in a launch with
+// nothing to do too (4 us now).
+struct FirstThenQueue {
+    unsigned long long* head;
+    uint32_t warps;
+    __device__ __forceinline__ unsigned long long operator()(uint32_t lane) const {
+        unsigned long long it = 0;
+        if (lane == 0) it = warps + atomicAdd(head, 1ull);
+        return __shfl_sync(0xffffffffu, it, 0);
+    }
+};
+
 __device__ __forceinline__ void load_task(MniTask& T, const MniTask* __restrict__ src, uint32_t lane) {
     __syncwarp();
     const uint32_t* s = reinterpret_cast<const uint32_t*>(src);
@@ -391,7 +409,7 @@ __device__ __forceinline__ void add_prof(unsigned long long* prof, const unsigne
     }
 }
 
-// Persistent: every warp pulls 128-seed items; per 32 seeds it checks the
+// Persistent: every warp pulls items; per 32 seeds it checks the
 // task's count against its cap, filters roots by neighbour-label degrees and
 // runs one search per surviving root.  A root that its lane does not decide
 // within its budget goes to the pieces of mni_piece_kernel.
@@ -417,11 +435,8 @@ mni_search_kernel(const MniTask* __restrict__ tasks, const MniSlot* __restrict__
     MniTask& T = tsh[w];
     unsigned long long cnt[P_NUM] = {0, 0, 0, 0, 0, 0};
     int cur = -1;
-    for (;;) {
-        unsigned long long it = 0;
-        if (lane == 0) it = atomicAdd(queue, 1ull);
-        it = __shfl_sync(0xffffffffu, it, 0);
-        if (it >= nitems) break;
+    const FirstThenQueue next{queue, gridDim.x * kMniWarps};
+    for (unsigned long long it = blockIdx.x * kMniWarps + w; it < nitems; it = next(lane)) {
         const int s = (int)__ldg(item_slot + it);
         const MniSlot sl = slots[s];
         if ((int)sl.task != cur) {
@@ -486,11 +501,8 @@ mni_piece_kernel(const MniTask* __restrict__ tasks, const PartPtr* __restrict__ 
     unsigned long long* state = H.state + 2 * q;
     const unsigned long long n = state[0];  // only read by this launch
     uint32_t cur = 0xffffffffu;
-    for (;;) {
-        unsigned long long it = 0;
-        if (lane == 0) it = atomicAdd(state + 1, 1ull);
-        it = __shfl_sync(0xffffffffu, it, 0);
-        if (it >= n) break;
+    const FirstThenQueue next{state + 1, gridDim.x * kMniWarps};
+    for (unsigned long long it = blockIdx.x * kMniWarps + w; it < n; it = next(lane)) {
         uint32_t word = 0;
         if (lane < kWorkWords) word = __ldg(reinterpret_cast<const uint32_t*>(H.queue[q] + it) + lane);
         auto field = [&](int k) { return __shfl_sync(0xffffffffu, word, k); };
@@ -867,7 +879,7 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
             }
             // items: a whole slot per warp when there are many (its count is
             // checked every 32 seeds, so a task stops right at its cap), cut
-            // down to 128 seeds when few tasks must fill the GPU
+            // down to 32 seeds when few tasks must fill the GPU
             const uint64_t want_items = (uint64_t)8 * per_sm * sms * kMniWarps;
             uint64_t item_len = std::max<uint64_t>(kMniItem, (total / want_items + 31) & ~(uint64_t)31);
             item_len = std::min<uint64_t>(item_len, 1u << 30);
@@ -906,7 +918,7 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
                                          ? slots_all
                                          : std::max<uint64_t>(1, slots_all * sm_percent / 100);
             const uint64_t grid = std::min<uint64_t>(cta_cap, (nitems + kMniWarps - 1) / kMniWarps);
-            const int many = nitems > 4 * cta_cap * kMniWarps;
+            const int many = total > 4 * cta_cap * kMniWarps * kMniManySeeds;
             cudaEvent_t ev = nullptr;
             const double rows = (double)total;
             mni_expand_kernel<<<(unsigned)std::min<uint64_t>((ns + 255) / 256, 4096), 256, 0, s>>>(d_item0, ns,
