@@ -164,6 +164,29 @@ __device__ __forceinline__ bool next_chunk(const Span& a, uint64_t& begin, uint6
     return begin < a.n;
 }
 
+// The same for a launch that may have few items: below four per warp every
+// warp's first one is that of its number, and the queue holds the rest (of a
+// round with an item for every warp: nothing, and no warp asks for it).
+// Thousands of warps asking one counter at once had taken as long as a small
+// round's work: 16 patterns 371 / 324 us per call, 61 queries on an R-MAT graph
+// 424 / 383 us.  With more items the queue holds them all: a CTA that starts
+// late, because the other class still fills its SM, must not hold any.
+__device__ __forceinline__ bool next_chunk_or_own(const Span& a, bool& first, uint64_t& begin, uint64_t& end) {
+    if (a.n >= 4ull * a.warps) return next_chunk(a, begin, end);
+    if (first) {
+        first = false;
+        begin = (uint64_t)blockIdx.x * kRoundWarps + (threadIdx.x >> 5);
+    } else if (a.n <= a.warps) {
+        return false;
+    } else {
+        unsigned long long b = 0;
+        if ((threadIdx.x & 31) == 0) b = a.warps + atomicAdd(a.queue, 1ull);
+        begin = __shfl_sync(0xffffffffu, b, 0);
+    }
+    end = begin + 1;
+    return begin < a.n;
+}
+
 // Last t in [0, n) with pfx[t] <= x (pfx ascending, pfx[0] <= x), by the whole
 // warp: 32 pivots per step, so three dependent loads find one of 32,768
 // tasks (a binary search takes 15, about half of what a small round's only
@@ -1138,6 +1161,7 @@ round_pass_kernel(const __grid_constant__ PassArgs a) {
                           : Span{FUSED ? light : 0, FUSED ? a.st->ni - light : light, a.st->heads + (FUSED ? 1 : 0),
                                  gridDim.x * kRoundWarps};
     uint32_t t = 0xffffffffu;
+    bool first = true;
     auto task_done = [&]() {
         pg.close(a, node);
         if (lane == 0 && total) atomicAdd(a.node_total + node, (unsigned long long)total);
@@ -1169,7 +1193,7 @@ round_pass_kernel(const __grid_constant__ PassArgs a) {
         pg.task = t;
     };
     if (UNITS) {
-        while (next_chunk(sp, begin, end)) {
+        while (next_chunk_or_own(sp, first, begin, end)) {
             for (uint64_t u = begin; u < end; ++u) {
                 const Unit unit = a.units[(FUSED ? kUnitCap : 0) + u];
                 if (unit.x0 >= unit.x1) continue;
@@ -1185,7 +1209,7 @@ round_pass_kernel(const __grid_constant__ PassArgs a) {
             }
         }
     } else
-    while (next_chunk(sp, begin, end)) {
+    while (next_chunk_or_own(sp, first, begin, end)) {
         const uint64_t stop = sp.base + end;
         for (uint64_t item = sp.base + begin; item < stop; ++item) {
             if (item >= t_hi || item < t_lo) open_task(find_slot(a.item0, a.nt + 1, item));
