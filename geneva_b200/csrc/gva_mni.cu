@@ -336,11 +336,13 @@ __device__ int lane_dfs(const MniTask& T, const PartPtr* __restrict__ parts, uin
 // for every warp, and steps of 32 candidates a warp may take on a piece before
 // it is cut again: [1] with several items for every warp, [0] with fewer, when
 // a lane's candidates are what the round waits for.  Lane budgets 16 / 32 / 64
-// / 96 / 128, device ms on R-MAT graphs: 1,200 patterns capped at 1,000 (many)
-// 17 / 5.4 / 2.7 / 2.4 / 2.5 (below 64 the queue runs over), 37 exact
-// patterns (few) 0.94 / 0.87 / 1.02 / - / -; 2.9 and 1.4 when the warp searched
-// 32 steps on each such root, one after another, before it gave it away.
-constexpr uint32_t kLaneBudget[2] = {16, 96}, kPieceBudget[2] = {64, 128};
+// / 96 / 128, device ms of 1,200 patterns capped at 1,000 on an R-MAT graph
+// (many): 17 / 5.4 / 2.7 / 2.4 / 2.5 (below 64 the queue runs over; 2.9 when the
+// warp searched 32 steps on each such root, one after another, before it gave
+// it away).  4 / 8 / 16 / 32, ms per call of 37 exact patterns (few): 2.60 /
+// 1.56 / 1.34 / 1.18, smaller calls 0.19 / 0.16 / 0.17 / 0.16; 64 gives 1.08 on
+// one graph and 4 % more on another.
+constexpr uint32_t kLaneBudget[2] = {32, 96}, kPieceBudget[2] = {64, 128};
 
 // What the lanes with `mine` have left of their searches (levels 1 .. i of s)
 // into queue 0, a piece per open level; false: no room, nothing was put there.
