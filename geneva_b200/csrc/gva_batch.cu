@@ -1059,11 +1059,13 @@ __device__ __forceinline__ uint64_t pass_extend(const PassArgs& a, const TaskDes
     return total;
 }
 
-// The same for a plain extension that nothing follows: a lane counts its row.
+// The same for a plain extension that feeds nothing: a lane counts its row.
+// Its node may still have children (none of which can match), so that its
+// mode is MODE_WRITE_AND_GRAPHS.
 __device__ __forceinline__ uint64_t pass_count(const PassArgs& a, const TaskDesc& d, const uint32_t* rows_s,
                                                uint32_t nr, const Found& f) {
     const uint32_t lane = threadIdx.x & 31, R = a.rows_per_item;
-    const bool graphs = d.mode == MODE_COUNT_GRAPHS;
+    const bool graphs = d.mode == MODE_COUNT_GRAPHS || d.mode == MODE_WRITE_AND_GRAPHS;
     const uint32_t found = pass_find(d.e, rows_s, nr, R, f);
     uint64_t total = 0;
     for (uint32_t base = 0; base < found; base += 32) {
