@@ -109,6 +109,10 @@ class _Tuning(ctypes.Structure):
                 ("default_ms", ctypes.c_double), ("tried", ctypes.c_uint32), ("round_region_mb", ctypes.c_uint32)]
 
 
+class _Limits(ctypes.Structure):
+    _fields_ = [("mni_pieces", ctypes.c_uint32), ("mni_roots", ctypes.c_uint32), ("mni_groups", ctypes.c_uint32)]
+
+
 class _BatchStats(ctypes.Structure):
     _fields_ = [("gpu_ms", ctypes.c_double), ("rounds", ctypes.c_uint64), ("splits", ctypes.c_uint64),
                 ("launches", ctypes.c_uint64), ("trie_nodes", ctypes.c_uint64), ("kernels", _KernelStat * 5),
@@ -169,6 +173,7 @@ def _declare(lib):
         "gva_batch_count_texts": (i32, [vp, vp, i32, i32, P(_BatchOpts), vp, vp, vp, vp, P(_BatchStats)]),
         "gva_db_get_tuning": (i32, [vp, P(_Tuning)]),
         "gva_db_set_tuning": (i32, [vp, P(_Tuning)]),
+        "gva_db_set_limits": (i32, [vp, P(_Limits)]),
         "gva_db_autotune": (i32, [vp, vp, i32, vp, P(_Tuning)]),
         "gva_mine_host": (i32, [u32, vp, u32, vp, u32, u32, u32, EVAL_FN, vp, REDUCE_FN, vp, P(vp)]),
         "gva_mine_num_patterns": (i32, [vp]),
@@ -257,6 +262,11 @@ class Database:
         (0 keeps the current size)."""
         t = _Tuning(rows_per_item, hub, 0.0, 0.0, 0, round_region_mb)
         _check(library().gva_db_set_tuning(self._h, ctypes.byref(t)))
+
+    def set_limits(self, **limits) -> None:
+        """Capacities of internal queues (gva_limits: mni_pieces, mni_roots,
+        mni_groups); results don't depend on them."""
+        _check(library().gva_db_set_limits(self._h, ctypes.byref(_Limits(**limits))))
 
     def autotune(self, plans, stream: Optional[int] = None) -> dict:
         """Times a calibration batch under each candidate launch shape and keeps
@@ -627,7 +637,7 @@ def mine(db: Database, max_edges: int, min_support: int, stream: Optional[int] =
     place) combines each level's counts across processes holding disjoint
     graph shards (graph support only).  `cancel` (a ctypes.c_int another
     thread may set to 1) stops the run at its next batch or round boundary
-    with GenevaError status 7.  sm_percent (MNI) caps the share of the SMs
+    (MNI: within a few launches) with GenevaError status 7.  sm_percent (MNI) caps the share of the SMs
     the search kernel fills and host_threads the host threads used (0 = all),
     so that a server's other work keeps running.  Returns (patterns, stats);
     stats["kernels"] is filled when profiling."""

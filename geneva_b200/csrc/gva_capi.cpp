@@ -641,6 +641,17 @@ int gva_db_set_tuning(gva_db* db, const gva_tuning* t) {
     return GVA_OK;
 }
 
+int gva_db_set_limits(gva_db* db, const gva_limits* l) {
+    if (!db || !l) return fail(GVA_ERR_ARG, "null argument");
+    if ((l->mni_pieces && l->mni_pieces < 32) || (l->mni_roots && l->mni_roots < 32))
+        return fail(GVA_ERR_ARG, "mni_pieces and mni_roots must be 32 or more");  // a warp's roots must fit
+    DevDB& d = *db->dev;
+    if (l->mni_pieces) d.mni_pieces = l->mni_pieces;
+    if (l->mni_roots) d.mni_roots = l->mni_roots;
+    if (l->mni_groups) d.mni_groups = l->mni_groups;
+    return GVA_OK;
+}
+
 int gva_db_autotune(gva_db* db, const gva_plan* const* plans, int nplans, void* stream, gva_tuning* out) {
     if (!db || nplans <= 0 || !plans) return fail(GVA_ERR_ARG, "null argument");
     std::vector<std::vector<Step>> steps(nplans);

@@ -48,6 +48,10 @@ struct DevDB {
     // one-pass rounds (BatchSession::run_pages): bytes of each of a
     // run's two frontier regions; doubled after a run that overflowed them
     std::atomic<uint64_t> round_region_bytes{0};
+    // MNI searches (gva_mni.cu): pieces of unfinished searches per queue and
+    // roots that they may belong to, groups of 32 seeds that a warp does in one
+    // launch (512 x a lane's 96 candidates: some tens of milliseconds)
+    uint32_t mni_pieces = 1u << 18, mni_roots = 1u << 18, mni_groups = 512;
 };
 
 int upload_graph(HostGraph& g, int device, DevDB*& out);

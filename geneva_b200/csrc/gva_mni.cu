@@ -41,6 +41,7 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <cstddef>
 #include <cstring>
 #include <memory>
 #include <string>
@@ -212,33 +213,57 @@ __device__ int warp_search(const MniTask& T, const PartPtr* __restrict__ parts, 
 }
 
 // What is left of a search that ran out of its budget, as pieces that any
-// warp can take: the matched prefix f[0 .. level) and a range of the
-// candidates of `level`, read from the segment of f[gsel].
+// warp can take: the matched prefix f[0 .. top) and what is left of the
+// candidates of the levels base .. top, each read from the segment of f[gsel].
+// A piece cut from one level has base == top; a whole search put back has all
+// of its open levels.
 struct MniWork {
-    uint32_t hard;  // the root's flag in MniHard::found
+    uint32_t hard;    // the root's flag in MniHard::found
     uint32_t task;
-    uint32_t cap;   // of the root's slot
-    uint32_t level;
-    uint32_t pos, end;
-    uint32_t gsel;
+    uint32_t cap;     // of the root's slot
+    uint32_t levels;  // base | top << 8
+    uint32_t gsel;    // 4 bits per level
     uint32_t f[kMniMaxVertices - 1];
+    uint32_t pos[kMniMaxVertices - 1], end[kMniMaxVertices - 1];  // of level k + 1
+    uint32_t pad[6];  // a 128-byte line
 };
 constexpr uint32_t kWorkWords = sizeof(MniWork) / 4;
-static_assert(kWorkWords <= 32, "one lane per word");
+constexpr uint32_t kWorkF = 5, kWorkPos = kWorkF + kMniMaxVertices - 1, kWorkEnd = kWorkPos + kMniMaxVertices - 1;
+static_assert(kWorkWords == 32 && kWorkEnd + kMniMaxVertices - 1 <= 32, "one lane per word");
+static_assert(offsetof(MniWork, f) == 4 * kWorkF && offsetof(MniWork, end) == 4 * kWorkEnd, "words by lane");
 
 // The pieces of one round: two queues (a launch takes from one and puts what
 // its searches leave into the other) and the roots they belong to.
+//
+// No launch searches a root to its end.  A queue of cap_work pieces always has
+// room for what a launch leaves: of the n pieces that it takes each may put one
+// back, whole, and only the cap_work - n entries beyond those are given to
+// searches that are cut (extra).  A root that finds no room stays with its seed
+// (MniSave).  Whatever the graph, a launch of the pieces thus lasts as long as
+// cap_work / resident warps times a budget, 262,144 / 7,104 x 128 steps: some
+// milliseconds; a root's flag and its task's count are looked at before each
+// budget, and the host looks at `cancel` after every fourth launch.
 struct MniHard {
     MniWork* queue[2];
-    unsigned long long* state;  // [0 .. 2) = queue 0: pieces, head; [2 .. 4) = queue 1; [4] = roots
+    // per queue {pieces, head, extra}; roots; warps of the search kernel that stopped early
+    unsigned long long* state;
     uint32_t* found;            // per root: an embedding was found
     uint32_t cap_work, cap_roots;
 };
-constexpr uint32_t kMniWorkCap = 1u << 18, kMniRootCap = 1u << 18;
+constexpr uint32_t kQueueWords = 3, kRootsWord = 2 * kQueueWords, kLeftWord = kRootsWord + 1, kStateWords = kLeftWord + 1;
 constexpr uint32_t kMniPieces = 16;      // pieces of one level's range
-constexpr uint32_t kMniCrowded = 1u << 15;  // with this many pieces waiting, ranges are no longer cut
+constexpr uint32_t kMniCrowded = 1u << 15;  // with this many pieces waiting, searches are no longer cut
 
-// Room for n entries in a counted array of `cap`; cap or more: there is none.
+// Where a warp of the search kernel stopped: the lanes `mask` of the group of
+// 32 seeds at c0 of an item are undecided, the seeds behind them untouched.
+struct MniSave {
+    unsigned long long item;  // ~0: nothing left of an item
+    uint32_t c0, mask;
+};
+constexpr unsigned long long kNoItem = ~0ull;
+
+// Room for n more entries in a counted array of `cap`; cap or more: there is
+// none.
 __device__ __forceinline__ unsigned long long reserve(unsigned long long* count, uint32_t n, uint32_t cap) {
     unsigned long long at = *(volatile unsigned long long*)count;
     while (at + n <= cap) {
@@ -246,40 +271,57 @@ __device__ __forceinline__ unsigned long long reserve(unsigned long long* count,
         if (seen == at) return at;
         at = seen;
     }
-    return cap;
+    return ~0ull;
 }
 
-// Puts the open levels base .. i of a search into queue `q`; false: it is
-// full (nothing was put there).
-__device__ bool put_pieces(const MniHard& H, int q, const Dfs& s, int base, int i, uint32_t hard, uint32_t task,
-                           uint32_t cap, uint32_t lane) {
-    unsigned long long* count = H.state + 2 * q;
-    uint32_t most = 1, total = 0;
-    unsigned long long at = 0;
-    if (lane == 0) most = *(volatile unsigned long long*)count < kMniCrowded ? kMniPieces : 1;
-    most = __shfl_sync(0xffffffffu, most, 0);
+// Puts the open levels base .. i of a search into queue `q`, while `taken`
+// pieces are taken from the other one: cut into ranges of candidates, or whole.
+__device__ void put_pieces(const MniHard& H, int q, unsigned long long taken, const Dfs& s, int base, int i,
+                           uint32_t hard, uint32_t task, uint32_t cap, uint32_t lane) {
+    unsigned long long* count = H.state + kQueueWords * q;
+    uint32_t total = 0;
     for (int j = base; j <= i; ++j)
-        if (s.pos[j] < s.end[j]) total += min(most, s.end[j] - s.pos[j]);
-    if (lane == 0) at = reserve(count, total, H.cap_work);
+        if (s.pos[j] < s.end[j]) total += min(kMniPieces, s.end[j] - s.pos[j]);
+    if (total == 0) return;
+    bool cut = false;
+    unsigned long long at = 0;
+    if (lane == 0) {
+        cut = *(volatile unsigned long long*)count < min(kMniCrowded, H.cap_work) &&
+              reserve(count + 2, total - 1, H.cap_work - (uint32_t)taken) != ~0ull;
+        at = atomicAdd(count, (unsigned long long)(cut ? total : 1));
+    }
+    cut = __shfl_sync(0xffffffffu, cut, 0);
     at = __shfl_sync(0xffffffffu, at, 0);
-    if (at >= H.cap_work) return total == 0;
+    if (!cut) {
+        uint32_t word = lane == 0 ? hard : lane == 1 ? task : lane == 2 ? cap : lane == 3 ? (uint32_t)(base | i << 8) : 0;
+        uint32_t gsel = 0;
+        for (int j = base; j <= i; ++j) gsel |= s.gsel[j] << 4 * j;
+        if (lane == 4) word = gsel;
+        for (int k = 0; k < i; ++k) {
+            if (lane == kWorkF + k) word = s.f[k];
+            if (k + 1 < base) continue;
+            if (lane == kWorkPos + k) word = s.pos[k + 1];
+            if (lane == kWorkEnd + k) word = s.end[k + 1];
+        }
+        reinterpret_cast<uint32_t*>(H.queue[q] + at)[lane] = word;
+        return;
+    }
     for (int j = base; j <= i; ++j) {
         if (s.pos[j] >= s.end[j]) continue;
-        const uint32_t len = s.end[j] - s.pos[j], np = min(most, len);
+        const uint32_t len = s.end[j] - s.pos[j], np = min(kMniPieces, len);
         if (lane < np) {
             MniWork& w = H.queue[q][at + lane];
             w.hard = hard;
             w.task = task;
             w.cap = cap;
-            w.level = (uint32_t)j;
-            w.pos = s.pos[j] + (uint32_t)((uint64_t)len * lane / np);
-            w.end = s.pos[j] + (uint32_t)((uint64_t)len * (lane + 1) / np);
-            w.gsel = s.gsel[j];
-            for (int k = 0; k < kMniMaxVertices - 1; ++k) w.f[k] = k < j ? s.f[k] : 0u;
+            w.levels = (uint32_t)(j | j << 8);
+            w.gsel = s.gsel[j] << 4 * j;
+            w.pos[j - 1] = s.pos[j] + (uint32_t)((uint64_t)len * lane / np);
+            w.end[j - 1] = s.pos[j] + (uint32_t)((uint64_t)len * (lane + 1) / np);
+            for (int k = 0; k < j; ++k) w.f[k] = s.f[k];
         }
         at += np;
     }
-    return true;
 }
 
 // One lane's own depth-first search for an embedding with level 0 at `root`,
@@ -345,45 +387,61 @@ __device__ int lane_dfs(const MniTask& T, const PartPtr* __restrict__ parts, uin
 constexpr uint32_t kLaneBudget[2] = {32, 96}, kPieceBudget[2] = {64, 128};
 
 // What the lanes with `mine` have left of their searches (levels 1 .. i of s)
-// into queue 0, a piece per open level; false: no room, nothing was put there.
+// into queue 0: a piece per open level, or the whole search as one when many
+// pieces wait or room is short.  false: no room, nothing was put there.
 __device__ bool put_lanes(const MniHard& H, bool mine, const Dfs& s, int i, uint32_t task, uint32_t cap, uint32_t lane) {
-    uint32_t n = 0;
+    uint32_t open = 0;  // open levels
     if (mine)
-        for (int j = 1; j <= i; ++j) n += s.pos[j] < s.end[j] ? 1 : 0;
+        for (int j = 1; j <= i; ++j) open |= s.pos[j] < s.end[j] ? 1u << j : 0;
+    const uint32_t voters = __ballot_sync(0xffffffffu, open != 0);
+    if (!voters) return true;
+    const uint32_t n = __popc(open);
     uint32_t inc = n;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
         if (lane >= (uint32_t)o) inc += y;
     }
-    const uint32_t total = __shfl_sync(0xffffffffu, inc, 31), voters = __ballot_sync(0xffffffffu, mine);
-    unsigned long long at = 0, root = 0;
+    const uint32_t total = __shfl_sync(0xffffffffu, inc, 31), below = __popc(voters & ((1u << lane) - 1u));
+    unsigned long long at = ~0ull, root = ~0ull;
+    bool whole = false;
     if (lane == 0) {
-        root = reserve(H.state + 4, __popc(voters), H.cap_roots);
-        at = root < H.cap_roots ? reserve(H.state, total, H.cap_work) : H.cap_work;
+        root = reserve(H.state + kRootsWord, __popc(voters), H.cap_roots);
+        if (root != ~0ull) {
+            if (*(volatile unsigned long long*)H.state < kMniCrowded) at = reserve(H.state, total, H.cap_work);
+            if (at == ~0ull) {
+                whole = true;
+                at = reserve(H.state, __popc(voters), H.cap_work);
+            }
+        }
     }
     at = __shfl_sync(0xffffffffu, at, 0);
-    root = __shfl_sync(0xffffffffu, root, 0) + __popc(voters & ((1u << lane) - 1u));
-    if (at >= H.cap_work) return total == 0;
-    at += inc - n;
-    if (mine)
-        for (int j = 1; j <= i; ++j) {
-            if (s.pos[j] >= s.end[j]) continue;
-            MniWork& w = H.queue[0][at++];
-            w.hard = (uint32_t)root;
-            w.task = task;
-            w.cap = cap;
-            w.level = (uint32_t)j;
-            w.pos = s.pos[j];
-            w.end = s.end[j];
-            w.gsel = s.gsel[j];
-            for (int k = 0; k < kMniMaxVertices - 1; ++k) w.f[k] = k < j ? s.f[k] : 0u;
+    whole = __shfl_sync(0xffffffffu, whole, 0);
+    if (at == ~0ull) return false;
+    root = __shfl_sync(0xffffffffu, root, 0) + below;
+    at += whole ? below : inc - n;
+    if (whole && open) open = 1u << (31 - __clz(open));  // the deepest one stands for all
+    for (; open; open &= open - 1) {
+        const int top = __ffs(open) - 1, base = whole ? 1 : top;
+        MniWork& w = H.queue[0][at++];
+        w.hard = (uint32_t)root;
+        w.task = task;
+        w.cap = cap;
+        w.levels = (uint32_t)(base | top << 8);
+        uint32_t gsel = 0;
+        for (int j = base; j <= top; ++j) {
+            gsel |= s.gsel[j] << 4 * j;
+            w.pos[j - 1] = s.pos[j];
+            w.end[j - 1] = s.end[j];
         }
+        w.gsel = gsel;
+        for (int k = 0; k < top; ++k) w.f[k] = s.f[k];
+    }
     return true;
 }
 
-// A warp's first item is that of its number, the others come from the queue's
-// head: 7,104 warps asking one counter at once took 10 us, in a launch with
+// A warp's first item is that of its number (or, in a launch that goes on where
+// one stopped, what it has left), the others come from the queue's head: 7,104 warps asking one counter at once took 10 us, in a launch with
 // nothing to do too (4 us now).
 struct FirstThenQueue {
     unsigned long long* head;
@@ -414,7 +472,9 @@ __device__ __forceinline__ void add_prof(unsigned long long* prof, const unsigne
 // Persistent: every warp pulls items; per 32 seeds it checks the
 // task's count against its cap, filters roots by neighbour-label degrees and
 // runs one search per surviving root.  A root that its lane does not decide
-// within its budget goes to the pieces of mni_piece_kernel.
+// within its budget goes to the pieces of mni_piece_kernel.  A warp whose roots
+// find no room there, or that has done max_groups groups, stops and notes where
+// (save); once the pieces are done the host launches the kernel again.
 //
 // Why: nearly every root is decided within a few candidates, but one without
 // an embedding under a hub can take millions of steps (pairs of a hub's
@@ -430,15 +490,29 @@ mni_search_kernel(const MniTask* __restrict__ tasks, const MniSlot* __restrict__
                   const uint64_t* __restrict__ item0, const uint32_t* __restrict__ item_slot, uint64_t nitems,
                   const uint32_t* __restrict__ seeds, uint32_t item_len,
                   const PartPtr* __restrict__ parts, uint32_t L, uint32_t* __restrict__ counts,
-                  unsigned long long* __restrict__ queue, MniHard H, uint32_t lane_budget,
-                  unsigned long long* __restrict__ prof) {
+                  unsigned long long* __restrict__ queue, MniHard H, MniSave* __restrict__ save, bool resume,
+                  uint32_t max_groups, uint32_t lane_budget, unsigned long long* __restrict__ prof) {
     __shared__ MniTask tsh[kMniWarps];
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     MniTask& T = tsh[w];
     unsigned long long cnt[P_NUM] = {0, 0, 0, 0, 0, 0};
     int cur = -1;
     const FirstThenQueue next{queue, gridDim.x * kMniWarps};
-    for (unsigned long long it = blockIdx.x * kMniWarps + w; it < nitems; it = next(lane)) {
+    unsigned long long it = blockIdx.x * kMniWarps + w;
+    uint32_t from = 0xffffffffu, redo = 0xffffffffu, groups = 0;  // of a resumed item: its group, the lanes left in it
+    MniSave* const mine = save + it;
+    if (resume) {
+        it = mine->item;
+        if (it != kNoItem) {
+            from = mine->c0;
+            redo = mine->mask;
+        } else {
+            it = next(lane);
+        }
+    }
+    unsigned long long left = kNoItem;
+    uint32_t left_c0 = 0, left_mask = 0;
+    for (; it < nitems && left == kNoItem; it = next(lane)) {
         const int s = (int)__ldg(item_slot + it);
         const MniSlot sl = slots[s];
         if ((int)sl.task != cur) {
@@ -447,51 +521,60 @@ mni_search_kernel(const MniTask* __restrict__ tasks, const MniSlot* __restrict__
         }
         const uint32_t a = sl.start + (uint32_t)(it - item0[s]) * item_len;
         const uint32_t b = min(a + item_len, sl.start + sl.len);
-        for (uint32_t c0 = a; c0 < b; c0 += 32) {
+        uint32_t c0 = from != 0xffffffffu ? from : a;
+        from = 0xffffffffu;
+        for (; c0 < b; c0 += 32) {
+            if (groups++ == max_groups) {
+                left = it;
+                left_c0 = c0;
+                left_mask = redo;
+                break;
+            }
             // one lane reads the count so that the whole warp takes the same branch
             uint32_t seen = 0;
             if (lane == 0) seen = *(volatile const uint32_t*)(counts + sl.task);
             if (__shfl_sync(0xffffffffu, seen, 0) >= sl.cap) break;
             uint32_t v = 0;
             bool ok = false;
-            if (c0 + lane < b) {
+            if (c0 + lane < b && (redo >> lane & 1)) {
                 v = __ldg(seeds + T.seed_begin + c0 + lane);
                 ok = root_ok(T, parts, L, v);
-                cnt[P_SEEDS] += 1;
+                cnt[P_SEEDS] += redo == 0xffffffffu ? 1 : 0;
             }
             const uint32_t roots = __ballot_sync(0xffffffffu, ok);  // all lanes vote
-            if (lane == 0) cnt[P_ROOTS] += __popc(roots);
+            if (lane == 0) cnt[P_ROOTS] += redo == 0xffffffffu ? __popc(roots) : 0;
+            redo = 0xffffffffu;
             // every lane searches its own root; what a search has left when
             // it runs out of budget is shared out
             int verdict = 0, i = 0;
             Dfs st;
             if (ok) verdict = lane_dfs(T, parts, L, v, lane_budget, st, i, cnt);
-            uint32_t found = __popc(__ballot_sync(0xffffffffu, verdict == 1));
-            uint32_t m = __ballot_sync(0xffffffffu, verdict < 0);
-            if (m && !put_lanes(H, verdict < 0, st, i, sl.task, sl.cap, lane)) {
-                while (m) {  // no room: to their ends here, by the whole warp
-                    const int l = __ffs(m) - 1;
-                    m &= m - 1;
-                    Dfs all;
-                    all.f[0] = __shfl_sync(0xffffffffu, v, l);
-                    int k = 1;
-                    dfs_open(T, parts, L, all, 1);
-                    cnt[P_OPENS] += lane == 0 ? 1 : 0;
-                    if (warp_search(T, parts, L, all, 1, k, 0xffffffffu, lane, cnt) > 0) ++found;
-                }
-            }
+            const uint32_t found = __popc(__ballot_sync(0xffffffffu, verdict == 1));
+            const uint32_t m = __ballot_sync(0xffffffffu, verdict < 0);
             if (found && lane == 0) atomicAdd(counts + sl.task, found);
             if (lane == 0) cnt[P_FOUND] += found;
+            if (m && !put_lanes(H, verdict < 0, st, i, sl.task, sl.cap, lane)) {
+                left = it;
+                left_c0 = c0;
+                left_mask = m;
+                break;
+            }
         }
+        redo = 0xffffffffu;
+        if (left != kNoItem) break;  // the queue's next item is for another warp
+    }
+    if (lane == 0) {
+        *mine = MniSave{left, left_c0, left_mask};
+        if (left != kNoItem) atomicAdd(H.state + kLeftWord, 1ull);
     }
     add_prof(prof, cnt, lane);
 }
 
 // The pieces of queue q, one per warp at a time: each is searched for up to
-// `piece_budget` steps and what is left goes, cut again, to the other queue (a
-// search thus spreads over the chip within two or three launches).  The first
-// embedding of a root counts it; the root's other pieces are then skipped, as
-// are pieces of a task at its cap.
+// `piece_budget` steps and what is left goes, cut again or whole, to the other
+// queue (a search thus spreads over the chip within two or three launches).
+// The first embedding of a root counts it; the root's other pieces are then
+// skipped, as are pieces of a task at its cap.
 __global__ void __launch_bounds__(kMniWarps * 32, 6)
 mni_piece_kernel(const MniTask* __restrict__ tasks, const PartPtr* __restrict__ parts, uint32_t L,
                  uint32_t* __restrict__ counts, MniHard H, int q, uint32_t piece_budget,
@@ -500,13 +583,12 @@ mni_piece_kernel(const MniTask* __restrict__ tasks, const PartPtr* __restrict__ 
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     MniTask& T = tsh[w];
     unsigned long long cnt[P_NUM] = {0, 0, 0, 0, 0, 0};
-    unsigned long long* state = H.state + 2 * q;
+    unsigned long long* state = H.state + kQueueWords * q;
     const unsigned long long n = state[0];  // only read by this launch
     uint32_t cur = 0xffffffffu;
     const FirstThenQueue next{state + 1, gridDim.x * kMniWarps};
     for (unsigned long long it = blockIdx.x * kMniWarps + w; it < n; it = next(lane)) {
-        uint32_t word = 0;
-        if (lane < kWorkWords) word = __ldg(reinterpret_cast<const uint32_t*>(H.queue[q] + it) + lane);
+        const uint32_t word = __ldg(reinterpret_cast<const uint32_t*>(H.queue[q] + it) + lane);
         auto field = [&](int k) { return __shfl_sync(0xffffffffu, word, k); };
         const uint32_t hard = field(0), task = field(1), cap = field(2);
         bool skip = false;
@@ -517,17 +599,19 @@ mni_piece_kernel(const MniTask* __restrict__ tasks, const PartPtr* __restrict__ 
             load_task(T, tasks + task, lane);
             cur = task;
         }
-        const int base = (int)field(3);
+        const uint32_t levels = field(3), gsel = field(4);
+        const int base = (int)(levels & 0xff);
+        int i = (int)(levels >> 8);
         Dfs s;
-        for (int k = 0; k < kMniMaxVertices - 1; ++k) s.f[k] = field(7 + k);
-        s.pos[base] = field(4);
-        s.end[base] = field(5);
-        s.gsel[base] = field(6);
-        s.gadj[base] = parts[T.part[base][s.gsel[base]] - 1].adj;
-        int i = base;
-        int r = warp_search(T, parts, L, s, base, i, piece_budget, lane, cnt);
-        if (r < 0 && !put_pieces(H, q ^ 1, s, base, i, hard, task, cap, lane))
-            r = warp_search(T, parts, L, s, base, i, 0xffffffffu, lane, cnt);
+        for (int k = 0; k < i; ++k) s.f[k] = field(kWorkF + k);
+        for (int j = base; j <= i; ++j) {
+            s.pos[j] = field(kWorkPos + j - 1);
+            s.end[j] = field(kWorkEnd + j - 1);
+            s.gsel[j] = gsel >> 4 * j & 15u;
+            s.gadj[j] = parts[T.part[j][s.gsel[j]] - 1].adj;
+        }
+        const int r = warp_search(T, parts, L, s, base, i, piece_budget, lane, cnt);
+        if (r < 0) put_pieces(H, q ^ 1, n, s, base, i, hard, task, cap, lane);
         if (r > 0 && lane == 0 && atomicExch(H.found + hard, 1u) == 0) {
             atomicAdd(counts + task, 1u);
             cnt[P_FOUND] += 1;
@@ -782,10 +866,16 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
     // the counts, the search queue's head and the pieces' state lie together:
     // one copy reads back the counts and whether pieces are left
-    const size_t o_queue = (bytes_counts + 15) & ~(size_t)15, bytes_state = 6 * 8;
-    const size_t bytes_found = (size_t)kMniRootCap * 4, bytes_work = 2 * (size_t)kMniWorkCap * sizeof(MniWork);
+    const size_t o_queue = (bytes_counts + 15) & ~(size_t)15, bytes_state = (1 + kStateWords) * 8;
+    int sms = 148, per_sm = 1;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, db.device);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mni_search_kernel, kMniWarps * 32, 0);
+    per_sm = std::max(per_sm, 1);
+    const uint32_t cap_work = db.mni_pieces, cap_roots = db.mni_roots;
+    const size_t bytes_found = (size_t)cap_roots * 4, bytes_work = 2 * (size_t)cap_work * sizeof(MniWork);
+    const size_t bytes_save = (size_t)per_sm * sms * kMniWarps * sizeof(MniSave);
     const size_t fixed = al(bytes_tasks) + al(o_queue + bytes_state) + al(bytes_parts) + al(bytes_prof) +
-                         al(bytes_found) + bytes_work;
+                         al(bytes_found) + al(bytes_save) + bytes_work;
     if (cudaMallocAsync(&dmem, fixed, s) != cudaSuccess) return fail(GVA_ERR_NOMEM, "MNI task allocation failed");
     struct Free {
         void* p;
@@ -805,11 +895,13 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
     MniHard H{};
     H.found = (uint32_t*)cur;
     cur += al(bytes_found);
+    MniSave* d_save = (MniSave*)cur;
+    cur += al(bytes_save);
     H.queue[0] = (MniWork*)cur;
-    H.queue[1] = H.queue[0] + kMniWorkCap;
+    H.queue[1] = H.queue[0] + cap_work;
     H.state = d_queue + 1;
-    H.cap_work = kMniWorkCap;
-    H.cap_roots = kMniRootCap;
+    H.cap_work = cap_work;
+    H.cap_roots = cap_roots;
     // every host<->device copy goes through pinned staging: a pageable copy
     // blocks its thread inside the driver until the stream drains, which
     // other threads' CUDA calls (a server's matching loop) would wait behind
@@ -825,11 +917,6 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
     GVA_CUDA_M(cudaMemsetAsync(d_counts, 0, bytes_counts, s));
     GVA_CUDA_M(cudaMemsetAsync(d_prof, 0, bytes_prof, s));
     GVA_CUDA_M(cudaMemsetAsync(H.found, 0, bytes_found, s));
-
-    int sms = 148, per_sm = 1;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, db.device);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mni_search_kernel, kMniWarps * 32, 0);
-    per_sm = std::max(per_sm, 1);
 
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     GVA_CUDA_M(cudaEventCreate(&e0));
@@ -925,50 +1012,60 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
             const double rows = (double)total;
             mni_expand_kernel<<<(unsigned)std::min<uint64_t>((ns + 255) / 256, 4096), 256, 0, s>>>(d_item0, ns,
                                                                                                   d_item_slot);
-            if (profile) prof.begin(K_MNI, 0.0, s, ev);
-            mni_search_kernel<<<(unsigned)std::max<uint64_t>(grid, 1), kMniWarps * 32, 0, s>>>(
-                d_tasks, d_slots, d_item0, d_item_slot, nitems, db.seed_by_degree, (uint32_t)item_len, d_parts, db.kernel_L(),
-                d_counts, d_queue, H, kLaneBudget[many], profile ? d_prof : nullptr);
-            if (profile) prof.end(ev, K_MNI, 0.0, s, rows);
-            st.launches += 2;
-            g_mni_launches += 2;
+            st.launches += 1;
+            g_mni_launches += 1;
             st.rounds++;
-            // counts back, and how many pieces are left for the piece kernel:
-            // they are taken four launches at a time until none is
+            // a search launch, then the pieces that it left until none is, four
+            // launches per look at their number; again while it stopped early
             const unsigned long long* hstate = (const unsigned long long*)((const char*)hcounts + o_queue) + 1;
-            uint64_t hard_roots = 0;
-            for (int q = 0;;) {
-                cudaError_t le = cudaGetLastError();
-                if (le == cudaSuccess) le = cudaMemcpyAsync(hcounts, d_counts, bytes_back, cudaMemcpyDeviceToHost, s);
-                if (le != cudaSuccess) {
-                    rc = fail(GVA_ERR_CUDA, std::string("MNI search launch failed: ") + cudaGetErrorString(le));
-                    break;
+            for (bool resume = false;; resume = true) {
+                if (profile) prof.begin(K_MNI, 0.0, s, ev);
+                mni_search_kernel<<<(unsigned)std::max<uint64_t>(grid, 1), kMniWarps * 32, 0, s>>>(
+                    d_tasks, d_slots, d_item0, d_item_slot, nitems, db.seed_by_degree, (uint32_t)item_len, d_parts,
+                    db.kernel_L(), d_counts, d_queue, H, d_save, resume, db.mni_groups, kLaneBudget[many],
+                    profile ? d_prof : nullptr);
+                if (profile) prof.end(ev, K_MNI, 0.0, s, resume ? 0.0 : rows);
+                st.launches += 1;
+                g_mni_launches += 1;
+                for (int q = 0;;) {
+                    cudaError_t le = cudaGetLastError();
+                    if (le == cudaSuccess) le = cudaMemcpyAsync(hcounts, d_counts, bytes_back, cudaMemcpyDeviceToHost, s);
+                    if (le != cudaSuccess) {
+                        rc = fail(GVA_ERR_CUDA, std::string("MNI search launch failed: ") + cudaGetErrorString(le));
+                        break;
+                    }
+                    const auto w0 = std::chrono::steady_clock::now();
+                    const cudaError_t e = cudaStreamSynchronize(s);
+                    st.wait_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - w0).count();
+                    if (e != cudaSuccess) {
+                        rc = fail(GVA_ERR_CUDA, std::string("MNI search failed: ") + cudaGetErrorString(e));
+                        break;
+                    }
+                    if (hstate[kQueueWords * q] == 0) break;
+                    if (cancel && *cancel) {
+                        rc = fail(GVA_ERR_CANCELLED, "cancelled");
+                        break;
+                    }
+                    for (int k = 0; k < 4; ++k, q ^= 1) {
+                        cudaMemsetAsync(H.state + kQueueWords * (q ^ 1), 0, kQueueWords * 8, s);  // taken by the launch before
+                        if (profile) prof.begin(K_MNI, 0.0, s, ev);
+                        mni_piece_kernel<<<(unsigned)cta_cap, kMniWarps * 32, 0, s>>>(
+                            d_tasks, d_parts, db.kernel_L(), d_counts, H, q, kPieceBudget[many], profile ? d_prof : nullptr);
+                        if (profile) prof.end(ev, K_MNI, 0.0, s, 0.0);
+                    }
+                    st.launches += 4;
+                    g_mni_launches += 4;
                 }
-                const auto w0 = std::chrono::steady_clock::now();
-                const cudaError_t e = cudaStreamSynchronize(s);
-                st.wait_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - w0).count();
-                if (e != cudaSuccess) {
-                    rc = fail(GVA_ERR_CUDA, std::string("MNI search failed: ") + cudaGetErrorString(e));
-                    break;
-                }
-                hard_roots = hstate[4];
-                if (hstate[2 * q] == 0) break;
+                if (rc) break;
+                if (hstate[kRootsWord]) cudaMemsetAsync(H.found, 0, hstate[kRootsWord] * 4, s);
+                if (hstate[kLeftWord] == 0) break;
                 if (cancel && *cancel) {
                     rc = fail(GVA_ERR_CANCELLED, "cancelled");
                     break;
                 }
-                for (int k = 0; k < 4; ++k, q ^= 1) {
-                    cudaMemsetAsync(H.state + 2 * (q ^ 1), 0, 16, s);  // taken by the launch before
-                    if (profile) prof.begin(K_MNI, 0.0, s, ev);
-                    mni_piece_kernel<<<(unsigned)cta_cap, kMniWarps * 32, 0, s>>>(
-                        d_tasks, d_parts, db.kernel_L(), d_counts, H, q, kPieceBudget[many], profile ? d_prof : nullptr);
-                    if (profile) prof.end(ev, K_MNI, 0.0, s, 0.0);
-                }
-                st.launches += 4;
-                g_mni_launches += 4;
+                cudaMemsetAsync(H.state, 0, kStateWords * 8, s);
             }
             if (rc) break;
-            if (hard_roots) cudaMemsetAsync(H.found, 0, hard_roots * 4, s);
             memcpy(counts.data(), hcounts, bytes_counts);
             // exhausted tasks fix their pattern's cap; capped ones retire
             w = 0;

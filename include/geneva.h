@@ -271,6 +271,16 @@ int gva_db_set_tuning(gva_db* db, const gva_tuning* tuning);
  * on this database.  Every shape must give the same counts. */
 int gva_db_autotune(gva_db* db, const gva_plan* const* plans, int nplans, void* stream, gva_tuning* out);
 
+/* Capacities of internal queues on one database.  Results don't depend on
+ * them; smaller ones take less memory and more launches.  0 leaves a field as
+ * it is.  Not to be changed while a call on the database runs. */
+typedef struct gva_limits {
+    uint32_t mni_pieces;  /* MNI: pieces of unfinished searches per queue, 128 bytes each (32 or more; 262144) */
+    uint32_t mni_roots;   /* MNI: roots that they may belong to at once (32 or more; 262144) */
+    uint32_t mni_groups;  /* MNI: groups of 32 seeds that a warp does per launch (512) */
+} gva_limits;
+int gva_db_set_limits(gva_db* db, const gva_limits* limits);
+
 /* ---- serving: a persistent batch -------------------------------------------
  * The batched engine kept open: plans may be submitted at any time and join
  * the running work at the next round (continuous batching); each round
@@ -318,7 +328,8 @@ typedef struct gva_mine_opts {
     uint32_t support_mode; /* GVA_SUPPORT_GRAPHS or GVA_SUPPORT_MNI */
     uint32_t mni_cap;      /* MNI: supports are min(MNI, mni_cap); 0 = min_support */
     const volatile int* cancel; /* optional: once *cancel != 0 (set by another thread), the run stops at
-                                   its next batch or round boundary with GVA_ERR_CANCELLED */
+                                   its next batch or round boundary (MNI: within a few launches of
+                                   its searches, tens of milliseconds) with GVA_ERR_CANCELLED */
     uint32_t sm_percent;   /* MNI: the search kernel fills at most this share of the SMs (0 = all),
                               leaving room for other work on the GPU (a server's matching rounds) */
     uint32_t host_threads; /* host threads for candidate generation and planning (0 = all cores) */
