@@ -992,7 +992,8 @@ def batch_bench(args, rank, world, local, dist, torch, gv, workloads):
                                         "path": f"the same step with every round scheduled on the {other} "
                                                 f"(GVA_BATCH_{other.upper()}_ROUNDS), mean of 2 after 1 warm-up"}),
         "tuning": dict(tuning, calibration=f"first {min(args.tune_patterns, len(plans))} patterns of the list, "
-                                           f"counted with supports, each launch shape twice (gva_db_autotune)"),
+                                           f"counted with supports: rows by one-pass rounds, hub by counted rounds "
+                                           f"(gva_db_autotune)"),
         "e2e": {"value": e2e_value, "unit": "embeddings/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "note": "pattern texts read, planned on the host's cores and matched in one call each step "
                         "(gva_batch_count_texts), counts and supports copied to host memory; database resident",

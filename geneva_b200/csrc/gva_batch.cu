@@ -2597,6 +2597,16 @@ void trim_round_pool(int device) {
     if (pool) cudaMemPoolTrimTo(pool, (size_t)9 << 30);
 }
 
+// Rows of a page, before wide rows cut it: twice the tuned rows (128 by
+// default) where a tenth of them is left after the lookups.  64 / 128 rows, per
+// call: 16,384 patterns 9.1 / 8.2 ms, 1,501 texts 2.04 / 1.96 ms, 16 patterns
+// 458 / 447 us.  With long lists nearly all are left, items differ more, and
+// every piece stages its whole item: 32 / 64 / 128 rows, 61 queries on an R-MAT
+// graph 604 / 570 / 621 us.
+static uint32_t page_rows(const DevDB& db, uint32_t rows_per_item) {
+    return std::min<uint32_t>((db.max_degree > kUnitLen ? 1 : 2) * rows_per_item, kMaxItemRows);
+}
+
 int BatchSession::run_pages() {
     if (host_rounds || profile || waves.size() != 1 || rounds != 0 || active.empty() || !db.seed_verts) return GVA_OK;
     const auto t_start = std::chrono::steady_clock::now();
@@ -2660,13 +2670,7 @@ int BatchSession::run_pages() {
     const bool long_lists = db.max_degree > kUnitLen;
     std::vector<uint32_t> R(D + 2, 32);
     for (int d = 1; d <= D; ++d) {
-        // twice the tuned rows (128 by default) where a tenth of them is left
-        // after the lookups.  64 / 128 rows, per call: 16,384 patterns 9.1 /
-        // 8.2 ms, 1,501 texts 2.04 / 1.96 ms, 16 patterns 458 / 447 us.  With
-        // long lists nearly all are left, items differ more, and every piece
-        // stages its whole item: 32 / 64 / 128 rows, 61 queries on an R-MAT
-        // graph 604 / 570 / 621 us
-        R[d] = std::min<uint32_t>((long_lists ? 1 : 2) * tune.rows_per_item, std::max<uint32_t>(32, (768 / kmax[d]) & ~31u));
+        R[d] = std::min<uint32_t>(page_rows(db, tune.rows_per_item), std::max<uint32_t>(32, (768 / kmax[d]) & ~31u));
         R[d] = R[d] >= 128 ? 128 : R[d] >= 64 ? 64 : 32;  // a power of two (stage_page)
     }
     uint2* h_tasks = (uint2*)(h + o_tasks);
@@ -3281,55 +3285,77 @@ int run_batch(DevDB& db, std::vector<std::vector<Step>> steps, cudaStream_t s, u
 }
 
 // Candidate launch shapes: rows per work item x the list length from which a
-// row's candidates are shared by its warp (1 << 30: never).  Each shape runs
-// the calibration batch twice; the faster run counts.
+// row's candidates are shared by its warp (1 << 30: never).  Rows per item are
+// chosen by one-pass rounds, the default path; their kernels have no list
+// length, which is chosen by counted rounds (sessions, profiled runs, small
+// budgets) at those rows.  Row counts that give one-pass rounds the same pages
+// are timed there once and told apart by counted rounds.  A run's fastest of
+// three counts, and a shape takes the default's place only if it is more than
+// 3 % faster: repeated runs of one shape differ by 1-2 %.
 int autotune_batch(DevDB& db, const std::vector<std::vector<Step>>& steps, cudaStream_t s, bool per_graph,
                    TuneResult& out) {
     out = TuneResult();
     if (steps.empty()) return fail(GVA_ERR_ARG, "empty calibration batch");
-    const uint32_t keep_r = db.tune_rows_per_item, keep_h = db.tune_hub;
-    const uint32_t rows[] = {32, 64, 128};
-    const uint32_t hubs[] = {16, 32, 64, 1u << 30};
+    struct Keep {  // the database's own shape again, unless the end is reached
+        DevDB& db;
+        uint32_t r = db.tune_rows_per_item, h = db.tune_hub;
+        ~Keep() {
+            db.tune_rows_per_item = r;
+            db.tune_hub = h;
+        }
+    } keep{db};
+    constexpr int kRows = 3, kHubs = 4, kDefRow = 1, kDefHub = 1;
+    const uint32_t rows[kRows] = {32, 64, 128};
+    const uint32_t hubs[kHubs] = {16, 32, 64, 1u << 30};
     std::vector<uint64_t> counts(steps.size()), first_counts;
     std::vector<uint32_t> sup(per_graph ? steps.size() : 0);
-    double best = 1e300;
-    int rc = GVA_OK;
-    for (uint32_t r : rows) {
-        for (uint32_t hb : hubs) {
-            db.tune_rows_per_item = r;
-            db.tune_hub = hb;
-            double t = 1e300;
-            for (int rep = 0; rep < 2 && !rc; ++rep) {
-                BatchStats bs;
-                rc = run_batch(db, steps, s, 0, nullptr, 0, counts.data(), nullptr, per_graph ? sup.data() : nullptr,
-                               false, &bs);
-                t = std::min(t, bs.gpu_ms);
-            }
-            if (rc) break;
-            if (first_counts.empty()) {
-                first_counts = counts;
-            } else if (counts != first_counts) {  // every shape counts the same rows
-                rc = fail(GVA_ERR_CUDA, "launch shapes disagree on the calibration counts");
-                break;
-            }
-            out.tried.push_back({(double)r, (double)hb, t});
-            if (r == 64 && hb == 32) out.default_ms = t;
-            if (t < best) {
-                best = t;
-                out.rows_per_item = r;
-                out.hub = hb;
-            }
+    auto timed = [&](int mode, double& t) {
+        t = 1e300;
+        for (int rep = 0; rep < 3; ++rep) {
+            BatchStats bs;
+            const int rc = run_batch(db, steps, s, 0, nullptr, 0, counts.data(), nullptr,
+                                     per_graph ? sup.data() : nullptr, false, &bs, mode);
+            if (rc) return rc;
+            t = std::min(t, bs.gpu_ms);
         }
-        if (rc) break;
+        if (first_counts.empty()) first_counts = counts;
+        return counts == first_counts ? GVA_OK  // every shape counts the same rows
+                                      : fail(GVA_ERR_CUDA, "launch shapes disagree on the calibration counts");
+    };
+    double pass[kRows], counted[kRows][kHubs];
+    for (int i = 0; i < kRows; ++i) {
+        db.tune_rows_per_item = rows[i];
+        int same = 0;
+        while (page_rows(db, rows[same]) != page_rows(db, rows[i])) ++same;
+        if (same < i) {
+            pass[i] = pass[same];
+        } else {
+            const int rc = timed(ROUNDS_AUTO, pass[i]);
+            if (rc) return rc;
+        }
+        for (int j = 0; j < kHubs; ++j) {
+            db.tune_hub = hubs[j];
+            const int rc = timed(ROUNDS_HOST, counted[i][j]);
+            if (rc) return rc;
+            out.tried.push_back({(double)rows[i], (double)hubs[j], counted[i][j]});
+        }
     }
-    if (rc) {
-        db.tune_rows_per_item = keep_r;
-        db.tune_hub = keep_h;
-        return rc;
-    }
-    out.ms = best;
-    db.tune_rows_per_item = out.rows_per_item;
-    db.tune_hub = out.hub;
+    auto faster = [](double a, double b) { return a < 0.97 * b; };
+    int br = kDefRow;
+    for (int i = 0; i < kRows; ++i)
+        if (faster(pass[i], pass[kDefRow]) && pass[i] < pass[br]) br = i;
+    auto best_hub = [&](int i) {
+        int bh = kDefHub;
+        for (int j = 0; j < kHubs; ++j)
+            if (faster(counted[i][j], counted[i][kDefHub]) && counted[i][j] < counted[i][bh]) bh = j;
+        return bh;
+    };
+    for (int i = 0, to = br; i < kRows; ++i)
+        if (pass[i] == pass[to] && faster(counted[i][best_hub(i)], counted[br][best_hub(br)])) br = i;
+    keep.r = out.rows_per_item = rows[br];
+    keep.h = out.hub = hubs[best_hub(br)];
+    out.ms = pass[br];
+    out.default_ms = pass[kDefRow];
     return GVA_OK;
 }
 

@@ -255,8 +255,8 @@ int gva_batch_count_texts(gva_db* db, const char* const* query_texts, int n, int
 typedef struct gva_tuning {
     uint32_t rows_per_item;
     uint32_t hub;
-    double ms;          /* gva_db_autotune: calibration time of the chosen shape */
-    double default_ms;  /* gva_db_autotune: calibration time of the default shape */
+    double ms;          /* gva_db_autotune: calibration time at the chosen rows (one-pass rounds) */
+    double default_ms;  /* gva_db_autotune: the same at the default rows */
     uint32_t tried;     /* gva_db_autotune: shapes timed */
     /* MiB of each of the two frontier regions of one-pass rounds
      * (0: unchanged by gva_db_set_tuning; default 2048); doubled after a run
@@ -266,9 +266,10 @@ typedef struct gva_tuning {
 int gva_db_get_tuning(const gva_db* db, gva_tuning* out);
 int gva_db_set_tuning(gva_db* db, const gva_tuning* tuning);
 /* Counts a calibration batch (as gva_batch_count does, with supports when
- * the database has graph ids) under each candidate launch shape, twice each,
- * and keeps the fastest for every later batched run, mining run and session
- * on this database.  Every shape must give the same counts. */
+ * the database has graph ids), three times each under the candidate rows per
+ * item with one-pass rounds and under the hub lengths with counted rounds, and
+ * keeps the fastest for every later batched run, mining run and session on
+ * this database.  Every shape must give the same counts. */
 int gva_db_autotune(gva_db* db, const gva_plan* const* plans, int nplans, void* stream, gva_tuning* out);
 
 /* Capacities of internal queues on one database.  Results don't depend on
