@@ -29,6 +29,7 @@
 #include "../../include/geneva.h"
 #include "gva_engine.cuh"
 #include "gva_kernels.cuh"
+#include "gva_pool.h"
 
 namespace gva {
 
@@ -903,6 +904,23 @@ constexpr uint64_t kChainRows = 1ull << 22;
 constexpr size_t kChainResult = 256u << 10;
 constexpr size_t kChainSteps = 64;
 
+// What a query's step leads one to expect of its rows, of the steps before it:
+// the degrees as the database has them, labels and edges as if independent.
+// Column labels are kept in `lab`.
+double expected_rows(const DevDB& db, const Step& st, size_t i, double rows, std::vector<uint32_t>& lab) {
+    if (st.kind == STEP_REDUCE) return rows / 4;
+    const double* ends = db.ends.data() + (size_t)(st.part - 1) * db.L;
+    const uint32_t from = lab[st.src_col];
+    const double of_label = db.seed_off[from + 1] - db.seed_off[from];
+    double all = 0;
+    for (uint32_t l = 0; l < db.L; ++l) all += ends[l];
+    lab.push_back(st.label);
+    if (all == 0 || of_label == 0) return 0;
+    rows *= ends[from] / of_label * (ends[st.label] / all);
+    if (i > 1) rows *= db.bias[st.part - 1];  // only the first step's sources are any vertices
+    return st.bound_col >= 0 ? rows / 2 : rows;
+}
+
 // Runs every step of a query at once (Chain).  `done` is set when the query is
 // finished: res and the totals are as run_match leaves them, `final` the last
 // step's rows.  Not set: the query does not qualify or an output had no room;
@@ -928,6 +946,16 @@ int run_chain(DevDB& db, const std::vector<Step>& steps, cudaStream_t s, uint64_
     const uint64_t cap = 4 * rows0 + 65536;
     const size_t bytes = cap * wmax * 4;
     if (bytes > budget) return GVA_OK;
+    // With few labels frontiers grow instead: a query that has no room runs
+    // twice, as a chain that fails and counted.  A path / a star of four
+    // vertices / a triangle on one label over 20,000 graphs of 20 to 60 vertices
+    // took 530 / 715 / 203 us after an attempt, 340 / 388 / 201 us counted alone.
+    double rows = (double)rows0;
+    std::vector<uint32_t> lab(1, steps[0].label);
+    for (size_t i = 1; i < n; ++i) {
+        rows = expected_rows(db, steps[i], i, rows, lab);
+        if (rows > (double)cap && !(count_only && i + 1 == n)) return GVA_OK;
+    }
     int rc = set_smem_limits();
     if (rc) return rc;
     const uint64_t most_tiles = (cap + kRowsPerBlock - 1) / kRowsPerBlock;
@@ -941,6 +969,13 @@ int run_chain(DevDB& db, const std::vector<Step>& steps, cudaStream_t s, uint64_
         ctl += 8 * (i == 1 ? (rows0 + kRowsPerBlock - 1) / kRowsPerBlock : most_tiles);
     }
     const bool keep_rows = !count_only;
+    const uint32_t w_last = steps[n - 1].kind == STEP_EXT ? steps[n - 1].width_in + 1 : steps[n - 1].width_in;
+    // a result that is surely larger than kChainResult is written to the chain's
+    // own memory and copied, for which a small one pays (its four-vertex paths on
+    // labelled graphs, 100 KB: 97 us without, 111 with the copy); a second launch
+    // of the last step takes as long as its first
+    const bool via_buf = keep_rows && rows * w_last * 4 > 2.0 * kChainResult;
+    const uint64_t room = via_buf ? cap : kChainResult / 4 / w_last;
     const size_t o_buf = align256(ctl), o_buf2 = o_buf + align256(bytes);
     char* mem = nullptr;
     uint32_t* fin = nullptr;
@@ -953,7 +988,7 @@ int run_chain(DevDB& db, const std::vector<Step>& steps, cudaStream_t s, uint64_
         cudaStream_t s;
         ~Free() { cudaFreeAsync(mem, s); }
     } free_mem{mem, s};
-    if (keep_rows && cudaMallocAsync((void**)&fin, kChainResult, s) != cudaSuccess) {
+    if (keep_rows && !via_buf && cudaMallocAsync((void**)&fin, kChainResult, s) != cudaSuccess) {
         cudaGetLastError();
         return GVA_OK;
     }
@@ -1020,11 +1055,11 @@ int run_chain(DevDB& db, const std::vector<Step>& steps, cudaStream_t s, uint64_
     };
     // from here on errors of the driver end the query
     e = cudaMemsetAsync(mem, 0, ctl, s);
-    const uint32_t w_last = steps[n - 1].kind == STEP_EXT ? steps[n - 1].width_in + 1 : steps[n - 1].width_in;
+    uint32_t* const last_buf = (uint32_t*)(mem + ((n - 1) & 1 ? o_buf : o_buf2));
     for (size_t i = 1; i < n; ++i) {
         const bool last = i + 1 == n;
-        uint32_t* out = last ? fin : (uint32_t*)(mem + (i & 1 ? o_buf : o_buf2));
-        launch(i, i, out, last ? kChainResult / 4 / w_last : cap);
+        uint32_t* out = last ? (via_buf ? last_buf : fin) : (uint32_t*)(mem + (i & 1 ? o_buf : o_buf2));
+        launch(i, i, out, last ? room : cap);
     }
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaEventRecord(hs->ev1, s);
@@ -1038,7 +1073,7 @@ int run_chain(DevDB& db, const std::vector<Step>& steps, cudaStream_t s, uint64_
     bool reached = true;  // the last step's total is known
     for (size_t i = 1; i < n; ++i) totals[i] = h_tot[i];
     for (size_t i = 1; i + 1 < n; ++i) reached = reached && totals[i] <= cap;
-    const bool big = keep_rows && *h_failed == 1 && reached && totals[n - 1] * w_last * 4 > kChainResult;
+    const bool big = keep_rows && *h_failed == 1 && reached && totals[n - 1] > room;
     if (*h_failed && !big) {  // an output had no room (or a wait ran out): counted steps
         drop();
         return GVA_OK;
@@ -1053,15 +1088,19 @@ int run_chain(DevDB& db, const std::vector<Step>& steps, cudaStream_t s, uint64_
         }
     }
     if (keep_rows && totals[n - 1] == 0) drop();
-    if (big) {
+    if (big || (via_buf && totals[n - 1])) {
         drop();
         if (cudaMallocAsync((void**)&fin, totals[n - 1] * w_last * 4, s) != cudaSuccess) {
             fin = nullptr;
             return fail(GVA_ERR_NOMEM, "frontier allocation failed");
         }
         *h_failed = 0;
-        e = cudaMemsetAsync(mem, 0, 8, s);  // the failure mark
-        launch(n - 1, n, fin, totals[n - 1]);
+        if (big) {
+            e = cudaMemsetAsync(mem, 0, 8, s);  // the failure mark
+            launch(n - 1, n, fin, totals[n - 1]);
+        } else {
+            e = cudaMemcpyAsync(fin, last_buf, totals[n - 1] * w_last * 4, cudaMemcpyDeviceToDevice, s);
+        }
         if (e == cudaSuccess) e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaEventRecord(hs->ev1, s);
         if (e == cudaSuccess) e = cudaEventSynchronize(hs->ev1);
@@ -1196,6 +1235,28 @@ int upload_graph(HostGraph& g, int device, DevDB*& out) {
         for (const HostPartition& p : g.parts)
             if (!p.off.empty()) deg += p.off[v * L + L] - p.off[v * L];
         db->max_degree = std::max(db->max_degree, deg);
+    }
+    if (db->max_degree <= kEvenDegree) {  // for expected_rows
+        const size_t P = g.parts.size();
+        db->ends.assign(P * L, 0.0);
+        db->bias.assign(P, 1.0);
+        pool_run((unsigned)P, [&](unsigned p) {
+            const HostPartition& hp = g.parts[p];
+            if (hp.off.empty()) return;
+            double sum = 0, squares = 0;
+            for (uint32_t l = 0; l < L; ++l) {
+                uint64_t at = 0;
+                for (uint32_t i = seed_off[l]; i < seed_off[l + 1]; ++i) {
+                    const uint32_t* o = hp.off.data() + (uint64_t)seed_verts[i] * L;
+                    const uint64_t d = o[L] - o[0];
+                    at += d;
+                    squares += (double)(d * d);
+                }
+                db->ends[p * L + l] = (double)at;
+                sum += (double)at;
+            }
+            if (sum > 0) db->bias[p] = std::max(1.0, squares * (double)seed_verts.size() / (sum * sum));
+        });
     }
     db->arena = arena;
     db->arena_bytes = bytes;

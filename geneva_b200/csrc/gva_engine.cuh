@@ -37,6 +37,11 @@ struct DevDB {
     size_t arena_bytes = 0;
     uint64_t n_adj = 0;
     uint64_t max_degree = 0;              // the most neighbours of one vertex, over all partitions
+    // databases whose queries run as chains (run_chain): per (partition, dense
+    // label) the neighbours that lie there, all vertices' lists together; per
+    // partition how many more a vertex reached by an edge has than any vertex
+    std::vector<double> ends;
+    std::vector<double> bias;
     HostGraph meta;                       // labels/partition presence for lowering (no adjacency)
     uint32_t* vgraph = nullptr;           // optional vertex -> graph id map (graph databases)
     uint32_t num_graphs = 0;
