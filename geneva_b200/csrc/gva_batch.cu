@@ -1524,18 +1524,29 @@ Staging::~Staging() { pin_give(p, cap); }
 // cores taking pieces as they arrive: a copy into pageable memory runs on one
 // core of the driver's, and memory that the caller has never touched is
 // faulted in page by page on the one that writes.  The workers are woken once
-// per 64 MiB (once per piece cost more than it gave).
+// per 64 MiB (once per piece cost more than it gave).  Memory that the driver
+// knows (pinned, managed, a device's) is copied to directly, as is all memory
+// when no staging can be had.
 int copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s) {
     constexpr size_t kWindow = 64u << 20, kPiece = 2u << 20;
     const unsigned T = pool_width();
-    if (bytes < 4 * kPiece || T < 4) {
+    Staging stage;
+    char* from = nullptr;
+    if (bytes >= 4 * kPiece && T >= 4) {
+        cudaPointerAttributes first{}, last{};
+        const bool known = cudaPointerGetAttributes(&first, dst) == cudaSuccess &&
+                           cudaPointerGetAttributes(&last, (char*)dst + bytes - 1) == cudaSuccess;
+        if (!known) cudaGetLastError();
+        if (!known || first.type == cudaMemoryTypeUnregistered || last.type == cudaMemoryTypeUnregistered) {
+            from = stage.get(std::min(bytes, kWindow));
+            if (!from) cudaGetLastError();
+        }
+    }
+    if (!from) {
         GVA_CUDA_B(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
         GVA_CUDA_B(cudaStreamSynchronize(s));
         return GVA_OK;
     }
-    Staging stage;
-    char* from = stage.get(std::min(bytes, kWindow));
-    if (!from) return fail(GVA_ERR_NOMEM, "pinned staging allocation failed");
     std::vector<cudaEvent_t> ev;
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
