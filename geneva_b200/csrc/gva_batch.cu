@@ -2717,26 +2717,26 @@ int BatchSession::run_pages() {
     // of a page = rows of an item of the round that reads it
     uint64_t region = db.round_region_bytes.load();
     if (region == 0) region = 2ull << 30;
-    if (2 * region > budget) return GVA_OK;
     uint64_t slot_most = 1;
     auto page_words = [&](int d) { return (uint64_t)R[d + 1] * wmax[d]; };  // output of depth d
     auto slot_cap = [&](int d) { return std::min<uint64_t>(region / 4 / page_words(d), (1ull << 32) / R[d + 1] - 2); };  // rows of a node: a word
     for (int d = 1; d < D; ++d) slot_most = std::max(slot_most, slot_cap(d));
+    // one allocation, of nearly the same size in every run (a multiple of 256
+    // MiB where the budget holds that): regions, then the schedule's arrays; on
+    // a graph with long lists also the queues of their pieces
+    const size_t o_units = o_rec + al(slot_most * sizeof(uint4));
+    const size_t region_bytes = al(region);
+    const size_t need = 2 * region_bytes + o_units + (long_lists ? 2 * (size_t)kUnitCap * sizeof(Unit) : 0);
+    if (need > budget) return GVA_OK;
+    const size_t unit = (size_t)256 << 20, even = (need + unit - 1) / unit * unit;
     {
         const int rc = ship_nodes();
         if (rc) return rc;
     }
     lap(0);
-    // one allocation, of nearly the same size in every run: regions, then the
-    // schedule's arrays; on a graph with long lists also the queues of their
-    // pieces
-    const size_t o_units = o_rec + al(slot_most * sizeof(uint4));
-    const size_t region_bytes = al(region);
-    const size_t unit = (size_t)256 << 20, blk_bytes = o_units + (long_lists ? 2 * (size_t)kUnitCap * sizeof(Unit) : 0);
     char* mem = nullptr;
     cudaMemPool_t pool = round_pool(db.device);
-    if (!pool || cudaMallocFromPoolAsync((void**)&mem, 2 * region_bytes + (blk_bytes + unit - 1) / unit * unit, pool, s) !=
-                     cudaSuccess) {
+    if (!pool || cudaMallocFromPoolAsync((void**)&mem, even <= budget ? even : need, pool, s) != cudaSuccess) {
         cudaGetLastError();  // no room: counted rounds
         return GVA_OK;
     }

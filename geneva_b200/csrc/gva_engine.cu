@@ -945,7 +945,6 @@ int run_chain(DevDB& db, const std::vector<Step>& steps, cudaStream_t s, uint64_
     // queries on such graphs mostly shrink
     const uint64_t cap = 4 * rows0 + 65536;
     const size_t bytes = cap * wmax * 4;
-    if (bytes > budget) return GVA_OK;
     // With few labels frontiers grow instead: a query that has no room runs
     // twice, as a chain that fails and counted.  A path / a star of four
     // vertices / a triangle on one label over 20,000 graphs of 20 to 60 vertices
@@ -956,8 +955,6 @@ int run_chain(DevDB& db, const std::vector<Step>& steps, cudaStream_t s, uint64_
         rows = expected_rows(db, steps[i], i, rows, lab);
         if (rows > (double)cap && !(count_only && i + 1 == n)) return GVA_OK;
     }
-    int rc = set_smem_limits();
-    if (rc) return rc;
     const uint64_t most_tiles = (cap + kRowsPerBlock - 1) / kRowsPerBlock;
     // control: failed | tile counters | totals | statuses (one step more, for
     // the last step's second launch)
@@ -976,10 +973,13 @@ int run_chain(DevDB& db, const std::vector<Step>& steps, cudaStream_t s, uint64_
     // of the last step takes as long as its first
     const bool via_buf = keep_rows && rows * w_last * 4 > 2.0 * kChainResult;
     const uint64_t room = via_buf ? cap : kChainResult / 4 / w_last;
-    const size_t o_buf = align256(ctl), o_buf2 = o_buf + align256(bytes);
+    const size_t o_buf = align256(ctl), o_buf2 = o_buf + align256(bytes), need = o_buf2 + align256(bytes);
+    if (need + (keep_rows && !via_buf ? kChainResult : 0) > budget) return GVA_OK;
+    const int rc = set_smem_limits();
+    if (rc) return rc;
     char* mem = nullptr;
     uint32_t* fin = nullptr;
-    if (cudaMallocAsync((void**)&mem, o_buf2 + align256(bytes), s) != cudaSuccess) {
+    if (cudaMallocAsync((void**)&mem, need, s) != cudaSuccess) {
         cudaGetLastError();
         return GVA_OK;
     }

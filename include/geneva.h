@@ -174,7 +174,8 @@ void gva_result_free(gva_result* res);
  * plan only counts. */
 typedef struct gva_batch_opts {
     void* stream;          /* cudaStream_t; NULL = legacy default stream            */
-    uint64_t budget_bytes; /* frontier memory cap (0 = 3/4 of free HBM)            */
+    uint64_t budget_bytes; /* frontier memory cap (0 = 3/4 of free HBM), of each half of a run of 12,288 plans or more:
+                              one-pass rounds take two frontier regions and their schedule for each */
     int profile;           /* 1: per-kernel CUDA-event timing in stats->kernels     */
     int flags;             /* GVA_BATCH_* below; 0 = none                           */
 } gva_batch_opts;
