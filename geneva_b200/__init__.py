@@ -110,7 +110,8 @@ class _Tuning(ctypes.Structure):
 
 
 class _Limits(ctypes.Structure):
-    _fields_ = [("mni_pieces", ctypes.c_uint32), ("mni_roots", ctypes.c_uint32), ("mni_groups", ctypes.c_uint32)]
+    _fields_ = [("mni_pieces", ctypes.c_uint32), ("mni_roots", ctypes.c_uint32), ("mni_groups", ctypes.c_uint32),
+                ("round_pieces", ctypes.c_uint32), ("round_sum", ctypes.c_uint32), ("chain_polls", ctypes.c_uint32)]
 
 
 class _BatchStats(ctypes.Structure):
@@ -265,7 +266,8 @@ class Database:
 
     def set_limits(self, **limits) -> None:
         """Capacities of internal queues (gva_limits: mni_pieces, mni_roots,
-        mni_groups); results don't depend on them."""
+        mni_groups, round_pieces, round_sum, chain_polls); results don't
+        depend on them."""
         _check(library().gva_db_set_limits(self._h, ctypes.byref(_Limits(**limits))))
 
     def autotune(self, plans, stream: Optional[int] = None) -> dict:

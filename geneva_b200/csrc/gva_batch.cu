@@ -828,7 +828,6 @@ struct Unit {
     uint32_t task, base, x0, x1;
 };
 constexpr uint32_t kUnitLen = 256;        // candidates that stay with the warp that found them; of a piece
-constexpr uint32_t kUnitCap = 1u << 19;   // pieces of a round, per class
 
 struct PassArgs {
     const TaskDesc* nodes;
@@ -848,7 +847,9 @@ struct PassArgs {
     uint4* rec;                  // per slot written: (task, place among its node's rows, rows, width)
     uint32_t* node_rows;         // per node: rows written
     unsigned long long* node_total;  // per node: rows
-    Unit* units;                 // kUnitCap per class, light class first (null: no list is long)
+    Unit* units;                 // unit_cap per class, light class first (null: no list is long)
+    uint32_t unit_cap;
+    uint32_t most_sum;           // a longer list has its group's rows walked one at a time
     PassState* st;
     BatchCtx ctx;
 };
@@ -994,7 +995,7 @@ __device__ __forceinline__ uint64_t pass_extend(const PassArgs& a, const TaskDes
         }
         if (FUSED) __syncwarp();  // generator states written before other lanes read them
         // lists so long that their sum might not fit a word: one row at a time
-        const bool huge = __any_sync(0xffffffffu, mine > (1u << 26));
+        const bool huge = __any_sync(0xffffffffu, mine > a.most_sum);
         for (uint32_t h = 0; h < (huge ? 32u : 1u); ++h) {
             const uint32_t len = huge && lane != h ? 0 : mine;
             uint32_t inc = len;
@@ -1014,10 +1015,10 @@ __device__ __forceinline__ uint64_t pass_extend(const PassArgs& a, const TaskDes
                 unsigned long long at = 0;
                 if (lane == 0) at = atomicAdd(a.st->units + (FUSED ? 1 : 0), (unsigned long long)np);
                 at = __shfl_sync(0xffffffffu, at, 0);
-                if (at + np <= kUnitCap) stop = kUnitLen;  // else the list stays here, and empty pieces there
-                for (uint32_t i = lane; i < np && at + i < kUnitCap; i += 32) {
+                if (at + np <= a.unit_cap) stop = kUnitLen;  // else the list stays here, and empty pieces there
+                for (uint32_t i = lane; i < np && at + i < a.unit_cap; i += 32) {
                     const uint32_t x = (i + 1) * kUnitLen;
-                    a.units[(FUSED ? kUnitCap : 0) + at + i] =
+                    a.units[(FUSED ? a.unit_cap : 0) + at + i] =
                         Unit{item, task, base, x, stop == all ? x : min(all, x + kUnitLen)};
                 }
             }
@@ -1177,7 +1178,7 @@ round_pass_kernel(const __grid_constant__ PassArgs a) {
     bool ready = false;               // light class: the current item's rows were issued with the previous item
     Pages pg;
     const uint64_t light = a.st->ni_light;
-    const Span sp = UNITS ? Span{0, umin64(a.st->units[FUSED ? 1 : 0], kUnitCap), a.st->unit_heads + (FUSED ? 1 : 0),
+    const Span sp = UNITS ? Span{0, umin64(a.st->units[FUSED ? 1 : 0], a.unit_cap), a.st->unit_heads + (FUSED ? 1 : 0),
                                  gridDim.x * kRoundWarps}
                           : Span{FUSED ? light : 0, FUSED ? a.st->ni - light : light, a.st->heads + (FUSED ? 1 : 0),
                                  gridDim.x * kRoundWarps};
@@ -1216,7 +1217,7 @@ round_pass_kernel(const __grid_constant__ PassArgs a) {
     if (UNITS) {
         while (next_chunk_or_own(sp, first, begin, end)) {
             for (uint64_t u = begin; u < end; ++u) {
-                const Unit unit = a.units[(FUSED ? kUnitCap : 0) + u];
+                const Unit unit = a.units[(FUSED ? a.unit_cap : 0) + u];
                 if (unit.x0 >= unit.x1) continue;
                 if (unit.task != t) open_task(unit.task);
                 __syncwarp();
@@ -2745,7 +2746,7 @@ int BatchSession::run_pages() {
     // a graph with long lists also the queues of their pieces
     const size_t o_units = o_rec + al(slot_most * sizeof(uint4));
     const size_t region_bytes = al(region);
-    const size_t need = 2 * region_bytes + o_units + (long_lists ? 2 * (size_t)kUnitCap * sizeof(Unit) : 0);
+    const size_t need = 2 * region_bytes + o_units + (long_lists ? 2 * (size_t)db.round_pieces * sizeof(Unit) : 0);
     if (need > budget) return GVA_OK;
     const size_t unit = (size_t)256 << 20, even = (need + unit - 1) / unit * unit;
     {
@@ -2828,6 +2829,8 @@ int BatchSession::run_pages() {
         pa.rec = (uint4*)(blk + o_rec);
         pa.node_rows = (uint32_t*)(blk + o_nrows);
         pa.node_total = ntot;
+        pa.unit_cap = db.round_pieces;
+        pa.most_sum = db.round_sum;
         pa.units = long_lists ? (Unit*)(blk + o_units) : nullptr;
         pa.st = states + d;
         pa.ctx = ctx;

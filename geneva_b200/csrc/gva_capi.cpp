@@ -645,7 +645,12 @@ int gva_db_set_limits(gva_db* db, const gva_limits* l) {
     if (!db || !l) return fail(GVA_ERR_ARG, "null argument");
     if ((l->mni_pieces && l->mni_pieces < 32) || (l->mni_roots && l->mni_roots < 32))
         return fail(GVA_ERR_ARG, "mni_pieces and mni_roots must be 32 or more");  // a warp's roots must fit
+    if (l->round_pieces > (1u << 20) || l->round_sum > (1u << 26))
+        return fail(GVA_ERR_ARG, "round_pieces may be 2^20, round_sum 2^26 at most");  // 32 lists fit a word
     DevDB& d = *db->dev;
+    if (l->round_pieces) d.round_pieces = l->round_pieces;
+    if (l->round_sum) d.round_sum = l->round_sum;
+    if (l->chain_polls) d.chain_polls = l->chain_polls;
     if (l->mni_pieces) d.mni_pieces = l->mni_pieces;
     if (l->mni_roots) d.mni_roots = l->mni_roots;
     if (l->mni_groups) d.mni_groups = l->mni_groups;

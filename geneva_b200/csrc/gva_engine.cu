@@ -412,8 +412,8 @@ struct Chain {
     uint64_t* host_out;              // the same, in host memory
     uint32_t* failed;                // 1: an output has no room, 2: a wait ran out
     uint32_t* host_failed;
+    uint32_t polls;                  // of a tile for the ones before it, then the chain fails
 };
-constexpr uint32_t kWaitPolls = 1u << 20;  // of a tile for the ones before it, then the chain fails
 
 __device__ __forceinline__ void chain_fail(const Chain& c, uint32_t why) {
     *(volatile uint32_t*)c.failed = why;
@@ -470,7 +470,7 @@ __device__ __forceinline__ uint64_t chain_place(const Chain& c, uint64_t tile, u
                 // lanes up to the nearest finished prefix
                 const uint32_t upto = done ? (done & -done) | ((done & -done) - 1) : 0xffffffffu;
                 if (none & upto) {
-                    ok = ++polls < kWaitPolls;
+                    ok = ++polls < c.polls;
                     continue;
                 }
                 sum += __shfl_sync(0xffffffffu, warp_sum((upto >> lane & 1) ? (uint64_t)(w & kMask) : 0), 0);
@@ -1013,6 +1013,7 @@ int run_chain(DevDB& db, const std::vector<Step>& steps, cudaStream_t s, uint64_
         c.host_out = const_cast<uint64_t*>(h_tot) + (i == slot ? i : 0);
         c.failed = (uint32_t*)mem;
         c.host_failed = const_cast<uint32_t*>(h_failed);
+        c.polls = db.chain_polls;
         const uint32_t* in = i == 1 ? db.seed_verts + db.seed_off[steps[0].label] : (uint32_t*)(mem + (i & 1 ? o_buf2 : o_buf));
         // a CTA per tile of the seeds while they fit the chip at once (a tile
         // waits for the ones before it); later steps mostly have fewer, and a

@@ -57,6 +57,12 @@ struct DevDB {
     // roots that they may belong to, groups of 32 seeds that a warp does in one
     // launch (512 x a lane's 96 candidates: some tens of milliseconds)
     uint32_t mni_pieces = 1u << 18, mni_roots = 1u << 18, mni_groups = 512;
+    // one-pass rounds: pieces of long lists per class, and the longest list
+    // that a group of 32 rows adds up in a word
+    uint32_t round_pieces = 1u << 19, round_sum = 1u << 26;
+    // chained steps: looks of a tile at the ones before it until the chain
+    // gives up (some tenths of a second)
+    uint32_t chain_polls = 1u << 20;
 };
 
 int upload_graph(HostGraph& g, int device, DevDB*& out);

@@ -280,6 +280,10 @@ typedef struct gva_limits {
     uint32_t mni_pieces;  /* MNI: pieces of unfinished searches per queue, 128 bytes each (32 or more; 262144) */
     uint32_t mni_roots;   /* MNI: roots that they may belong to at once (32 or more; 262144) */
     uint32_t mni_groups;  /* MNI: groups of 32 seeds that a warp does per launch (512) */
+    uint32_t round_pieces; /* one-pass rounds: pieces of long lists per class, 24 bytes each (up to 1048576; 524288) */
+    uint32_t round_sum;   /* one-pass rounds: the longest list that is added up with its group's (up to 67108864, its
+                             default) */
+    uint32_t chain_polls; /* chained steps: looks at the tiles before a tile until the chain gives up (1048576) */
 } gva_limits;
 int gva_db_set_limits(gva_db* db, const gva_limits* limits);
 
