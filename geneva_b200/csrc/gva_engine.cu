@@ -29,7 +29,6 @@
 #include "../../include/geneva.h"
 #include "gva_engine.cuh"
 #include "gva_kernels.cuh"
-#include "gva_pool.h"
 
 namespace gva {
 
@@ -1237,27 +1236,30 @@ int upload_graph(HostGraph& g, int device, DevDB*& out) {
             if (!p.off.empty()) deg += p.off[v * L + L] - p.off[v * L];
         db->max_degree = std::max(db->max_degree, deg);
     }
-    if (db->max_degree <= kEvenDegree) {  // for expected_rows
-        const size_t P = g.parts.size();
+    if (db->max_degree <= kEvenDegree) {  // for expected_rows: some of each label's vertices
+        const size_t P = g.parts.size(), most = std::max<size_t>(16, 16384 / std::max<uint32_t>(L, 1));
         db->ends.assign(P * L, 0.0);
         db->bias.assign(P, 1.0);
-        pool_run((unsigned)P, [&](unsigned p) {
+        for (size_t p = 0; p < P; ++p) {
             const HostPartition& hp = g.parts[p];
-            if (hp.off.empty()) return;
-            double sum = 0, squares = 0;
+            if (hp.off.empty()) continue;
+            double all = 0, squares = 0;
             for (uint32_t l = 0; l < L; ++l) {
-                uint64_t at = 0;
-                for (uint32_t i = seed_off[l]; i < seed_off[l + 1]; ++i) {
-                    const uint32_t* o = hp.off.data() + (uint64_t)seed_verts[i] * L;
+                const size_t n = seed_off[l + 1] - seed_off[l], m = std::min(n, most);
+                uint64_t sum = 0, sq = 0;
+                for (size_t i = 0; i < m; ++i) {
+                    const uint32_t* o = hp.off.data() + (uint64_t)seed_verts[seed_off[l] + n * i / m] * L;
                     const uint64_t d = o[L] - o[0];
-                    at += d;
-                    squares += (double)(d * d);
+                    sum += d;
+                    sq += d * d;
                 }
-                db->ends[p * L + l] = (double)at;
-                sum += (double)at;
+                if (m == 0) continue;
+                db->ends[p * L + l] = (double)sum * (double)n / (double)m;
+                squares += (double)sq * (double)n / (double)m;
+                all += db->ends[p * L + l];
             }
-            if (sum > 0) db->bias[p] = std::max(1.0, squares * (double)seed_verts.size() / (sum * sum));
-        });
+            if (all > 0) db->bias[p] = std::max(1.0, squares * (double)seed_verts.size() / (all * all));
+        }
     }
     db->arena = arena;
     db->arena_bytes = bytes;
