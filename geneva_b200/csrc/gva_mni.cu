@@ -1008,6 +1008,24 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
                                          : std::max<uint64_t>(1, slots_all * sm_percent / 100);
             const uint64_t grid = std::min<uint64_t>(cta_cap, (nitems + kMniWarps - 1) / kMniWarps);
             const int many = total > 4 * cta_cap * kMniWarps * kMniManySeeds;
+            // Beside other work the searches leave the SMs' memory to it: an SM's
+            // split of shared memory and L1 stays as its first kernel asks while
+            // any of its CTAs run, and these, which ask for almost none, kept a
+            // server's matching rounds waiting for whole launches (requests at
+            // 1,000 per second: p99 108 ms, 28 now; a mining run beside them 400 / 485).
+            auto start = [&](auto kernel, uint64_t ctas, auto... args) {
+                cudaLaunchConfig_t cfg{};
+                cfg.gridDim = dim3((unsigned)ctas);
+                cfg.blockDim = dim3(kMniWarps * 32);
+                cfg.stream = s;
+                cudaLaunchAttribute at{};
+                at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+                at.val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+                cfg.attrs = &at;
+                cfg.numAttrs = cta_cap < slots_all ? 1 : 0;
+                return cudaLaunchKernelEx(&cfg, kernel, args...);
+            };
+            cudaError_t started = cudaSuccess;
             cudaEvent_t ev = nullptr;
             const double rows = (double)total;
             mni_expand_kernel<<<(unsigned)std::min<uint64_t>((ns + 255) / 256, 4096), 256, 0, s>>>(d_item0, ns,
@@ -1020,15 +1038,15 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
             const unsigned long long* hstate = (const unsigned long long*)((const char*)hcounts + o_queue) + 1;
             for (bool resume = false;; resume = true) {
                 if (profile) prof.begin(K_MNI, 0.0, s, ev);
-                mni_search_kernel<<<(unsigned)std::max<uint64_t>(grid, 1), kMniWarps * 32, 0, s>>>(
-                    d_tasks, d_slots, d_item0, d_item_slot, nitems, db.seed_by_degree, (uint32_t)item_len, d_parts,
-                    db.kernel_L(), d_counts, d_queue, H, d_save, resume, db.mni_groups, kLaneBudget[many],
-                    profile ? d_prof : nullptr);
+                started = start(mni_search_kernel, std::max<uint64_t>(grid, 1), d_tasks, d_slots, d_item0, d_item_slot,
+                                nitems, db.seed_by_degree, (uint32_t)item_len, d_parts, db.kernel_L(), d_counts, d_queue,
+                                H, d_save, resume, db.mni_groups, kLaneBudget[many], profile ? d_prof : nullptr);
                 if (profile) prof.end(ev, K_MNI, 0.0, s, resume ? 0.0 : rows);
                 st.launches += 1;
                 g_mni_launches += 1;
                 for (int q = 0;;) {
                     cudaError_t le = cudaGetLastError();
+                    if (le == cudaSuccess) le = started;
                     if (le == cudaSuccess) le = cudaMemcpyAsync(hcounts, d_counts, bytes_back, cudaMemcpyDeviceToHost, s);
                     if (le != cudaSuccess) {
                         rc = fail(GVA_ERR_CUDA, std::string("MNI search launch failed: ") + cudaGetErrorString(le));
@@ -1049,8 +1067,9 @@ int mni_run_prepared(DevDB& db, const MniPrepared& prep, uint32_t cap, bool plai
                     for (int k = 0; k < 4; ++k, q ^= 1) {
                         cudaMemsetAsync(H.state + kQueueWords * (q ^ 1), 0, kQueueWords * 8, s);  // taken by the launch before
                         if (profile) prof.begin(K_MNI, 0.0, s, ev);
-                        mni_piece_kernel<<<(unsigned)cta_cap, kMniWarps * 32, 0, s>>>(
-                            d_tasks, d_parts, db.kernel_L(), d_counts, H, q, kPieceBudget[many], profile ? d_prof : nullptr);
+                        const cudaError_t pe = start(mni_piece_kernel, cta_cap, d_tasks, d_parts, db.kernel_L(), d_counts, H,
+                                                     q, kPieceBudget[many], profile ? d_prof : nullptr);
+                        if (started == cudaSuccess) started = pe;
                         if (profile) prof.end(ev, K_MNI, 0.0, s, 0.0);
                     }
                     st.launches += 4;
