@@ -725,12 +725,13 @@ void fill_red(RedArgs& a, const DevDB& db, const Step& st, const uint32_t* in, u
 // SM, at least a block's worth and at most 32,768.  On a graph without long
 // lists the blocks' outputs are alike and a CTA takes its block without a
 // search (chunk 0; 6.0 against 8.6 us for 1,144 blocks).
-uint64_t chunk_of(uint64_t total, uint64_t nb) {
+uint64_t chunk_of(const DevDB& db, uint64_t total, uint64_t nb) {
     const uint64_t all = total + nb * kBlockWork;
-    return std::min<uint64_t>(std::max<uint64_t>((all + 148 * 24 - 1) / (148 * 24), kBlockWork + 256), 32768);
+    const uint64_t ctas = (uint64_t)db.sms * 24;
+    return std::min<uint64_t>(std::max<uint64_t>((all + ctas - 1) / ctas, kBlockWork + 256), 32768);
 }
-uint64_t num_chunks(uint64_t total, uint64_t nb) {
-    const uint64_t c = chunk_of(total, nb);
+uint64_t num_chunks(const DevDB& db, uint64_t total, uint64_t nb) {
+    const uint64_t c = chunk_of(db, total, nb);
     return (total + nb * kBlockWork + c - 1) / c;
 }
 
@@ -807,10 +808,10 @@ int launch_write(const DevDB& db, const Step& st, const uint32_t* in, uint64_t n
         const double bytes = (4.0 * k + 8.0) * (double)nrows + (4.0 + 4.0 * (k + 1)) * (double)nout;
         if (prof) prof->begin(K_EXT_WRITE, bytes, s, ev);
         const bool even = db.max_degree <= kEvenDegree;
-        const uint64_t nch = even ? nb : num_chunks(nout, nb);
+        const uint64_t nch = even ? nb : num_chunks(db, nout, nb);
         if (nch > 0x7fffffffull) return fail(GVA_ERR_UNSUPPORTED, "frontier too large for one launch");
         ext_write_kernel<<<(unsigned)nch, kThreads, ext_smem_bytes(a.k, a.n_eq), s>>>(a, sums, nb,
-                                                                                      even ? 0 : chunk_of(nout, nb));
+                                                                                      even ? 0 : chunk_of(db, nout, nb));
         if (prof) prof->end(ev, K_EXT_WRITE, bytes, s, (double)nrows);
     } else {
         RedArgs a;
@@ -833,7 +834,7 @@ int launch_ext_red(const DevDB& db, const Step& st, const Step& rd, const uint32
                    Profiler* prof) {
     int rc = set_smem_limits();
     if (rc) return rc;
-    const uint64_t nb = (nrows + kRowsPerBlock - 1) / kRowsPerBlock, nch = num_chunks(total, nb);
+    const uint64_t nb = (nrows + kRowsPerBlock - 1) / kRowsPerBlock, nch = num_chunks(db, total, nb);
     if (nch > 0x7fffffffull) return fail(GVA_ERR_UNSUPPORTED, "frontier too large for one launch");
     ExtArgs a;
     fill_ext(a, db, st, in, nrows, out);
@@ -854,8 +855,8 @@ int launch_ext_red(const DevDB& db, const Step& st, const Step& rd, const uint32
     if (!out) {
         const double bytes = (4.0 * k + 8.0) * (double)nrows + (4.0 + 8.0 * rd.n_pairs) * (double)total;
         if (prof) prof->begin(K_RED_COUNT, bytes, s, ev);
-        ext_red_kernel<false><<<(unsigned)nch, kThreads, smem, s>>>(a, sums, nb, chunk_of(total, nb), csums, masks,
-                                                                        mask_cap(chunk_of(total, nb), a.n_eq));
+        ext_red_kernel<false><<<(unsigned)nch, kThreads, smem, s>>>(a, sums, nb, chunk_of(db, total, nb), csums, masks,
+                                                                        mask_cap(chunk_of(db, total, nb), a.n_eq));
         if (prof) prof->end(ev, K_RED_COUNT, bytes, s, (double)total);
         GVA_CUDA(cudaGetLastError());
         if (prof) prof->begin(K_SCAN, 16.0 * (double)nch, s, ev);
@@ -866,8 +867,8 @@ int launch_ext_red(const DevDB& db, const Step& st, const Step& rd, const uint32
         const double bytes = (4.0 * k + 8.0) * (double)nrows + (4.0 + 8.0 * rd.n_pairs) * (double)total +
                              4.0 * (k + 1) * (double)kept;
         if (prof) prof->begin(K_RED_WRITE, bytes, s, ev);
-        ext_red_kernel<true><<<(unsigned)nch, kThreads, smem, s>>>(a, sums, nb, chunk_of(total, nb), csums, masks,
-                                                                        mask_cap(chunk_of(total, nb), a.n_eq));
+        ext_red_kernel<true><<<(unsigned)nch, kThreads, smem, s>>>(a, sums, nb, chunk_of(db, total, nb), csums, masks,
+                                                                        mask_cap(chunk_of(db, total, nb), a.n_eq));
         if (prof) prof->end(ev, K_RED_WRITE, bytes, s, (double)total);
         g_launches += 1;
     }
@@ -1019,8 +1020,8 @@ int run_chain(DevDB& db, const std::vector<Step>& steps, cudaStream_t s, uint64_
         // CTA that finds none costs a launch slot: 1,184 CTAs for 228 tiles
         // took 16 us, 444 take 11
         const uint64_t tiles = (rows0 + kRowsPerBlock - 1) / kRowsPerBlock;
-        const unsigned grid = (unsigned)(i == 1 ? std::min<uint64_t>(tiles, 148 * 8)
-                                                : std::min<uint64_t>(std::max<uint64_t>(2 * tiles, 64), 148 * 3));
+        const unsigned grid = (unsigned)(i == 1 ? std::min<uint64_t>(tiles, db.sms * 8)
+                                                : std::min<uint64_t>(std::max<uint64_t>(2 * tiles, 64), db.sms * 3));
         const bool counts = count_only && i + 1 == n;
         auto start = [&](auto kernel, size_t smem, auto args) {
             cudaLaunchConfig_t cfg{};
@@ -1223,6 +1224,7 @@ int upload_graph(HostGraph& g, int device, DevDB*& out) {
     if (e != cudaSuccess) return fail(GVA_ERR_NOMEM, std::string("database allocation failed: ") + cudaGetErrorString(e));
     DevDB* db = new DevDB();
     db->device = device;
+    cudaDeviceGetAttribute(&db->sms, cudaDevAttrMultiProcessorCount, device);
     db->max_id = g.max_id;
     db->L = L;
     db->packed = packed;
@@ -1446,9 +1448,9 @@ int run_match(DevDB& db, const Plan& plan, const std::vector<Step>& steps, cudaS
                 }
                 if (st.phase_end >= 0) res.phase_rows[st.phase_end] = total;
                 const Step& rd = steps[i + 1];
-                const uint64_t nch = num_chunks(total, nb);
+                const uint64_t nch = num_chunks(db, total, nb);
                 uint64_t* csums = nullptr;
-                ce = cudaMallocAsync((void**)&csums, (nch + 1) * 8 + nch * mask_cap(chunk_of(total, nb), st.n_eq), s);
+                ce = cudaMallocAsync((void**)&csums, (nch + 1) * 8 + nch * mask_cap(chunk_of(db, total, nb), st.n_eq), s);
                 if (ce != cudaSuccess) { status = fail(GVA_ERR_NOMEM, "scratch allocation failed"); break; }
                 uint8_t* masks = (uint8_t*)(csums + nch + 1);
                 status = launch_ext_red(db, st, rd, cur, rows, total, sums, csums, masks, nullptr, 0, s, prof);

@@ -24,6 +24,7 @@ struct DevPart {
 //   seed_verts[...] | seed_by_degree[...] | per partition: off[...] adj[...]
 struct DevDB {
     int device = 0;
+    int sms = 148;                        // of the device
     uint32_t max_id = 0;
     uint32_t L = 0;                       // dense vertex labels
     bool packed = false;                  // segment index layout (seg_of): packed records, else dense
