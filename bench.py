@@ -855,9 +855,9 @@ def batch_bench(args, rank, world, local, dist, torch, gv, workloads):
     torch.cuda.nvtx.range_pop()
     stream.synchronize()
 
-    # ---- the same step with its rounds scheduled the other way (on the
-    # device when the timed steps were scheduled on the host, and the
-    # reverse), for comparison
+    # ---- the same step with its rounds scheduled another way, for
+    # comparison: one-pass rounds launched at once when the timed steps
+    # launched them one after another, else counted rounds
     other = "device" if tstats["device_rounds"] == 0 else "host"
     host_ms = []
     for i in range(3):
@@ -976,7 +976,9 @@ def batch_bench(args, rank, world, local, dist, torch, gv, workloads):
                           "to host, support from their graph ids (count_only: embeddings only)"},
         "roofline": {"bound": "hbm", "kernel": name, "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_source": peak_kind, "traffic": ncu_traffic(name, s),
-                     "launches": s["launches"], "kernel_ms": s["ms"]},
+                     "launches": s["launches"], "kernel_ms": s["ms"],
+                     "path": "kernels of the profiled step, which runs counted rounds on one stream; the timed steps "
+                             "run one-pass rounds"},
         "kernels": kstats,
         # host figures of the last timed step (the profiled step keeps one
         # stream and synchronises around every kernel)
@@ -985,12 +987,14 @@ def batch_bench(args, rank, world, local, dist, torch, gv, workloads):
                                                 "round_phase_ms", "wait_ms", "session_ms", "timeline_ms")},
                       timeline="ms from the start of the batched run: plans ordered; per half: session prepared, "
                                "rounds done, results read, session freed",
-                      scheduling="device" if tstats["device_rounds"] else "host",
+                      scheduling="one-pass rounds, " + ("launched at once" if tstats["device_rounds"]
+                                                        else "each launched when the one before was read"),
                       other_scheduling={"scheduling": other, "ms_per_step": statistics.mean(host_ms),
                                         "embeddings_per_s": emb_local / args.steps / (statistics.mean(host_ms) / 1000.0),
                                         "agree": host_rounds_agree,
-                                        "path": f"the same step with every round scheduled on the {other} "
-                                                f"(GVA_BATCH_{other.upper()}_ROUNDS), mean of 2 after 1 warm-up"}),
+                                        "path": "the same step with " + ("one-pass rounds launched at once" if other == "device"
+                                                                         else "counted rounds") +
+                                                f" (GVA_BATCH_{other.upper()}_ROUNDS), mean of 2 after 1 warm-up"}),
         "tuning": dict(tuning, calibration=f"first {min(args.tune_patterns, len(plans))} patterns of the list, "
                                            f"counted with supports: rows by one-pass rounds, hub by counted rounds "
                                            f"(gva_db_autotune)"),

@@ -146,7 +146,8 @@ void gva_plan_free(gva_plan* plan);
 /* ---- L3: one query end to end -----------------------------------------------
  * Replaces the phase loop of gpumine / gpumineSV main (src/gpumine.cpp:932-1061):
  * init, every E and R phase, frontier growth handled by chunking against
- * budget_bytes instead of host spill.  The result stays on the device. */
+ * budget_bytes instead of host spill.  The result stays on the device (a small
+ * one may hold 256 KiB) until it is freed. */
 int gva_match(gva_db* db, const gva_plan* plan, const gva_match_opts* opts, gva_result** out);
 uint64_t gva_result_num_rows(const gva_result* res);
 int gva_result_num_columns(const gva_result* res);
@@ -274,7 +275,7 @@ int gva_db_set_tuning(gva_db* db, const gva_tuning* tuning);
 int gva_db_autotune(gva_db* db, const gva_plan* const* plans, int nplans, void* stream, gva_tuning* out);
 
 /* Capacities of internal queues on one database.  Results don't depend on
- * them; smaller ones take less memory and more launches.  0 leaves a field as
+ * them; smaller ones take less memory and more launches, or a fallback path.  0 leaves a field as
  * it is.  Not to be changed while a call on the database runs. */
 typedef struct gva_limits {
     uint32_t mni_pieces;  /* MNI: pieces of unfinished searches per queue, 128 bytes each (32 or more; 262144) */
