@@ -37,7 +37,7 @@ def test_kept_regions_are_given_back_when_the_device_is_full(graphs):
     """64 GiB of regions stay with their pool after a run; a query's 15 GB
     frontier is then allocated on a device that has 4 GiB free beside them."""
     gdb, plans = graphs
-    free, _ = torch.cuda.mem_get_info()
+    free, total = torch.cuda.mem_get_info()
     if free < (100 << 30):
         pytest.skip("needs 100 GiB of free device memory")
     leaves = 50_000
@@ -49,7 +49,7 @@ def test_kept_regions_are_given_back_when_the_device_is_full(graphs):
     assert stats["device_rounds"] > 0
     torch.cuda.synchronize()
     kept, _ = torch.cuda.mem_get_info()
-    assert kept < free - (60 << 30)
+    assert kept < total - (64 << 30)  # the pool may have held some of it before
     fill = torch.empty(kept - (4 << 30), dtype=torch.uint8, device="cuda")
     res = gv.match(star, gv.Plan.from_text("v 0 1\nv 1 2\nv 2 2\ne 0 1 1\ne 0 2 1\n"), budget_bytes=40 << 30)
     assert res.num_rows == leaves * (leaves - 1) // 2
