@@ -83,7 +83,7 @@ struct BatchCtx {
 // pass's items [item0[t], item0[t + 1]).
 struct TaskRef {
     uint32_t node;
-    uint32_t pad;
+    uint32_t counted;  // an earlier round accounted for the slice per graph
     const uint32_t* in;
     uint64_t nrows;
 };
@@ -570,6 +570,10 @@ round_count_kernel(RoundArgs a) {
                 nrows = ref.nrows;
                 __syncwarp();
                 load_desc(d, a.nodes + ref.node);
+                if (ref.counted) {
+                    d.mode = MODE_WRITE;  // all lanes store the same word
+                    __syncwarp();
+                }
             }
             const uint64_t row0 = (item - t_lo) * a.rows_per_item;
             const uint32_t nr = (uint32_t)umin64(a.rows_per_item, nrows - row0);
@@ -2287,7 +2291,7 @@ int BatchSession::round() {
         const BTask& tk = active[t];
         BNode& nd = nodes[tk.node];
         if (!nd.fused) ni_light = ni + (tk.rows + R - 1) / R;
-        refs[t] = TaskRef{(uint32_t)tk.node, 0u, tk.in, tk.rows};
+        refs[t] = TaskRef{(uint32_t)tk.node, tk.counted, tk.in, tk.rows};
         ni += (tk.rows + R - 1) / R;
         h_item0[t + 1] = ni;
         cbytes += (4.0 * nd.width_in + 8.0 * (nd.kind == STEP_EXT ? 1 : nd.n_pairs)) * (double)tk.rows;
@@ -2410,7 +2414,9 @@ int BatchSession::round() {
     order.clear();
     for (int t = 0; t < nt; ++t) {
         const BNode& nd = nodes[active[t].node];
-        for (int q = nd.first_term; q >= 0; q = plans[q].next_term) plans[q].count += h_totals[t];
+        if (!active[t].counted)
+            for (int q = nd.first_term; q >= 0; q = plans[q].next_term) plans[q].count += h_totals[t];
+        active[t].counted = true;  // also of its halves, and when it waits
         if (nd.first_child >= 0 && h_totals[t] > 0) order.push_back(t);
     }
     if (want > budget)

@@ -180,6 +180,7 @@ public:
         const uint32_t* in;  // frontier slice
         uint64_t rows;
         std::shared_ptr<void> owner;
+        bool counted = false;  // the plans that end at its node have its rows (it is back: split, or it waits for room)
     };
     struct PlanRec {
         uint64_t tag = 0;
