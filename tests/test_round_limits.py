@@ -51,6 +51,30 @@ def test_chain_that_gives_up(native, oracle, polls):
     db.close()
 
 
+@pytest.fixture(scope="module")
+def one_label(native):
+    labels, src, dst, el = small_graphs(3000, 6, 3)
+    labels[1:] = 1
+    db = gv.Database.from_edges(labels, src, dst, el)
+    yield db
+    db.close()
+
+
+@pytest.mark.parametrize("polls", [1, 2, 4, 8, 16, 64])
+def test_last_step_that_gives_up(one_label, polls):
+    """A result beyond the small buffer: the last step runs a second time, and
+    its tiles may give up waiting in either run, or in neither."""
+    plan = gv.Plan.from_text("v 0 1\nv 1 1\ne 0 1 1\n")
+    want = gv.match(one_label, plan, profile=True)
+    rows = want.rows()
+    assert 256 << 10 < rows.nbytes < 512 << 10
+    one_label.set_limits(chain_polls=polls)
+    for _ in range(60):
+        res = gv.match(one_label, plan)
+        assert res.phase_rows == want.phase_rows
+        assert np.array_equal(res.rows(), rows)
+
+
 def test_limits_are_checked(native):
     db = gv.Database.from_edges(np.array([0, 1, 1], np.uint32), np.array([1], np.uint32), np.array([2], np.uint32),
                                 np.array([1], np.uint32))
