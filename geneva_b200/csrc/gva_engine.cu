@@ -923,8 +923,8 @@ double expected_rows(const DevDB& db, const Step& st, size_t i, double rows, std
 
 // Runs every step of a query at once (Chain).  `done` is set when the query is
 // finished: res and the totals are as run_match leaves them, `final` the last
-// step's rows.  Not set: the query does not qualify or an output had no room;
-// nothing is kept.
+// step's rows.  Not set: the query does not qualify, an output had no room or a
+// wait ran out; nothing is kept.
 int run_chain(DevDB& db, const std::vector<Step>& steps, cudaStream_t s, uint64_t budget, bool count_only,
               HostStage* hs, std::vector<uint64_t>& totals, uint32_t*& final, bool& done) {
     done = false;
